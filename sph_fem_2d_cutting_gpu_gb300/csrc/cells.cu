@@ -159,16 +159,21 @@ __global__ void __launch_bounds__(kBlock) k_gather_plain(int N, const int32_t *_
 
 // FP64 record: (x, y, vx, vy) (sA, sB, sC, Rxx) (Rxy, Ryy, h, rho) (c, vol, T, flags)
 // with sA = (Sxx-p)/rho^2, sB = Sxy/rho^2, sC = (Syy-p)/rho^2 (interactions_gpu.cu:278-281),
-// c = sqrtf(K/rho) (:294-295), vol = mass/rho (:250).
-__device__ __forceinline__ void write_record64(dbl4 *__restrict__ rec, int k, const KConsts &K, double2 pos,
+// c = -alpha/2 sqrtf(K/rho), the share of this particle in -alpha c_ij (:294-303),
+// vol = mass/rho (:250); and the candidate entry.
+__device__ __forceinline__ void write_record64(dbl4 *__restrict__ rec, float2 *__restrict__ cand, int k,
+                                               const KConsts &K, double2 pos,
                                                double2 vel, dbl4 S, dbl4 R, double p, double h, double rho,
-                                               double T, double blanked, double tool, int row) {
+                                               double T, double blanked, double tool, int hash) {
+    const sph_geom_constants &g = K.g;
+    int ci = 0, row = 0;
+    if (hash >= 0 && hash < g.num_cell) { ci = hash / g.ny; row = hash - ci * g.ny; }
     double rho21 = 1. / (rho * rho);
     dbl4 r0 = mk4(pos.x, pos.y, vel.x, vel.y);
     dbl4 r1 = mk4((S.x - p) * rho21, S.y * rho21, (S.z - p) * rho21, R.x);
     dbl4 r2 = mk4(R.y, R.z, h, rho);
     int flags = (row & kRowMask) | (blanked == 1. ? kFlagBlanked : 0) | (tool == 1. ? kFlagTool : 0);
-    const double c = sqrtf_d(K.c.phys.K / rho), vol = K.c.phys.mass / rho;
+    const double c = -0.5 * K.c.corr.alpha * sqrtf_d(K.c.phys.K / rho), vol = K.c.phys.mass / rho;
     if (!(flags & kFlagBlanked) && (nonfinite4(r0) || nonfinite4(r1) || nonfinite4(r2) || is_nan_or_inf(c) ||
                                     is_nan_or_inf(vol) || is_nan_or_inf(T)))
         flags |= kFlagNonFinite;   // blanked records are skipped as neighbours: no mark
@@ -177,6 +182,8 @@ __device__ __forceinline__ void write_record64(dbl4 *__restrict__ rec, int k, co
     rec[4 * k + 1] = r1;
     rec[4 * k + 2] = r2;
     rec[4 * k + 3] = r3;
+    cand[k] = cand_pack64((float)(pos.x - (g.bbmin_x + (double)ci * g.dx)),
+                          (float)(pos.y - (g.bbmin_y + (double)row * g.dx)), K.f.cell, flags);
 }
 
 // FP32 record: (xr, yr, flags|row, h) (vx, vy, rho, c) (sA, sB, sC, vol) (Rxx, Rxy, Ryy, T)
@@ -223,10 +230,8 @@ __global__ void __launch_bounds__(kBlock) k_build_records(int N, KConsts K, Sort
     double T = A.T[k];
     int hash = A.hash[k];
     if (rec64) {
-        int row = 0;
-        if (hash >= 0 && hash < K.g.num_cell) row = hash - (hash / K.g.ny) * K.g.ny;
-        write_record64(rec64, k, K, A.pos[k], A.vel[k], A.S[k], F.R[k], F.p[k], A.h[k], A.rho[k], T, A.blanked[k],
-                       tool, row);
+        write_record64(rec64, cand32, k, K, A.pos[k], A.vel[k], A.S[k], F.R[k], F.p[k], A.h[k], A.rho[k], T,
+                       A.blanked[k], tool, hash);
     } else {
         write_record32(rec32, cand32, k, K, A.pos[k], A.vel[k], A.S[k], F.R[k], F.p[k], A.h[k], A.rho[k], T, A.blanked[k],
                        tool, hash);
@@ -303,9 +308,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused(int N, const int32_t *_
     }
     double Tn = T;   // every record carries T (k_build_records)
     if (!kF32) {
-        int row = 0;
-        if (hash >= 0 && hash < K.g.num_cell) row = hash - (hash / K.g.ny) * K.g.ny;
-        write_record64(rec64, k, K, pos, vel, S, R, p, h, rho, Tn, blanked, tool, row);
+        write_record64(rec64, cand32, k, K, pos, vel, S, R, p, h, rho, Tn, blanked, tool, hash);
     } else {
         write_record32(rec32, cand32, k, K, pos, vel, S, R, p, h, rho, Tn, blanked, tool, hash);
     }

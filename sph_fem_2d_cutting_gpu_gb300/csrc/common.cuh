@@ -110,8 +110,10 @@ __device__ __forceinline__ int case_of_hash(const KConsts &K, int hash) {
 __device__ __forceinline__ bool flag_is_one(double v) {            // v == 1.
     return __double_as_longlong(v) == 0x3FF0000000000000LL;
 }
+// (From the two words: the compiler turns a test of the 64 bits, shifted, into the
+// double compare.)
 __device__ __forceinline__ bool flag_nonzero(double v) {           // v != 0. (NaN counts as non-zero)
-    return (__double_as_longlong(v) << 1) != 0;
+    return ((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) != 0;
 }
 __device__ __forceinline__ bool is_nan_or_inf(double v) {          // isnan(v) || isinf(v)
     return (__double_as_longlong(v) & 0x7FF0000000000000LL) == 0x7FF0000000000000LL;

@@ -64,7 +64,6 @@ __device__ __forceinline__ int cand_row_diff(int gj, float cy) {
 // blocks, 40 entries take 120 KB of shared memory per SM, 48 take 144 KB and
 // were 1.3 % slower (44: the same as 48).
 constexpr int kChunk32 = 40;
-constexpr int kChunk64 = 48;   // FP64: 48 x 256 threads x 4 B = the 48 KB static limit
 
 // Sums of the fused FP32 pair loop, each Kahan-compensated.  The epilogue needs
 // the stress divergence and the artificial viscosity only through the

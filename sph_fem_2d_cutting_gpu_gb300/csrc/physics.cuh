@@ -5,7 +5,7 @@
 
 #include <cfloat>
 
-#include "common.cuh"
+#include "fix64.cuh"
 
 namespace sphfem {
 
@@ -100,6 +100,32 @@ __device__ __forceinline__ double solve_secant(const sph_joco_constants &jc, dou
     }
 }
 
+// Whether the FP64 test svm < sigma_Y of the return mapping below is certain to
+// hold, from FP32 evaluations of both sides with margins far above their errors
+// (about 1e-6; every NaN and every constant outside the margins' premises gives
+// false): an elastic particle then needs nothing else of the three pow() calls
+// that the yield stress costs on the FP64 pipe.  The von Mises stress is formed
+// from the deviatoric differences, which the pressure does not enter; `pf`
+// bounds the reference's own cancellation.  The flow stress is discontinuous at
+// eps_dot = 1 (plasticity.cuh:29-33).
+__device__ __forceinline__ bool surely_elastic(const KConsts &K, dbl4 S, double p, double eps_pl, double eps_pl_dot,
+                                               double T) {
+    const JcF32 &j = K.f.jc;
+    const float a = float_trunc(S.x), b = float_trunc(S.z), c = float_trunc(S.w), d = float_trunc(S.y);
+    const float pf = float_trunc(p);
+    const float ab = a - b, bc = b - c, ca = c - a;
+    const float svm = sqrtf(0.5f * (ab * ab + bc * bc + ca * ca) + 3.f * d * d + 1e-12f * pf * pf) +
+                      1e-5f * (fabsf(a) + fabsf(b) + fabsf(c) + fabsf(d));
+    const float theta = fminf(float_trunc(T - K.c.joco.Tref) * j.inv_dT, 1.f);
+    const float term_c = 1.f - powf(theta, j.m) - 1e-5f;
+    const float eps_dot = float_trunc(eps_pl_dot) * j.inv_epsdot_ref;
+    if (!(eps_dot < 1e30f) || fabsf(eps_dot - 1.f) < 1e-3f || !(j.B >= 0.f)) return false;
+    const float bp = j.B * powf(float_trunc(eps_pl), j.n), cl = j.C * logf(fmaxf(eps_dot, 1.f));
+    const float term_a = j.A + bp - 1e-5f * (fabsf(j.A) + bp);
+    const float term_b = (eps_dot > 1.f ? 1.f + cl : powf(1.f + eps_dot, j.C)) - 1e-5f * (1.f + fabsf(cl));
+    return term_a > 0.f && term_b > 0.f && term_c > 0.f && svm * 1.0001f < term_a * term_b * term_c * 0.9999f;
+}
+
 // ---- actions_gpu.cu:689-754 do_plasticity_johnson_cook (one particle) --------
 // Reads/writes the particle's S, eps_pl, eps_pl_dot, T, blanked.  Returns
 // status bits.  `iters_out` receives the secant iteration count (0 if elastic).
@@ -110,6 +136,11 @@ __device__ __forceinline__ uint32_t plasticity_one(const KConsts &K, double dt, 
                                                    int *iters_out) {
     const sph_joco_constants &jc = K.c.joco;
     const double mu = K.c.phys.G;
+    *iters_out = 0;
+    if (!kF32Yield && surely_elastic(K, S, p, eps_pl, eps_pl_dot, T)) {
+        eps_pl_dot = 0.;
+        return 0u;
+    }
     double Sxx = S.x, Syy = S.z, Szz = S.w, Sxy = S.y;
     double norm_Strial = sqrtf_d(Sxx * Sxx + Syy * Syy + Szz * Szz + 2. * Sxy * Sxy);
     double cxx = Sxx - p, cyy = Syy - p, czz = Szz - p, cxy = Sxy;
@@ -117,7 +148,6 @@ __device__ __forceinline__ uint32_t plasticity_one(const KConsts &K, double dt, 
     double term_c = jc_term_c(jc, T);
     double sigma_Y = kF32Yield ? sigma_yield_tc_f32(jc, eps_pl, eps_pl_dot, term_c)
                                : sigma_yield_tc(jc, eps_pl, eps_pl_dot, term_c);
-    *iters_out = 0;
     if (svm < sigma_Y) {
         eps_pl_dot = 0.;
         return 0u;
@@ -165,10 +195,10 @@ __device__ __forceinline__ uint32_t fric_heat_one(const KConsts &K, double dt, c
                                                   double2 ft, double2 nrm, double2 fc, double rho, double eps_pl,
                                                   int seg, int n_seg, double &T, double &blanked,
                                                   double *__restrict__ fric_heat, const WearAcc &wear) {
+    if (seg < 0 || seg >= n_seg) return 0u;
     if (blanked == 1.) return 0u;
     if (eps_pl > 20.) return 0u;
     double f_fric_mag = sqrtf_d(ft.x * ft.x + ft.y * ft.y);
-    if (seg < 0 || seg >= n_seg) return 0u;
     const double partition_wp = K.c.tool.beta;
     double vdx = vel.x - vel_tool[0], vdy = vel.y - vel_tool[1];
     double vdn = vdx * nrm.x + vdy * nrm.y;

@@ -161,10 +161,20 @@ struct WearDev {
     double A, B, C, D;                   // wear constants (constants_structs.h:113-119)
 };
 
+// The same entries beside the FP64 records, for a test that only sorts out
+// candidates that cannot be in the support: kCandSpecial marks the ones that it
+// may not sort out -- a non-finite record, or coordinates further than 4 cells
+// from the cell (positions moved since the sort), where FP32 is too coarse.
+constexpr int kCandSpecial = kCandNonFinite;
+__device__ __forceinline__ float2 cand_pack64(float xr, float yr, float cell, int flags) {
+    const bool near = fabsf(xr) <= 4.f * cell && fabsf(yr) <= 4.f * cell;
+    return cand_pack(xr, yr, near ? flags : flags | kFlagNonFinite);
+}
+
 struct StepScratch {
     dbl4 *rec64;      // [N][4] FP64 records
     float4 *rec32;       // [N][4] FP32 records
-    float2 *cand32;      // [N] candidate entries of the FP32 records (cand_pack)
+    float2 *cand32;      // [N] candidate entries of the records (cand_pack, cand_pack64)
     double2 *pos_init, *vel_init;   // leap_frog snapshots (staged path)
     dbl4 *S_init;
     double *rho_init, *T_init;
