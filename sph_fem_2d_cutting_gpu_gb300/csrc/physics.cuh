@@ -5,7 +5,7 @@
 
 #include <cfloat>
 
-#include "fix64.cuh"
+#include "fix64_math.cuh"
 
 namespace sphfem {
 
@@ -38,23 +38,24 @@ __device__ __forceinline__ void cubic_spline(double xij, double yij, double hi, 
 // Term_C depends only on the temperature, which is constant during one return
 // mapping, so callers may pass it precomputed (identical arithmetic).
 __device__ __forceinline__ double jc_term_c(const sph_joco_constants &jc, double t) {
-    double theta = (t - jc.Tref) / (jc.Tmelt - jc.Tref);
+    double theta = fix_div(t - jc.Tref, jc.Tmelt - jc.Tref);
     if (theta > 1.) theta = 1.;
-    return 1.0 - pow(theta, jc.m);
+    return 1.0 - fix_pow(theta, jc.m);
+}
+
+// eps_dot = eps_pl_dot / eps_dot_ref
+__device__ __forceinline__ double sigma_yield_rate(const sph_joco_constants &jc, double eps_pl, double eps_dot,
+                                                   double term_c) {
+    const double Term_A = jc.A + jc.B * fix_pow(eps_pl, jc.n);
+    double Term_B = 1.;
+    if (eps_dot > 1.0) Term_B = 1.0 + jc.C * fix_log_above_1(eps_dot);
+    else if (flag_nonzero(eps_dot)) Term_B = pow_general(1.0 + eps_dot, jc.C);
+    return Term_A * Term_B * term_c;
 }
 
 __device__ __forceinline__ double sigma_yield_tc(const sph_joco_constants &jc, double eps_pl, double eps_pl_dot,
                                                  double term_c) {
-    double Term_A = jc.A + jc.B * pow(eps_pl, jc.n);
-    double Term_B;
-    double eps_dot = eps_pl_dot / jc.eps_dot_ref;
-    if (eps_dot > 1.0) Term_B = 1.0 + jc.C * log(eps_dot);
-    else Term_B = pow((1.0 + eps_dot), jc.C);
-    return Term_A * Term_B * term_c;
-}
-
-__device__ __forceinline__ double sigma_yield(const sph_joco_constants &jc, double eps_pl, double eps_pl_dot, double t) {
-    return sigma_yield_tc(jc, eps_pl, eps_pl_dot, jc_term_c(jc, t));
+    return sigma_yield_rate(jc, eps_pl, fix_div(eps_pl_dot, jc.eps_dot_ref), term_c);
 }
 
 // Same flow stress with the rate/strain terms in FP32 (powf/logf).  Used by the
@@ -77,10 +78,12 @@ __device__ __forceinline__ double solve_secant(const sph_joco_constants &jc, dou
                                               double norm_Strial, double eps_pl_init, double term_c, double delta_t,
                                               double mu, int *iters, int max_iter = 100) {
     const double s23 = sqrt(2.0 / 3.0);
+    const double rate = s23 / delta_t, rate_rel = rate / jc.eps_dot_ref;
     auto opt_fun = [&](double dl) {
-        double eq = eps_pl_init + s23 * fmax(dl, 0.);
-        double eqd = s23 * fmax(dl, 0.) / delta_t;
-        double sY = kF32Yield ? sigma_yield_tc_f32(jc, eq, eqd, term_c) : sigma_yield_tc(jc, eq, eqd, term_c);
+        const double dlp = fmax(dl, 0.);
+        double eq = eps_pl_init + s23 * dlp;
+        double sY = kF32Yield ? sigma_yield_tc_f32(jc, eq, rate * dlp, term_c)
+                              : sigma_yield_rate(jc, eq, rate_rel * dlp, term_c);
         return norm_Strial - 2 * mu * dl - s23 * sY;
     };
     double delta_lambda = init;
@@ -90,9 +93,9 @@ __device__ __forceinline__ double solve_secant(const sph_joco_constants &jc, dou
         double g = opt_fun(delta_lambda);
         double delta_lambda_1 = delta_lambda * 1.01;
         double g_1 = opt_fun(delta_lambda_1);
-        double slope = (g - g_1) / (delta_lambda - delta_lambda_1);
+        // g / slope, slope = (g - g_1) / (dl - dl_1)
         delta_lambda_old = delta_lambda;
-        delta_lambda = delta_lambda - g / slope;
+        delta_lambda = delta_lambda - fix_div(g * (delta_lambda - delta_lambda_1), g - g_1);
         if (delta_lambda < 0.) delta_lambda = -0.1 * delta_lambda;
         if (fabs(delta_lambda - delta_lambda_old) < tol) { *iters = iter + 1; return delta_lambda; }
         if (iter > max_iter) { *iters = -(iter + 1); return delta_lambda; }
@@ -165,19 +168,20 @@ __device__ __forceinline__ uint32_t plasticity_one(const KConsts &K, double dt, 
     // reference multiplies in float (actions_gpu.cu:728-729)
     const float inc = sqrtf((float)(2.0 / 3.0)) * fmaxf((float)delta_lambda, 0.f);
     double eps_pl_new = eps_pl + (double)inc;
-    double eps_pl_dot_new = (double)inc / dt;
+    double eps_pl_dot_new = fix_div((double)inc, dt);
     double eps_old = eps_pl;
     eps_pl = eps_pl_new;
     eps_pl_dot = eps_pl_dot_new;
-    S.x = Sxx - Sxx / norm_Strial * delta_lambda * 2. * mu;
-    S.z = Syy - Syy / norm_Strial * delta_lambda * 2. * mu;
-    S.w = Szz - Szz / norm_Strial * delta_lambda * 2. * mu;
-    S.y = Sxy - Sxy / norm_Strial * delta_lambda * 2. * mu;
+    const double back = fix_div(2. * mu * delta_lambda, norm_Strial);
+    S.x = Sxx - Sxx * back;
+    S.z = Syy - Syy * back;
+    S.w = Szz - Szz * back;
+    S.y = Sxy - Sxy * back;
     if (K.c.trml_wp.tq != 0.) {
         double delta_eps_pl = eps_pl_new - eps_old;
         double sY = kF32Yield ? sigma_yield_tc_f32(jc, eps_pl_new, eps_pl_dot_new, term_c)
                               : sigma_yield_tc(jc, eps_pl_new, eps_pl_dot_new, term_c);
-        T += K.c.trml_wp.tq / (K.c.trml_wp.cp * rho) * delta_eps_pl * sY;
+        T += fix_div(K.c.trml_wp.tq * delta_eps_pl * sY, K.c.trml_wp.cp * rho);
     }
     if (T > jc.Tmelt) {
         T = jc.Tmelt;

@@ -1,14 +1,20 @@
-"""Integer model of csrc/fix64.cuh's reciprocals and rounded product, against exact rationals.
+"""Integer model of csrc/fix64.cuh's reciprocals and rounded product, against exact rationals,
+and of csrc/fix64_math.cuh's log2 and exp2 (with the tables read from it), against 60 digits.
 
 The device functions restated step by step on Python integers: the third-order Newton
 reciprocal of a 53-bit mantissa stays within the stated 2^5 units of 2^114 / M from every
 FP32 start within two units in the last place, fix_recip_rn gives the correctly rounded
 double 1 / x, and fix_mul_rn the correctly rounded double product with a float."""
 import random
+import re
 import struct
+from decimal import Decimal, getcontext
 from fractions import Fraction
+from pathlib import Path
 
 import pytest
+
+MATH = Path(__file__).resolve().parents[1] / "sph_fem_2d_cutting_gpu_gb300" / "csrc" / "fix64_math.cuh"
 
 M64 = (1 << 64) - 1
 
@@ -88,3 +94,57 @@ def test_reciprocal_and_product(ulps):
         r = f32(rng.uniform(1, 2) * 2.0 ** rng.randint(-15, 3))
         m2, e2 = mul_rn(m, e, r)
         assert Fraction(m2) * Fraction(2) ** e2 == Fraction((1 / x) * r)
+
+
+def table(name):
+    body = re.search(name + r"\[\d+\] = \{(.*?)\};", MATH.read_text(), re.S).group(1)
+    return [int(x.rstrip("ul"), 0) for x in re.findall(r"0x[0-9a-f]+ull|\d+", body)]
+
+
+def mul_hi(a, b):
+    al, ah, bl, bh = a & 0xFFFFFFFF, a >> 32, b & 0xFFFFFFFF, b >> 32
+    return ah * bh + ((ah * bl) >> 32) + ((al * bh) >> 32)
+
+
+def umulhi(a, b):
+    return (a * b) >> 32
+
+
+def log2_frac(m, K, T):
+    i = (m >> 56) & 0x7F
+    S = ((((m >> 9) * K[i]) & M64) - (1 << 63)) << 7
+    assert 0 <= S <= M64
+    s = S >> 32
+    h = 0x1C71C71C - (umulhi(s, 0x1999999A) >> 6)
+    for c in (0x20000000, 0x24924925, 0x2AAAAAAB):
+        h = c - (umulhi(s, h) >> 6)
+    H = 0x3333333333333333 - (mul_hi(S, h << 32) >> 6)
+    for c in (0x4000000000000000, 0x5555555555555555, 0x8000000000000000, M64):
+        H = c - (mul_hi(S, H) >> 6)
+    return T[i] + (mul_hi(mul_hi(S, H), 0xB8AA3B295C17F0BC) >> 5)
+
+
+def exp2_frac(F, E):
+    T = E[F >> 58]
+    w = mul_hi((F << 6) & M64, 0xB17217F7D1CF79AC)
+    v = w >> 32
+    h = 0x5B05B0 + (umulhi(v, 0xD00D0) >> 6)
+    for c in (0x2222222, 0xAAAAAAB):
+        h = c + (umulhi(v, h) >> 6)
+    H = 0x2AAAAAAAAAAAAAAB + (mul_hi(w, h << 32) >> 6)
+    H = 0x8000000000000000 + (mul_hi(w, H) >> 6)
+    return T + (mul_hi(T, w + mul_hi(w, mul_hi(w, H) >> 6)) >> 6)
+
+
+def test_log2_exp2():
+    getcontext().prec = 60
+    K, T, E = table("kLog2K"), table("kLog2T"), table("kExp2T")
+    two = Decimal(2)
+    rng = random.Random(11)
+    for k in range(6000):
+        m = (1 << 52) + k if k < 1000 else (1 << 53) - 1 - k if k < 2000 else rng.getrandbits(52) | (1 << 52)
+        f = log2_frac(m << 11, K, T)
+        assert f <= M64 and abs(f - (Decimal(m) / (1 << 52)).ln() / two.ln() * two ** 64) < 2
+        F = k if k < 1000 else M64 - k if k < 2000 else rng.getrandbits(64)
+        y = exp2_frac(F, E)
+        assert (1 << 63) <= y <= M64 and abs(y - two ** (Decimal(F) / (1 << 64)) * two ** 63) < 40
