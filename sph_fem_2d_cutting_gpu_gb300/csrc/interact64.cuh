@@ -41,7 +41,7 @@ struct Sums64 {
 // Plain FP64 sums over every active candidate j = first, first + kLanes64, ... of
 // the stencil's columns (the reference's body with cubic_spline's zero weights,
 // kernels.cuh:37-39).
-__device__ __noinline__ void sums64_plain(Sums64 &out, int k, int sub, const int32_t *__restrict__ offsets,
+static __device__ __noinline__ void sums64_plain(Sums64 &out, int k, int sub, const int32_t *__restrict__ offsets,
                                           const dbl4 *__restrict__ rec, int hash, int nx, int ny, int R, double inv_wdp,
                                           double eta2, double beta, bool tool_i, bool thermal) {
     const dbl4 i0 = rec[4 * k + 0], i1 = rec[4 * k + 1], i2 = rec[4 * k + 2], i3 = rec[4 * k + 3];

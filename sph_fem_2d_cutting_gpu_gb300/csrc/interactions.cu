@@ -50,7 +50,7 @@ void interact_variant_shape(int v, int *block, int *min_blocks, int *staged, int
     *lanes = kInteractVariants[v][3];
 }
 
-// Threads per block of the FP64 per-particle kernels: the largest of 256, 128,
+// Threads per block of the per-particle kernels with FP64 work: the largest of 256, 128,
 // 64 that still gives every SM two blocks, else 32.  The FP64 pipe is narrow, so
 // a small system (the reference's own cases are 7k-12k particles) must spread
 // over all SMs rather than fill a few.  Results do not depend on it: each
@@ -75,44 +75,64 @@ int fp64_block(int N) {
 // cut-off, blanked neighbours included), W2 = 4 / (h^4 pi) exp(-|r|^2 / h^2)
 // (kernels.cuh:67-84).  Reads the predicted state from the FP64 records; the
 // block's columns are contiguous slot ranges as in the neighbour sums.
-template <int kB>
-__global__ void __launch_bounds__(kB) k_heat_pse64(int N, KConsts K, const int32_t *__restrict__ offsets,
-                                                       const dbl4 *__restrict__ rec,
-                                                       const int32_t *__restrict__ hashes, double *__restrict__ T_t) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= N) return;
-    const dbl4 i3 = rec[4 * k + 3];
+// Bound by the FP64 pipe and, on the reference's own size, by the latency of its
+// chains: the Gaussian and its product with the volume run on the integer pipes
+// (6 FP64 operations a candidate instead of about 26) and kPseLanes lanes share a
+// particle.  7,355 particles: 92 -> 14 us; 121,620: 471 -> 110 us; 490,072: 1.45 -> 0.42 ms.
+constexpr int kPseLanes = 8;
+// The term of a candidate whose numbers the mantissa form does not take.
+static __device__ __noinline__ double pse_weight_general(double rr2, double inv_h2, double vol) {
+    return exp(-rr2 * inv_h2) * vol;
+}
+__global__ void __launch_bounds__(128) k_heat_pse64(int N, KConsts K, const int32_t *__restrict__ offsets,
+                                                    const dbl4 *__restrict__ rec,
+                                                    const int32_t *__restrict__ hashes, double *__restrict__ T_t) {
+    const int k = (int)(blockIdx.x * 128u + threadIdx.x) / kPseLanes, sub = (int)threadIdx.x % kPseLanes;
+    const int kk = min(k, N - 1);
+    const dbl4 i0 = rec[4 * kk + 0], i2 = rec[4 * kk + 2], i3 = rec[4 * kk + 3];
     const int fi = (int)__double_as_longlong(i3.w);
-    if (fi & kFlagBlanked) return;
-    const dbl4 i0 = rec[4 * k + 0], i2 = rec[4 * k + 2];
-    const double xi = i0.x, yi = i0.y, hi = i2.z, Ti = i3.z;
+    const bool live = k < N && !(fi & kFlagBlanked);
+    const double xi = i0.x, yi = i0.y, Ti = i3.z;
+    const double h2 = i2.z * i2.z;
+    const bool plain = !fix_range(h2);
+    // log2(e) / h^2
+    const Fix64 ch = fix_norm(Fix64{0xb8aa3b295c17f0bcull, -63} * fix_recip(plain ? 1. : h2));
+    double sum = 0.;
+    const int hash = hashes[kk];
+    const sph_geom_constants &g = K.g;
+    if (live && hash >= 0 && hash < g.num_cell) {
+        const int gi = hash / g.ny, gj = hash - gi * g.ny;
+        int ii = max(gi - 2, 0);
+        const int ii1 = min(gi + 3, g.nx), lo_j = max(gj - 2, 0), hi_j = min(gj + 3, g.ny);
+        int j = __ldg(offsets + ii * g.ny + lo_j) + sub, j1 = __ldg(offsets + ii * g.ny + hi_j);
+        while (true) {   // every kPseLanes-th candidate of the columns' ranges, end to end
+            while (j >= j1 && ++ii < ii1) {
+                j += __ldg(offsets + ii * g.ny + lo_j) - j1;
+                j1 = __ldg(offsets + ii * g.ny + hi_j);
+            }
+            if (j >= j1) break;
+            const dbl4 n0 = rec[4 * j + 0], n3 = rec[4 * j + 3];
+            const double ex = n0.x - xi, ey = n0.y - yi;
+            const double rr2 = ex * ex + ey * ey;
+            double w;
+            const Fix64 y = fix_norm(fix_of(rr2) * ch);
+            if (plain || !fix_range(n3.y) || (uint32_t)__double2hiint(rr2) >= 0x7ff00000u) {
+                w = pse_weight_general(rr2, 1. / h2, n3.y);
+            } else {
+                w = y.e + 63 > 9 ? 0. : fix_double(fix_exp2(y, true) * fix_of(n3.y));
+            }
+            sum += (n3.z - Ti) * w;
+            j += kPseLanes;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 1; o < kPseLanes; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (!live || sub != 0) return;
     // the reference binds the tool flags (doubles) for N ints, half the array
     // (interactions_gpu.cu:448): from index N/2 on its fetch reads zero
     const double alpha = ((fi & kFlagTool) && k < N / 2) ? K.c.trml_tool_sph.alpha : K.c.trml_wp.alpha;
-    const double h2 = hi * hi, h4 = h2 * h2;
-    const double c = 4. / (h4 * kRigidPi);
-    const double inv_h2 = 1. / h2;
-    double sum = 0.;
-    const int hash = hashes[k];
-    const sph_geom_constants &g = K.g;
-    if (hash >= 0 && hash < g.num_cell) {
-        const int gi = hash / g.ny, gj = hash - gi * g.ny;
-        const int lo_i = max(gi - 2, 0), hi_i = min(gi + 3, g.nx);
-        const int lo_j = max(gj - 2, 0), hi_j = min(gj + 3, g.ny);
-        for (int ii = lo_i; ii < hi_i; ii++) {
-            const int j1 = __ldg(offsets + ii * g.ny + hi_j);
-            for (int j = __ldg(offsets + ii * g.ny + lo_j); j < j1; j++) {
-                const dbl4 n0 = rec[4 * j + 0], n3 = rec[4 * j + 3];
-                const double xij = xi - n0.x, yij = yi - n0.y;
-                // |r|^2 / h^2 as a product with 1/h^2; n3.y = m / rho_j.  Both differ
-                // from the reference's sqrt-square, division and m / rho_j order by
-                // rounding only (relative 1e-16 per term).
-                const double w2 = c * exp(-(xij * xij + yij * yij) * inv_h2);
-                sum += (n3.z - Ti) * w2 * n3.y;
-            }
-        }
-    }
-    T_t[k] = alpha * sum;
+    T_t[k] = alpha * (fix_div(4., h2 * h2 * kRigidPi) * sum);
 }
 
 // FP32-compensated form of the PSE sum over the FP32 records: positions as
@@ -169,12 +189,7 @@ void launch_heat_pse(cudaStream_t s, int N, const KConsts &K, const int32_t *off
         k_heat_pse32<<<div_up(N, tb), tb, 0, s>>>(N, K, offsets, W.rec32, B.hash, B.T_t);
         return;
     }
-    switch (fp64_block(N)) {
-        case 32: k_heat_pse64<32><<<div_up(N, 32), 32, 0, s>>>(N, K, offsets, W.rec64, B.hash, B.T_t); break;
-        case 64: k_heat_pse64<64><<<div_up(N, 64), 64, 0, s>>>(N, K, offsets, W.rec64, B.hash, B.T_t); break;
-        case 128: k_heat_pse64<128><<<div_up(N, 128), 128, 0, s>>>(N, K, offsets, W.rec64, B.hash, B.T_t); break;
-        default: k_heat_pse64<256><<<div_up(N, 256), 256, 0, s>>>(N, K, offsets, W.rec64, B.hash, B.T_t); break;
-    }
+    k_heat_pse64<<<div_up((int64_t)N * kPseLanes, 128), 128, 0, s>>>(N, K, offsets, W.rec64, B.hash, B.T_t);
 }
 
 void launch_interactions32_fused(cudaStream_t s, int N, const KConsts &K, const int32_t *offsets,
