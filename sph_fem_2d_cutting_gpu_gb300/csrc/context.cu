@@ -519,10 +519,11 @@ int issue_fused_body(sph_ctx *ctx, int64_t &n, int w, cudaEvent_t *ev = nullptr)
         n += 1;
     }
     if (ev) CK(cudaEventRecord(ev[4], s));
-    CK(cudaMemsetAsync(ctx->X.counts, 0, sizeof(int32_t) * (size_t)(ctx->K.g.num_cell + 1), s));
+    // the next step's histogram and, behind it, the contact queue's length
+    CK(cudaMemsetAsync(ctx->X.counts, 0, sizeof(int32_t) * (size_t)(ctx->K.g.num_cell + 2), s));
     if (f32) launch_step_tail(s, N, ctx->K, B32, ctx->seg, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status, true);
     else launch_step_tail(s, N, ctx->K, B, ctx->seg, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status, true);
-    n += ctx->has_tool ? 3 : 1;   // with the FEM tool: the segment y-bins and the contact pass, then the tail
+    n += ctx->has_tool ? 3 : 1;   // with the FEM tool: the segment y-bins, then the tail and the contact queue
     if (ev) CK(cudaEventRecord(ev[5], s));
     CK_LAUNCH();
     return SPH_OK;
@@ -738,7 +739,7 @@ int ctx_begin(const sph_constants *c, const sph_grid_params *g, const sph_geom_c
     DALLOC(ctx->F.p, N); DALLOC(ctx->F.R, N); DALLOC(ctx->F.S_der, N); DALLOC(ctx->F.v_der, N); DALLOC(ctx->F.idx, N);
     const int nc = ctx->K.g.num_cell;
     DALLOC(ctx->X.key, N); DALLOC(ctx->X.arrival, N); DALLOC(ctx->X.slots, N); DALLOC(ctx->X.hash_next, N);
-    DALLOC(ctx->X.counts, (size_t)nc + 1); DALLOC(ctx->X.offsets, (size_t)nc + 2);
+    DALLOC(ctx->X.counts, (size_t)nc + 2); DALLOC(ctx->X.offsets, (size_t)nc + 2);
     DALLOC(ctx->X.block_sums, (size_t)scan_blocks(nc) + 1);
     DALLOC(ctx->X.cell_start, nc); DALLOC(ctx->X.cell_end, nc);
     if (precision == SPH_PREC_FP32K) {

@@ -60,9 +60,9 @@ struct SortScratch {
     int32_t *hash_next;  // [N] raw hash taken by the histogram pass (the fused step keeps the
                          //     visible hash array as the reference leaves it until the next sort)
     int32_t *arrival;    // [N] arrival slot inside its cell (atomic counter value)
-    int32_t *counts;     // [num_cell+1] particles per cell (last = out-of-grid bucket)
+    int32_t *counts;     // [num_cell+1] particles per cell (last = out-of-grid bucket), then the contact queue's length
     int32_t *offsets;    // [num_cell+2] exclusive scan of counts
-    int32_t *slots;      // [N] particle ids grouped by cell, arbitrary order inside a cell
+    int32_t *slots;      // [N] particle ids grouped by cell, arbitrary order inside a cell; the tail's contact queue
     int32_t *block_sums; // scan partials
     int32_t *cell_start, *cell_end;   // grid_gpu_green m_cell_start / m_cell_end
 };

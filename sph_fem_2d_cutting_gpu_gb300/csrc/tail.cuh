@@ -320,9 +320,8 @@ __device__ __forceinline__ void contact_s2_one(const KConsts &K, double dt, cons
 }
 
 // ---- the FEM tool's contact of the fused step: actions_gpu.cu:423-617 (s1 + s2) -----------------------
-// Its own pass before the tail: the contact search's registers would otherwise
-// hold down the occupancy of the memory-bound tail for every particle, although
-// only the particles near a tool reach it.  The tail that follows sees the
+// One particle by one thread: a stage of the persistent step, before its tail (the
+// step of launches searches with a warp, below).  The tail that follows sees the
 // contact's results (forces, segment id, blanking, temperature) in memory, in the
 // order of the reference's step.
 // SF: SortedFields (FP64 state) or SortedFields32 (the compact state of FP32K
@@ -382,14 +381,15 @@ __device__ __forceinline__ void contact_fem_one(int i, const KConsts &K, const S
     if (st) set_status(status, st);
 }
 
-// ---- the same contact with the few particles at the tool searched by their whole warp --------------
+// ---- the same contact with the few particles at the tool searched by a warp each -------------------
 // contact_fem_one's results, bit for bit: each segment test and distance is the
 // reference's expression; the loops over a case's segments are spread over the
 // 32 lanes (lane k takes segments k, k + 32, ...) and combined in the reference's
 // order of preference -- the crossing count as a sum, the nearest segment as the
 // smallest (distance, index), the first matching neighbour as the smallest index.
-// Called by every lane of every warp (no lane may have left): 1-D blocks, a
-// multiple of 32 threads.  Needs the y-bins and SegGeo (k_seg_bins).
+// The particles come from the tail's queue (contact_probe), one to a warp: at the
+// tool's tip they are neighbours in cell order, and a warp that searched for each
+// of its own lanes in turn held up the step.
 constexpr unsigned kFullMask = 0xffffffffu;
 
 __device__ __forceinline__ void warp_argmin(double &d, int &idx) {
@@ -495,60 +495,45 @@ __device__ __forceinline__ int shortest_distance_lanes(double2 qp, double &dN, d
     return s_near;
 }
 
+// Whether particle i (not blanked) can be inside its case's tool and has to be
+// searched for; if not, it is out of contact and its contact state is cleared.
 template <class SF>
-__device__ __forceinline__ void contact_fem_warp(int i, int N, const KConsts &K, const SF &A, const SegDev &seg,
+__device__ __forceinline__ bool contact_probe(int i, const KConsts &K, const SF &A, const SegDev &seg,
+                                              const ToolDev *__restrict__ tool) {
+    const double2 pos = A.pos[i];
+    const int c = case_of_hash(K, A.hash[i]);
+    const ToolDev &tc = tool[c];
+    if (contact_near(pos, case_segments(seg, tc, c), tc)) {
+        const double ddx = pos.x - tc.tl_point_ref[0], ddy = pos.y - tc.tl_point_ref[1];
+        // right of every segment of its y-bin a particle crosses none (no scan needed)
+        if (order_key(pos.x) <= seg.bin_xkey[c * kSegBins + seg_bin_of(pos.y, tc.bin_y0, tc.bin_scale)] &&
+            sqrt(ddx * ddx + ddy * ddy) < 1.05 * tc.ref_dist)
+            return true;
+    }
+    put(A.ft[i], make_double2(0., 0.));
+    put(A.n[i], make_double2(0., 0.));
+    A.on_seg[i] = -1;
+    put(A.fc[i], make_double2(0., 0.));
+    return false;
+}
+
+// The contact of a probed particle by a whole warp (i is the same in every lane);
+// lane 0 writes the results.
+template <class SF>
+__device__ __forceinline__ void contact_fem_warp(int i, const KConsts &K, const SF &A, const SegDev &seg,
                                                  const ToolDev *__restrict__ tool,
                                                  const double *__restrict__ T_nodes, uint32_t *status) {
     const int lane = (int)(threadIdx.x & 31u);
-    const bool live = i < N && !flag_is_one(A.blanked[i]);
-    double2 pos = make_double2(0., 0.);
-    int c = 0;
-    bool near = false, probe = false;
-    if (live) {
-        pos = A.pos[i];
-        c = case_of_hash(K, A.hash[i]);
-        const ToolDev &tc = tool[c];
-        near = contact_near(pos, case_segments(seg, tc, c), tc);
-        if (!near) {   // out of contact: zeros, no FP64 work
-            put(A.ft[i], make_double2(0., 0.));
-            put(A.n[i], make_double2(0., 0.));
-            A.on_seg[i] = -1;
-            put(A.fc[i], make_double2(0., 0.));
-        } else {
-            const double ddx = pos.x - tc.tl_point_ref[0], ddy = pos.y - tc.tl_point_ref[1];
-            // right of every segment of its y-bin a particle crosses none (no scan needed)
-            probe = sqrt(ddx * ddx + ddy * ddy) < 1.05 * tc.ref_dist &&
-                    order_key(pos.x) <= seg.bin_xkey[c * kSegBins + seg_bin_of(pos.y, tc.bin_y0, tc.bin_scale)];
-        }
-    }
-    // the ray casting of each probing lane, by the warp
-    int inside = 0;
-    for (unsigned pend = __ballot_sync(kFullMask, probe); pend; pend &= pend - 1) {
-        const int src = __ffs(pend) - 1;
-        const double2 qp = make_double2(__shfl_sync(kFullMask, pos.x, src), __shfl_sync(kFullMask, pos.y, src));
-        const int cc = __shfl_sync(kFullMask, c, src);
-        const int cr = __reduce_add_sync(kFullMask, crossings_lanes(qp, case_segments(seg, tool[cc], cc), tool[cc], lane));
-        if (lane == src) inside = cr & 1;
-    }
-    // the nearest segment of each lane inside the tool, by the warp
+    const double2 pos = A.pos[i];
+    const int c = case_of_hash(K, A.hash[i]);
+    const ToolDev &tc = tool[c];
+    const SegDev cs = case_segments(seg, tc, c);
+    const int inside = __reduce_add_sync(kFullMask, crossings_lanes(pos, cs, tc, lane)) & 1;
     int seg_no = -1;
     double gN = 0.;
     double2 n_ = make_double2(0., 0.);
-    for (unsigned pend = __ballot_sync(kFullMask, inside != 0); pend; pend &= pend - 1) {
-        const int src = __ffs(pend) - 1;
-        const double2 qp = make_double2(__shfl_sync(kFullMask, pos.x, src), __shfl_sync(kFullMask, pos.y, src));
-        const int cc = __shfl_sync(kFullMask, c, src);
-        double dN;
-        double2 nr;
-        const int r = shortest_distance_lanes(qp, dN, nr, case_segments(seg, tool[cc], cc), lane);
-        if (lane == src) {
-            seg_no = r;
-            gN = dN;
-            n_ = nr;
-        }
-    }
-    if (!near) return;
-    const ToolDev &tc = tool[c];
+    if (inside) seg_no = shortest_distance_lanes(pos, gN, n_, cs, lane);
+    if (lane != 0) return;
     double2 fc = d2(A.fc[i]), ft = d2(A.ft[i]), nrm = d2(A.n[i]);
     int on = A.on_seg[i];
     double bl = 0.;
@@ -577,7 +562,7 @@ __device__ __forceinline__ void contact_fem_warp(int i, int N, const KConsts &K,
 // ---- fused tail of the step ----------------------------------------------------------------------
 // The tool's contact for one particle -- kMode 2: rigid tool, update_tool_particles
 // and do_compute_contact_forces (tool_gpu.cu:146-216); kMode 0: no tool, or the
-// FEM tool whose contact k_contact_fem has applied just before -- then
+// FEM tool whose contact has been applied just before -- then
 // do_boundary_conditions, do_boundary_conditions_thermal, do_invalidate
 // (actions_gpu.cu:756-824) and (kNextHash) the next step's compute_hashes and
 // the counting-sort histogram (grid.cu:25-42) on the final state.
