@@ -409,8 +409,7 @@ void launch_invalidate(cudaStream_t s, int N, const SortedFields &A, uint32_t *s
 template <class SF>
 static void step_tail(cudaStream_t s, int N, const KConsts &K, const SF &A, const SegDev &seg, ToolDev *tool,
                       const double *T_nodes, const SortScratch &X, uint32_t *status, bool next_hash) {
-    const int tb = fp64_block(N);   // the contact search is FP64 work: spread small systems over all SMs
-    if (K.has_tool) launch_seg_bins(s, K.n_cases, seg, tool);
+    const int tb = fp64_block(N);   // the rigid contact is FP64 work: spread small systems over all SMs
 #undef GRID
 #define GRID div_up(N, tb), tb, 0, s
     if (K.has_tool) {

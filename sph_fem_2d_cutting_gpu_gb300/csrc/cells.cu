@@ -9,6 +9,7 @@
 // among its cell-mates by original index.  The scan also yields cell_start /
 // cell_end directly.
 #include "cells.cuh"
+#include "fem.cuh"
 
 namespace sphfem {
 
@@ -74,8 +75,12 @@ __global__ void __launch_bounds__(1024) k_scan_top(int32_t *__restrict__ block_s
 // Writes offsets[0..n] (n = num_cell + 1 buckets, offsets[n] = N) and the
 // reference's cell tables: cell_start = first slot or -1 when empty; cell_end
 // = one past the last slot, left untouched for empty cells (stale, as the
-// reference leaves it).
-__global__ void __launch_bounds__(kScanThreads) k_scan_down(const int32_t *__restrict__ counts, int n,
+// reference leaves it).  kTop: block_sums holds the tiles' sums, which every block
+// adds up to its own start; otherwise k_scan_top has scanned them.  The counts,
+// read here for the last time, go back to zero for the next histogram (and with
+// them counts[n], the contact queue's length).
+template <bool kTop>
+__global__ void __launch_bounds__(kScanThreads) k_scan_down(int32_t *__restrict__ counts, int n,
                                                             const int32_t *__restrict__ block_sums,
                                                             int32_t *__restrict__ offsets,
                                                             int32_t *__restrict__ cell_start,
@@ -88,9 +93,18 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const int32_t *__res
     for (int k = 0; k < kScanItems; k++) {
         v[k] = (base + k < n) ? counts[base + k] : 0;
         s += v[k];
+        if (base + k <= n) counts[base + k] = 0;
+    }
+    int start = 0;
+    if (kTop) {
+        int p = 0;
+        for (int b = threadIdx.x; b < (int)blockIdx.x; b += kScanThreads) p += block_sums[b];
+        block_exclusive_scan(p, sw, start);
+    } else {
+        start = block_sums[blockIdx.x];
     }
     int total;
-    int ex = block_exclusive_scan(s, sw, total) + block_sums[blockIdx.x];
+    int ex = block_exclusive_scan(s, sw, total) + start;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
         int c = base + k;
@@ -111,11 +125,15 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const int32_t *__res
 }
 
 // ---- scatter into the cell's slot range (arbitrary order inside the cell) -------------
+// With a FEM tool the threads after the particles' run the nodes' half step
+// (calculate_temp(0.5 dt), independent of the sort).
 __global__ void __launch_bounds__(kBlock) k_scatter(int N, const int32_t *__restrict__ key,
                                                     const int32_t *__restrict__ arrival,
-                                                    const int32_t *__restrict__ offsets, int32_t *__restrict__ slots) {
+                                                    const int32_t *__restrict__ offsets, int32_t *__restrict__ slots,
+                                                    KConsts K, FemDev F, const ToolDev *__restrict__ tool) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) scatter_one(i, key, arrival, offsets, slots);
+    else if (i - N < F.n_nodes) fem_half_one(i - N, K, F, tool);
 }
 
 __global__ void __launch_bounds__(kBlock) k_rank(int N, const int32_t *__restrict__ key,
@@ -244,16 +262,20 @@ __global__ void __launch_bounds__(kBlock) k_build_records(int N, KConsts K, Sort
 // (actions_gpu.cu:234-278) + the neighbour record of the predicted state.
 // The sorted arrays B keep the start-of-step state (the reference's *_init
 // snapshots); the predicted values live only in the records and in p / R.
-// hash_src: the hashes the histogram pass took (compute_hashes of this step).
+// The hashes are those the histogram pass took (compute_hashes of this step).
+// One thread per slot of the counting sort: it ranks its particle inside the cell
+// (rank_of) and writes to the sorted position, which lies in the same cell, so a
+// pass over the permutation and a launch are saved: 12,000 particles, sort and
+// reorder 41 -> 26 us.
 template <bool kF32>
-__global__ void __launch_bounds__(kBlock) k_gather_fused(int N, const int32_t *__restrict__ perm, KConsts K,
+__global__ void __launch_bounds__(kBlock) k_gather_fused(int N, SortScratch X, KConsts K,
                                                          SortedFields A, SortedFields B, FixedFields F,
-                                                         const int32_t *__restrict__ hash_src,
                                                          dbl4 *__restrict__ rec64, float4 *__restrict__ rec32,
-                                                         float2 *__restrict__ cand32, const ToolDev *__restrict__ tools) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= N) return;
-    int i = perm[k];
+                                                         float2 *__restrict__ cand32, const ToolDev *__restrict__ tools,
+                                                         uint32_t *status) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= N) return;
+    const int i = X.slots[s], k = rank_of(s, i, X.key, X.offsets, X.slots, status);
     F.idx[k] = i;
     double2 pos = A.pos[i], vel = A.vel[i];
     dbl4 S = A.S[i];
@@ -262,7 +284,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused(int N, const int32_t *_
     double2 pos_t = A.pos_t[i], vel_t = A.vel_t[i];
     double rho_t = A.rho_t[i], T_t = A.T_t[i];
     dbl4 S_t = A.S_t[i];
-    int hash = hash_src[i];
+    int hash = X.hash_next[i];
     B.pos[k] = pos;
     B.vel[k] = vel;
     B.fc[k] = A.fc[i];
@@ -316,14 +338,15 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused(int N, const int32_t *_
 
 
 template <class SF, class FF>
-__global__ void __launch_bounds__(kBlock) k_gather_fused32(int N, const int32_t *__restrict__ perm, KConsts K, SF A,
-                                                           FF Fsrc, SortedFields32 B, FixedFields32 F,
-                                                           int32_t *__restrict__ idx,
-                                                           const int32_t *__restrict__ hash_src,
-                                                           float4 *__restrict__ rec, float2 *__restrict__ cand,
-                                                           const ToolDev *__restrict__ tools) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < N) gather32_one(k, perm, K, A, Fsrc, B, F, idx, hash_src, rec, cand, tools);
+__global__ void __launch_bounds__(kBlock) k_gather_fused32(int N, SortScratch X, KConsts K, SF A, FF Fsrc,
+                                                           SortedFields32 B, FixedFields32 F,
+                                                           int32_t *__restrict__ idx, float4 *__restrict__ rec,
+                                                           float2 *__restrict__ cand,
+                                                           const ToolDev *__restrict__ tools, uint32_t *status) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= N) return;
+    const int i = X.slots[s], k = rank_of(s, i, X.key, X.offsets, X.slots, status);
+    gather32_one(k, i, K, A, Fsrc, B, F, idx, X.hash_next, rec, cand, tools);
 }
 
 // The compact FP32 state (state) and its p, R (pr) widened into the FP64
@@ -390,14 +413,29 @@ void launch_count(cudaStream_t s, int N, const SortedFields32 &A, const SortScra
 
 int scan_blocks(int num_cell) { return div_up(num_cell + 1, kScanTile); }
 
-void launch_sort_rest(cudaStream_t s, int N, const SortScratch &X, sph_geom_constants g, int32_t *perm,
-                      uint32_t *status) {
+// k_scan_down adds up the tile sums before its tile itself while that is one load
+// for each of its threads or a few; the scan of longer lists is a launch of its own
+// (up to 1,024 tiles = 2.1 M cells the saved launch is worth more: 2.7 us).
+constexpr int kScanTopTiles = 1024;
+int launch_sort_slots(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const FemDev &F,
+                      const ToolDev *tool) {
+    const sph_geom_constants &g = K.g;
     const int n = g.num_cell + 1;
     const int nb = scan_blocks(g.num_cell);
     k_scan_reduce<<<nb, kScanThreads, 0, s>>>(X.counts, n, X.block_sums);
-    k_scan_top<<<1, 1024, 0, s>>>(X.block_sums, nb);
-    k_scan_down<<<nb, kScanThreads, 0, s>>>(X.counts, n, X.block_sums, X.offsets, X.cell_start, X.cell_end, g.num_cell);
-    k_scatter<<<div_up(N, kBlock), kBlock, 0, s>>>(N, X.key, X.arrival, X.offsets, X.slots);
+    if (nb <= kScanTopTiles) {
+        k_scan_down<true><<<nb, kScanThreads, 0, s>>>(X.counts, n, X.block_sums, X.offsets, X.cell_start, X.cell_end,
+                                                      g.num_cell);
+    } else {
+        k_scan_top<<<1, 1024, 0, s>>>(X.block_sums, nb);
+        k_scan_down<false><<<nb, kScanThreads, 0, s>>>(X.counts, n, X.block_sums, X.offsets, X.cell_start, X.cell_end,
+                                                       g.num_cell);
+    }
+    k_scatter<<<div_up((int64_t)N + F.n_nodes, kBlock), kBlock, 0, s>>>(N, X.key, X.arrival, X.offsets, X.slots, K, F,
+                                                                        tool);
+    return nb <= kScanTopTiles ? 3 : 4;
+}
+void launch_rank(cudaStream_t s, int N, const SortScratch &X, int32_t *perm, uint32_t *status) {
     k_rank<<<div_up(N, kBlock), kBlock, 0, s>>>(N, X.key, X.offsets, X.slots, perm, status);
 }
 
@@ -405,26 +443,24 @@ void launch_gather_plain(cudaStream_t s, int N, const int32_t *perm, const Sorte
     k_gather_plain<<<div_up(N, kBlock), kBlock, 0, s>>>(N, perm, A, B);
 }
 
-void launch_gather_fused(cudaStream_t s, int N, const int32_t *perm, const KConsts &K, const SortedFields &A,
-                         const SortedFields &B, const FixedFields &F, const StepScratch &W, const int32_t *hash_src,
-                         const ToolDev *tool) {
+void launch_gather_fused(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const SortedFields &A,
+                         const SortedFields &B, const FixedFields &F, const StepScratch &W, const ToolDev *tool) {
     const int tb = fp64_block(N);   // EOS and artificial stress per particle: spread small systems
-    k_gather_fused<false><<<div_up(N, tb), tb, 0, s>>>(N, perm, K, A, B, F, hash_src, W.rec64, W.rec32, W.cand32, tool);
+    k_gather_fused<false><<<div_up(N, tb), tb, 0, s>>>(N, X, K, A, B, F, W.rec64, W.rec32, W.cand32, tool, W.status);
 }
 
-void launch_gather_fused32(cudaStream_t s, int N, const int32_t *perm, const KConsts &K, const SortedFields *A64,
+void launch_gather_fused32(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const SortedFields *A64,
                            const SortedFields32 *A32, bool pr32, const FixedFields &F, const FixedFields32 &F32,
-                           const SortedFields32 &B, int32_t *idx, const StepScratch &W, const int32_t *hash_src,
-                           const ToolDev *tool) {
+                           const SortedFields32 &B, int32_t *idx, const StepScratch &W, const ToolDev *tool) {
     const int tb = fp64_block(N), g = div_up(N, tb);
     if (A32 && pr32)
-        k_gather_fused32<<<g, tb, 0, s>>>(N, perm, K, *A32, F32, B, F32, idx, hash_src, W.rec32, W.cand32, tool);
+        k_gather_fused32<<<g, tb, 0, s>>>(N, X, K, *A32, F32, B, F32, idx, W.rec32, W.cand32, tool, W.status);
     else if (A32)
-        k_gather_fused32<<<g, tb, 0, s>>>(N, perm, K, *A32, F, B, F32, idx, hash_src, W.rec32, W.cand32, tool);
+        k_gather_fused32<<<g, tb, 0, s>>>(N, X, K, *A32, F, B, F32, idx, W.rec32, W.cand32, tool, W.status);
     else if (pr32)
-        k_gather_fused32<<<g, tb, 0, s>>>(N, perm, K, *A64, F32, B, F32, idx, hash_src, W.rec32, W.cand32, tool);
+        k_gather_fused32<<<g, tb, 0, s>>>(N, X, K, *A64, F32, B, F32, idx, W.rec32, W.cand32, tool, W.status);
     else
-        k_gather_fused32<<<g, tb, 0, s>>>(N, perm, K, *A64, F, B, F32, idx, hash_src, W.rec32, W.cand32, tool);
+        k_gather_fused32<<<g, tb, 0, s>>>(N, X, K, *A64, F, B, F32, idx, W.rec32, W.cand32, tool, W.status);
 }
 
 void launch_state_to64(cudaStream_t s, int N, const SortedFields32 &A, const FixedFields32 &Fa, const SortedFields &B,

@@ -57,18 +57,24 @@ __device__ __forceinline__ void scatter_one(int i, const int32_t *__restrict__ k
 }
 
 // ---- stable order inside each cell: rank by original index -------------------------------
-// perm[k] = original index of the particle that lands at sorted position k
-// (the reference's particles->idx after sort_by_key).
-__device__ __forceinline__ void rank_one(int s, const int32_t *__restrict__ key, const int32_t *__restrict__ offsets,
-                                         const int32_t *__restrict__ slots, int32_t *__restrict__ perm,
-                                         uint32_t *status) {
-    int i = slots[s];
+// The sorted position of the particle i = slots[s] (the k with the reference's
+// particles->idx[k] == i after sort_by_key).
+__device__ __forceinline__ int rank_of(int s, int i, const int32_t *__restrict__ key,
+                                       const int32_t *__restrict__ offsets, const int32_t *__restrict__ slots,
+                                       uint32_t *status) {
     int c = key[i];
     int cs = offsets[c], ce = offsets[c + 1];
     if (ce - cs > kCellRankCap && s == cs) set_status(status, SPH_STATUS_CELL_OVERFLOW);
     int rank = 0;
     for (int t = cs; t < ce; t++) rank += (__ldg(slots + t) < i) ? 1 : 0;
-    perm[cs + rank] = i;
+    return cs + rank;
+}
+// perm[k] = original index of the particle that lands at sorted position k.
+__device__ __forceinline__ void rank_one(int s, const int32_t *__restrict__ key, const int32_t *__restrict__ offsets,
+                                         const int32_t *__restrict__ slots, int32_t *__restrict__ perm,
+                                         uint32_t *status) {
+    const int i = slots[s];
+    perm[rank_of(s, i, key, offsets, slots, status)] = i;
 }
 
 // FP32-compensated form of the fused reorder: the same gather into the compact
@@ -78,14 +84,14 @@ __device__ __forceinline__ void rank_one(int s, const int32_t *__restrict__ key,
 // into the FP32 record.  SF / FF: the state the step starts from -- the FP64
 // arrays after an upload or a staged call, the compact arrays after a fused
 // step.  p and R of tool particles are kept from FF at the sorted position, as
-// the reference leaves them (they are not part of the Green sort's buffer).
+// the reference leaves them (they are not part of the Green sort's buffer).  k:
+// sorted position, i: index in the source.
 template <class SF, class FF>
-__device__ __forceinline__ void gather32_one(int k, const int32_t *__restrict__ perm, const KConsts &K, const SF &A,
+__device__ __forceinline__ void gather32_one(int k, int i, const KConsts &K, const SF &A,
                                              const FF &Fsrc, const SortedFields32 &B, const FixedFields32 &F,
                                              int32_t *__restrict__ idx, const int32_t *__restrict__ hash_src,
                                              float4 *__restrict__ rec, float2 *__restrict__ cand,
                                              const ToolDev *__restrict__ tools) {
-    int i = perm[k];
     idx[k] = i;
     const double2 pos = A.pos[i];
     const float2 vel = f2(A.vel[i]), pos_t = f2(A.pos_t[i]), vel_t = f2(A.vel_t[i]);

@@ -422,8 +422,8 @@ bool pse_active(const sph_ctx *ctx) { return ctx->K.thermal_pse && ctx->K.c.trml
 // The fused step body (everything after the histogram of the current state),
 // reading buf[cur] and writing buf[w] -- in FP32K contexts the compact form
 // c32[w], from c32[cur] when it holds the state (v32) and buf[cur] otherwise.
-// ev (profiling, may be null): events recorded after the sort, the reorder, the
-// FEM half step + PSE, the neighbour sums, the tool updates and the tail
+// ev (profiling, may be null): events recorded after the sort (+ FEM half step), the
+// reorder, PSE, the neighbour sums, the tool updates and the tail
 // (ev[0..5]).
 // The persistent form covers this step: FP32K from the compact state, no wear,
 // rigid tool or PSE conduction, the warm start (if any) in its in-epilogue form.
@@ -460,21 +460,16 @@ int issue_fused_body(sph_ctx *ctx, int64_t &n, int w, cudaEvent_t *ev = nullptr)
         CK_LAUNCH();
         return SPH_OK;
     }
-    launch_sort_rest(s, N, ctx->X, ctx->K.g, ctx->F.idx, ctx->W.status);
-    n += 5;
+    n += launch_sort_slots(s, N, ctx->X, ctx->K, ctx->has_tool ? ctx->fem : FemDev{}, ctx->tool_dev);
     if (ev) CK(cudaEventRecord(ev[0], s));
     if (f32)
-        launch_gather_fused32(s, N, ctx->F.idx, ctx->K, ctx->v32[ctx->cur] ? nullptr : &A,
+        launch_gather_fused32(s, N, ctx->X, ctx->K, ctx->v32[ctx->cur] ? nullptr : &A,
                               ctx->v32[ctx->cur] ? &ctx->c32[ctx->cur] : nullptr, ctx->pr32, ctx->F, ctx->F32, B32,
-                              ctx->F.idx, ctx->W, ctx->X.hash_next, ctx->tool_dev);
+                              ctx->F.idx, ctx->W, ctx->tool_dev);
     else
-        launch_gather_fused(s, N, ctx->F.idx, ctx->K, A, B, ctx->F, ctx->W, ctx->X.hash_next, ctx->tool_dev);
+        launch_gather_fused(s, N, ctx->X, ctx->K, A, B, ctx->F, ctx->W, ctx->tool_dev);
     n += 1;
     if (ev) CK(cudaEventRecord(ev[1], s));
-    if (ctx->has_tool) {
-        launch_fem_half(s, ctx->K, ctx->fem, ctx->tool_dev);
-        n += 1;
-    }
     if (pse_active(ctx)) {
         if (f32) launch_heat_pse(s, N, ctx->K, ctx->X.offsets, ctx->W, B32);
         else launch_heat_pse(s, N, ctx->K, ctx->X.offsets, ctx->W, B);
@@ -505,25 +500,24 @@ int issue_fused_body(sph_ctx *ctx, int64_t &n, int w, cudaEvent_t *ev = nullptr)
     }
     if (ev) CK(cudaEventRecord(ev[3], s));
     if (ctx->has_tool) {
-        launch_fem_rate_update(s, ctx->K, ctx->fem, ctx->seg, ctx->tool_dev);
-        n += 1;
-        if (ctx->wear_mode == SPH_WEAR_SHIFT) {   // wear_adjustment (leap_frog.cu:224-229)
+        const bool shift = ctx->wear_mode == SPH_WEAR_SHIFT;
+        launch_fem_rate_update(s, ctx->K, ctx->fem, ctx->seg, ctx->tool_dev, !shift);
+        n += 2;
+        if (shift) {   // wear_adjustment (leap_frog.cu:224-229), then the nodes with its flank retreat
             launch_wear_adjustment(s, ctx->K, ctx->fem, ctx->seg, ctx->wear, ctx->tool_dev, ctx->K.dt);
-            n += 6;
+            launch_tool_move(s, ctx->K, ctx->seg, ctx->fem, ctx->tool_dev, ctx->K.dt, 4, true);
+            n += 7;
         }
-        launch_tool_move(s, ctx->K, ctx->seg, ctx->fem, ctx->tool_dev, ctx->K.dt, 3, true);
-        n += 1;
+        launch_tool_cases(s, ctx->K.n_cases, ctx->seg, ctx->tool_dev);
     }
     if (ctx->K.rigid) {
         launch_rigid_move(s, ctx->K.rigid, ctx->K.dt);
         n += 1;
     }
     if (ev) CK(cudaEventRecord(ev[4], s));
-    // the next step's histogram and, behind it, the contact queue's length
-    CK(cudaMemsetAsync(ctx->X.counts, 0, sizeof(int32_t) * (size_t)(ctx->K.g.num_cell + 2), s));
     if (f32) launch_step_tail(s, N, ctx->K, B32, ctx->seg, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status, true);
     else launch_step_tail(s, N, ctx->K, B, ctx->seg, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status, true);
-    n += ctx->has_tool ? 3 : 1;   // with the FEM tool: the segment y-bins, then the tail and the contact queue
+    n += ctx->has_tool ? 2 : 1;   // with the FEM tool: the tail and the contact queue
     if (ev) CK(cudaEventRecord(ev[5], s));
     CK_LAUNCH();
     return SPH_OK;
@@ -1174,10 +1168,11 @@ int sph_sort(sph_ctx *ctx) {
     REQUIRE_STATE(true);
     const int N = ctx->N;
     launch_count(ctx->stream, N, CUR(ctx), ctx->X, ctx->K.g, ctx->W.status, false);
-    launch_sort_rest(ctx->stream, N, ctx->X, ctx->K.g, ctx->F.idx, ctx->W.status);
+    const int sort_launches = launch_sort_slots(ctx->stream, N, ctx->X, ctx->K, FemDev{}, ctx->tool_dev);
+    launch_rank(ctx->stream, N, ctx->X, ctx->F.idx, ctx->W.status);
     const int w = pick_out(ctx);
     launch_gather_plain(ctx->stream, N, ctx->F.idx, CUR(ctx), ctx->buf[w]);
-    ctx->launches += 7;
+    ctx->launches += 3 + sort_launches;
     CK_LAUNCH();
     int rm = mark_used(ctx, ctx->cur, w);
     if (rm) return rm;

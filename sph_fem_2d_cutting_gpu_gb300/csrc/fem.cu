@@ -10,18 +10,33 @@
 // copy, without atomics and without the colour launches.
 #include "fem.cuh"
 #include "p1elem.h"
+#include "tail.cuh"
 
 namespace sphfem {
 
-__global__ void __launch_bounds__(kBlock) k_fem_half(KConsts K, FemDev F, const ToolDev *__restrict__ tool) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < F.n_nodes) fem_half_one(i, K, F, tool);
-}
-
+// kMove: the nodes move with the tool in the same pass (the Robin terms read the
+// segments' end points, not the nodes).
+template <bool kMove>
 __global__ void __launch_bounds__(kBlock) k_fem_rate_update(KConsts K, FemDev F, SegDev seg,
                                                             const ToolDev *__restrict__ tool) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < F.n_nodes) fem_rate_update_one(i, K, F, seg, tool);
+    if (i >= F.n_nodes) return;
+    fem_rate_update_one(i, K, F, seg, tool);
+    if (kMove) {
+        const ToolDev &tc = node_case(K, tool, i);
+        node_move(F, i, tc.vel, tc.dt, tc.flank_retreat);
+    }
+}
+
+// One block per case: its segments and tool state move, then its y-bins.
+__global__ void __launch_bounds__(kBlock) k_tool_cases(SegDev seg, ToolDev *tool) {
+    ToolDev &tc = tool[blockIdx.x];
+    for (int q = threadIdx.x; q < tc.seg_count; q += blockDim.x)
+        segment_move(seg, tc.seg_first + q, tc.vel, tc.dt, tc.flank_retreat);
+    __syncthreads();
+    if (threadIdx.x == 0) tool_case_move(tc, tc.dt);
+    __syncthreads();
+    seg_bins_block(blockIdx.x, seg, tool);
 }
 
 // Staged forms: the reference's separate calls.  K_temp / f_temp hold the
@@ -67,12 +82,14 @@ __global__ void __launch_bounds__(kBlock) k_tool_move(KConsts K, SegDev seg, Fem
 }
 
 // ---- host launchers ---------------------------------------------------------------------------
-void launch_fem_half(cudaStream_t s, const KConsts &K, const FemDev &F, const ToolDev *tool) {
-    k_fem_half<<<div_up(F.n_nodes, kBlock), kBlock, 0, s>>>(K, F, tool);
-}
 void launch_fem_rate_update(cudaStream_t s, const KConsts &K, const FemDev &F, const SegDev &seg,
-                            const ToolDev *tool) {
-    k_fem_rate_update<<<div_up(F.n_nodes, kBlock), kBlock, 0, s>>>(K, F, seg, tool);
+                            const ToolDev *tool, bool move_nodes) {
+    const int grid = div_up(F.n_nodes, kBlock);
+    if (move_nodes) k_fem_rate_update<true><<<grid, kBlock, 0, s>>>(K, F, seg, tool);
+    else k_fem_rate_update<false><<<grid, kBlock, 0, s>>>(K, F, seg, tool);
+}
+void launch_tool_cases(cudaStream_t s, int n_cases, const SegDev &seg, ToolDev *tool) {
+    k_tool_cases<<<n_cases, kBlock, 0, s>>>(seg, tool);
 }
 void launch_fem_reset(cudaStream_t s, const FemDev &F, double *T_old, double *f_temp, double *K_temp) {
     k_fem_reset<<<div_up(F.nnz > F.n_nodes ? F.nnz : F.n_nodes, kBlock), kBlock, 0, s>>>(F, T_old, f_temp, K_temp);
@@ -91,7 +108,7 @@ void launch_tool_move(cudaStream_t s, const KConsts &K, const SegDev &seg, const
                       int what, bool per_case) {
     int n = per_case ? K.n_cases : 1;
     if ((what & 1) && seg.n > n) n = seg.n;
-    if ((what & 2) && F.n_nodes > n) n = F.n_nodes;
+    if ((what & 6) && F.n_nodes > n) n = F.n_nodes;
     k_tool_move<<<div_up(n, kBlock), kBlock, 0, s>>>(K, seg, F, tool, dt, what, per_case ? 1 : 0);
 }
 

@@ -103,7 +103,7 @@ __device__ __forceinline__ void tool_case_move(ToolDev &t, double dt) {
     tool_range_move(t, dt);
 }
 
-// what = 1: segments only; 2: nodes + tool state only; 3: both.  With
+// what = 1: segments only; 2: nodes + tool state only; 3: both; 4: nodes only.  With
 // per_case the velocity and time step of each segment's / node's case are
 // used (the fused step, batched or not); otherwise case 0 with `dt`.
 __device__ __forceinline__ void tool_move_one(int i, const KConsts &K, const SegDev &seg, const FemDev &F,
@@ -112,7 +112,7 @@ __device__ __forceinline__ void tool_move_one(int i, const KConsts &K, const Seg
         const ToolDev &tc = tool[(per_case && K.case_of_seg) ? K.case_of_seg[i] : 0];
         segment_move(seg, i, tc.vel, per_case ? tc.dt : dt, tc.flank_retreat);
     }
-    if ((what & 2) && i < F.n_nodes) {
+    if ((what & 6) && i < F.n_nodes) {
         const ToolDev &tc = tool[(per_case && K.case_of_node) ? K.case_of_node[i] : 0];
         node_move(F, i, tc.vel, per_case ? tc.dt : dt, tc.flank_retreat);
     }

@@ -14,21 +14,23 @@ void launch_count(cudaStream_t s, int N, const SortedFields &A, const SortScratc
 void launch_count(cudaStream_t s, int N, const SortedFields32 &A, const SortScratch &X, sph_geom_constants g,
                   uint32_t *status, bool with_hash);
 int scan_blocks(int num_cell);
-void launch_sort_rest(cudaStream_t s, int N, const SortScratch &X, sph_geom_constants g, int32_t *perm,
-                      uint32_t *status);
+// the scan of the histogram (which it leaves zeroed) and the scatter into the cells'
+// slots, with the half step of F's nodes (none: n_nodes 0); returns the launches
+int launch_sort_slots(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const FemDev &F,
+                      const ToolDev *tool);
+// perm from the slots (the staged sort; the fused gathers rank as they go)
+void launch_rank(cudaStream_t s, int N, const SortScratch &X, int32_t *perm, uint32_t *status);
 void launch_gather_plain(cudaStream_t s, int N, const int32_t *perm, const SortedFields &A, const SortedFields &B);
-void launch_gather_fused(cudaStream_t s, int N, const int32_t *perm, const KConsts &K, const SortedFields &A,
-                         const SortedFields &B, const FixedFields &F, const StepScratch &W, const int32_t *hash_src,
-                         const ToolDev *tool);
+void launch_gather_fused(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const SortedFields &A,
+                         const SortedFields &B, const FixedFields &F, const StepScratch &W, const ToolDev *tool);
 void launch_build_records(cudaStream_t s, int N, const KConsts &K, const SortedFields &A, const FixedFields &F,
                           const StepScratch &W);
 // FP32K fused reorder into the compact state B, from the FP64 state (A64) or the
 // compact one (A32, exactly one of the two non-null); the p, R that tool
 // particles keep come from F32 (pr32) or F
-void launch_gather_fused32(cudaStream_t s, int N, const int32_t *perm, const KConsts &K, const SortedFields *A64,
+void launch_gather_fused32(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const SortedFields *A64,
                            const SortedFields32 *A32, bool pr32, const FixedFields &F, const FixedFields32 &F32,
-                           const SortedFields32 &B, int32_t *idx, const StepScratch &W, const int32_t *hash_src,
-                           const ToolDev *tool);
+                           const SortedFields32 &B, int32_t *idx, const StepScratch &W, const ToolDev *tool);
 // the compact state (state) and F32's p, R (pr) widened into the FP64 arrays
 void launch_state_to64(cudaStream_t s, int N, const SortedFields32 &A, const FixedFields32 &Fa, const SortedFields &B,
                        const FixedFields &F, bool state, bool pr);
@@ -74,7 +76,7 @@ void launch_contact(cudaStream_t s, int N, const KConsts &K, const SortedFields 
 void launch_bc(cudaStream_t s, int N, const SortedFields &A);
 void launch_bc_thermal(cudaStream_t s, int N, const KConsts &K, const SortedFields &A);
 void launch_invalidate(cudaStream_t s, int N, const SortedFields &A, uint32_t *status);
-// with the FEM tool: the segment y-bins first, and the contact queue after it (two more launches)
+// with the FEM tool (its y-bins built): the contact queue after it (one more launch)
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields &A, const SegDev &seg,
                       ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
                       bool next_hash);
@@ -93,9 +95,11 @@ void launch_reduce_cases(cudaStream_t s, int n_cases, const SortedFields &A, con
                          const int32_t *cell_bound, const int32_t *part_bound, double *out);
 
 // fem.cu
-void launch_fem_half(cudaStream_t s, const KConsts &K, const FemDev &F, const ToolDev *tool);
+// move_nodes: the nodes move with the tool in the same pass (tool_update_FEM_gpu)
 void launch_fem_rate_update(cudaStream_t s, const KConsts &K, const FemDev &F, const SegDev &seg,
-                            const ToolDev *tool);
+                            const ToolDev *tool, bool move_nodes);
+// every case's segments and tool state moved, then the segment y-bins (one block a case)
+void launch_tool_cases(cudaStream_t s, int n_cases, const SegDev &seg, ToolDev *tool);
 void launch_fem_reset(cudaStream_t s, const FemDev &F, double *T_old, double *f_temp, double *K_temp);
 void launch_fem_robin(cudaStream_t s, const KConsts &K, const FemDev &F, const SegDev &seg, double *f_temp,
                       double *K_temp);
