@@ -204,10 +204,10 @@ __device__ __forceinline__ void write_record64(dbl4 *__restrict__ rec, float2 *_
                           (float)(pos.y - (g.bbmin_y + (double)row * g.dx)), K.f.cell, flags);
 }
 
-// FP32 record: (xr, yr, flags|row, h) (vx, vy, rho, c) (sA, sB, sC, vol) (Rxx, Rxy, Ryy, T)
+// FP32 record: (xr, yr, flags|row, h) (vx, vy, rho, c) (sA, sC, sB, vol) (Rxx, Ryy, Rxy, T)
 // xr, yr = offset of the particle from its cell's lower-left corner; the first
 // 16 bytes are all the candidate test needs.
-__device__ __forceinline__ void write_record32(float4 *__restrict__ rec, float2 *__restrict__ cand, int k,
+__device__ __forceinline__ void write_record32(float4 *__restrict__ rec, float2 *__restrict__ cand, int N, int k,
                                                const KConsts &K, double2 pos,
                                                double2 vel, dbl4 S, dbl4 R, double p, double h, double rho,
                                                double T, double blanked, double tool, int hash) {
@@ -220,17 +220,15 @@ __device__ __forceinline__ void write_record32(float4 *__restrict__ rec, float2 
     int flags = (cj & kRowMask) | (blanked == 1. ? kFlagBlanked : 0) | (tool == 1. ? kFlagTool : 0);
     float4 r0 = make_float4((float)xr, (float)yr, 0.f, (float)h);
     const float4 r1 = make_float4((float)vel.x, (float)vel.y, (float)rho, sqrtf((float)(K.c.phys.K / rho)));
-    const float4 r2 = make_float4((float)((S.x - p) * rho21), (float)(S.y * rho21), (float)((S.z - p) * rho21),
+    const float4 r2 = make_float4((float)((S.x - p) * rho21), (float)((S.z - p) * rho21), (float)(S.y * rho21),
                                   (float)(K.c.phys.mass / rho));
-    const float4 r3 = make_float4((float)R.x, (float)R.y, (float)R.z, (float)T);
+    const float4 r3 = make_float4((float)R.x, (float)R.z, (float)R.y, (float)T);
     if (!(flags & kFlagBlanked) && (nonfinite4(r0) || nonfinite4(r1) || nonfinite4(r2) || nonfinite4(r3)))
         flags |= kFlagNonFinite;   // blanked records are skipped as neighbours: no mark
+    flags |= cand_far(r0.x, r0.y, K.f.cell);
     r0.z = __int_as_float(flags);
-    rec[4 * k + 0] = r0;
-    rec[4 * k + 1] = r1;
-    rec[4 * k + 2] = r2;
-    rec[4 * k + 3] = r3;
-    cand[k] = cand_pack(r0.x, r0.y, flags);
+    put_rec32(rec, N, k, r0, r1, r2, r3);
+    cand[k] = cand_pack32(r0.x, r0.y, flags, K.f.cell);
 }
 
 // Staged path helper: records from the particle arrays as they are now
@@ -251,7 +249,7 @@ __global__ void __launch_bounds__(kBlock) k_build_records(int N, KConsts K, Sort
         write_record64(rec64, cand32, k, K, A.pos[k], A.vel[k], A.S[k], F.R[k], F.p[k], A.h[k], A.rho[k], T,
                        A.blanked[k], tool, hash);
     } else {
-        write_record32(rec32, cand32, k, K, A.pos[k], A.vel[k], A.S[k], F.R[k], F.p[k], A.h[k], A.rho[k], T, A.blanked[k],
+        write_record32(rec32, cand32, N, k, K, A.pos[k], A.vel[k], A.S[k], F.R[k], F.p[k], A.h[k], A.rho[k], T, A.blanked[k],
                        tool, hash);
     }
 }
@@ -332,7 +330,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused(int N, SortScratch X, K
     if (!kF32) {
         write_record64(rec64, cand32, k, K, pos, vel, S, R, p, h, rho, Tn, blanked, tool, hash);
     } else {
-        write_record32(rec32, cand32, k, K, pos, vel, S, R, p, h, rho, Tn, blanked, tool, hash);
+        write_record32(rec32, cand32, N, k, K, pos, vel, S, R, p, h, rho, Tn, blanked, tool, hash);
     }
 }
 
@@ -346,7 +344,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused32(int N, SortScratch X,
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= N) return;
     const int i = X.slots[s], k = rank_of(s, i, X.key, X.offsets, X.slots, status);
-    gather32_one(k, i, K, A, Fsrc, B, F, idx, X.hash_next, rec, cand, tools);
+    gather32_one(N, k, i, K, A, Fsrc, B, F, idx, X.hash_next, rec, cand, tools);
 }
 
 // The compact FP32 state (state) and its p, R (pr) widened into the FP64

@@ -87,7 +87,7 @@ __device__ __forceinline__ void rank_one(int s, const int32_t *__restrict__ key,
 // the reference leaves them (they are not part of the Green sort's buffer).  k:
 // sorted position, i: index in the source.
 template <class SF, class FF>
-__device__ __forceinline__ void gather32_one(int k, int i, const KConsts &K, const SF &A,
+__device__ __forceinline__ void gather32_one(int N, int k, int i, const KConsts &K, const SF &A,
                                              const FF &Fsrc, const SortedFields32 &B, const FixedFields32 &F,
                                              int32_t *__restrict__ idx, const int32_t *__restrict__ hash_src,
                                              float4 *__restrict__ rec, float2 *__restrict__ cand,
@@ -157,7 +157,7 @@ __device__ __forceinline__ void gather32_one(int k, int i, const KConsts &K, con
     F.p[k] = p;
     F.R[k] = R;
     const float Tn = Tp;   // every record carries T (k_build_records)
-    // record: (xr, yr, flags|row, h) (vx, vy, rho, c) (sA, sB, sC, m/rho) (Rxx, Rxy, Ryy, T)
+    // record: (xr, yr, flags|row, h) (vx, vy, rho, c) (sA, sC, sB, m/rho) (Rxx, Ryy, Rxy, T)
     const sph_geom_constants &g = K.g;
     int ci = 0, cj = 0;
     if (hash >= 0 && hash < g.num_cell) { ci = hash / g.ny; cj = hash - ci * g.ny; }
@@ -167,16 +167,14 @@ __device__ __forceinline__ void gather32_one(int k, int i, const KConsts &K, con
     const float rho21 = 1.f / (rhof * rhof);
     float4 r0 = make_float4(xr, yr, 0.f, h);
     const float4 r1 = make_float4(vx, vy, rhof, sqrtf(K.f.K_bulk / rhof));
-    const float4 r2 = make_float4((Sp.x - p) * rho21, Sp.y * rho21, (Sp.z - p) * rho21, K.f.mass / rhof);
-    const float4 r3 = make_float4(R.x, R.y, R.z, Tn);
+    const float4 r2 = make_float4((Sp.x - p) * rho21, (Sp.z - p) * rho21, Sp.y * rho21, K.f.mass / rhof);
+    const float4 r3 = make_float4(R.x, R.z, R.y, Tn);
     if (!(flags & kFlagBlanked) && (nonfinite4(r0) || nonfinite4(r1) || nonfinite4(r2) || nonfinite4(r3)))
         flags |= kFlagNonFinite;   // blanked records are skipped as neighbours: no mark
+    flags |= cand_far(xr, yr, K.f.cell);
     r0.z = __int_as_float(flags);
-    rec[4 * k + 0] = r0;
-    rec[4 * k + 1] = r1;
-    rec[4 * k + 2] = r2;
-    rec[4 * k + 3] = r3;
-    cand[k] = cand_pack(r0.x, r0.y, flags);
+    put_rec32(rec, N, k, r0, r1, r2, r3);
+    cand[k] = cand_pack32(xr, yr, flags, K.f.cell);
 }
 
 }  // namespace sphfem

@@ -741,7 +741,7 @@ int ctx_begin(const sph_constants *c, const sph_grid_params *g, const sph_geom_c
     } else {
         DALLOC(ctx->W.rec64, (size_t)4 * N);
     }
-    DALLOC(ctx->W.cand32, N);
+    DALLOC(ctx->W.cand32, (size_t)N + 4);   // read in groups of 4
     DALLOC(ctx->W.pos_init, N); DALLOC(ctx->W.vel_init, N); DALLOC(ctx->W.S_init, N);
     DALLOC(ctx->W.rho_init, N); DALLOC(ctx->W.T_init, N);
     DALLOC(ctx->W.secant_iters, N); DALLOC(ctx->W.status, 1);

@@ -2,7 +2,19 @@
 // sums (k_interact32), its fused epilogue and launch shapes; included by
 // interactions.cu (the plain fused step and the staged call) and
 // interactions_mlp.cu (the fused step with the learned warm start folded into
-// its epilogue).  The kernel's comments are in interactions.cu's header.
+// its epilogue).  The sums are described in interactions.cu's header.
+//
+// Bound: instruction issue (75 % busy) and the L1's passes (64 % of peak), with 24
+// warps per SM.  The candidate entries are read four to a load and tested without
+// decoding (cand_pack32), every candidate is stored and the list grows past the ones
+// that are in, the spline and the viscosity are selections instead of branches, sums
+// and vectors use the packed FP32 instructions, and a record's quarters lie in four
+// arrays (put_rec32): 9,010 instructions a warp instead of 10,440 and 1,940 L1 passes
+// instead of 2,640.  4,194,304-particle lattice (2h cells) 1.453 -> 1.237 ms, 640,000-
+// particle cut 257 -> 215 us, 12 cuts of 1.33 M particles 511 -> 423 us, 121,620-particle
+// rigid cut (cells of h) 63 -> 50 us, 12,000-particle cut 39 -> 31 us.  Products with a
+// common factor as scalars instead of packed with the factor doubled, two pairs a
+// turn, or the list entry fetched a turn ahead were 0-2 % slower.
 #pragma once
 
 #include <type_traits>
@@ -35,20 +47,85 @@ struct KahanF {
     }
 };
 
-// One 32-byte-aligned 256-bit load (two float4) through the non-coherent path:
-// the neighbour records are read-only while the pair loops run.
-__device__ __forceinline__ void ld_nc_256(const float4 *p, float4 &a, float4 &b) {
+// Two FP32 values in a register pair, and the packed instructions on them (each half
+// rounded as by the scalar one): half the issue slots, which bound this kernel.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 pk(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ F2 pk(float a) { return pk(a, a); }
+__device__ __forceinline__ float f2lo(F2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return x;
+}
+__device__ __forceinline__ float f2hi(F2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return y;
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
+// Two KahanF accumulators side by side; n holds the negated compensations.
+struct Kahan2 {
+    F2 s, n;
+    // adds a * b (the products enter the compensated sums unrounded)
+    __device__ __forceinline__ void add_product(F2 a, F2 b) { fold(fma2(a, b, n)); }
+    __device__ __forceinline__ void add(F2 v) { fold(v + n); }
+    __device__ __forceinline__ void fold(F2 y) {
+        const F2 t = s + y;
+        n = y - (t - s);
+        s = t;
+    }
+    __device__ __forceinline__ KahanF first() const { return {f2lo(s), -f2lo(n)}; }
+    __device__ __forceinline__ KahanF second() const { return {f2hi(s), -f2hi(n)}; }
+};
+
+// Hardware approximations of positive normal arguments, without the library
+// functions' scaling of subnormal ones.
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Four candidate entries of an aligned group.
+__device__ __forceinline__ void ld_cand4(const float2 *p, float2 (&c)[4]) {
     asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "=f"(c[0].x), "=f"(c[0].y), "=f"(c[1].x), "=f"(c[1].y), "=f"(c[2].x), "=f"(c[2].y), "=f"(c[3].x),
+                   "=f"(c[3].y)
                  : "l"(p));
 }
 
-// The candidate flag bits (kCandBlanked, kCandNonFinite) of a record's flag word.
-__device__ __forceinline__ int rec_cand_flags(int fj) {
-    return ((fj & kFlagBlanked) ? kCandBlanked : 0) | ((fj & kFlagNonFinite) ? kCandNonFinite : 0);
-}
-
-// The row difference gj - row of a candidate entry (cand_pack): its y carries the
+// The row difference gj - row of an FP64 candidate entry (cand_pack64): its y carries the
 // row modulo 8 in the three lowest bits, and |gj - row| <= kMaxStencil = 3, so the
 // low three bits of the difference, sign-extended, are the difference.
 __device__ __forceinline__ int cand_row_diff(int gj, float cy) {
@@ -71,7 +148,8 @@ constexpr int kChunk32 = 40;
 // forces / m), so both go into one sum per component: nine sums instead of
 // the staged form's thirteen.
 struct Acc32Fused {
-    KahanF vd0, vd1, vd2, vd3, ax, ay, xt0, xt1, tl;
+    Kahan2 vd01, vd23, a, xt;
+    KahanF tl;
 };
 
 // A particle blanked before the step skips the neighbour sums, the corrector and
@@ -236,8 +314,9 @@ __device__ __forceinline__ void stage_issue(int vb, int N, int kB, const KConsts
     const bool issue = !(K.test_faults & SPH_TEST_SKIP_BULK_COPY);   // a test lets the wait run out
     for (int c = c_lo; c <= c_hi; c++)
         if (issue && len[c - c_lo] > 0)
-            bulk_g2s(smem_u32(srec + 4 * (start[c - c_lo] + h.delta[c - c_lo])), rec + 4 * (size_t)start[c - c_lo],
-                     (uint32_t)len[c - c_lo] * 64u, mbar);
+            for (int q = 0; q < 4; q++)
+                bulk_g2s(smem_u32(srec + q * cap + start[c - c_lo] + h.delta[c - c_lo]),
+                         rec + (size_t)q * N + start[c - c_lo], (uint32_t)len[c - c_lo] * 16u, mbar);
     h.staged = 1;
     h.ix = ix;
     h.r_lo = r_lo;
@@ -277,7 +356,7 @@ __device__ __forceinline__ void block_prefetch_l2(int vb, int N, int kB, const K
     for (int c = max(ix - R, 0); c <= min(ix + R, g.nx - 1); c++) {
         const int s0 = __ldg(offsets + c * g.ny + r_lo), s1 = __ldg(offsets + c * g.ny + r_hi + 1);
         if (s1 > s0) {
-            prefetch_l2_bulk(rec + 4 * (size_t)s0, (uint32_t)(s1 - s0) * 64u);
+            for (int q = 0; q < 4; q++) prefetch_l2_bulk(rec + (size_t)q * N + s0, (uint32_t)(s1 - s0) * 16u);
             const int a0 = s0 & ~1;   // 16-byte aligned start; the size is rounded down
             prefetch_l2_bulk(cand + a0, (uint32_t)(s1 - a0) * 8u);
         }
@@ -318,7 +397,8 @@ __device__ __forceinline__ void interact32_block(int vb, int N, const KConsts &K
     const unsigned gmask = ((1u << kSplit) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(kSplit - 1));
     if (kFused && threadIdx.x == 0) block_prefetch_l2(vb, N, kPPB, K, offsets, rec, cand, B, F);
     int (*s_list)[kB];
-    const float4 *nrec = rec;   // where the neighbour records are read from
+    const float4 *rec_b = rec + 2 * (size_t)N;   // the records' third and fourth quarters
+    const float4 *nrec = rec;   // staged: the copies in shared memory, quarter by quarter
     __shared__ StageHdr s_hdr;
     __shared__ alignas(8) unsigned long long s_mbar;
     bool staged = false;
@@ -337,24 +417,24 @@ __device__ __forceinline__ void interact32_block(int vb, int N, const KConsts &K
             }
         }
     } else {
-        __shared__ int s_list_st[kChunk32][kB];
+        __shared__ int s_list_st[kChunk32 + 1][kB];
         s_list = s_list_st;
     }
     bool pending = false;   // kMlp: this particle yields and waits for its warm start
     auto particle = [&]() {
     if (k >= N) return;
-    const float4 i0 = rec[4 * k + 0];
+    const float4 i0 = rec[k];
     const int fi = __float_as_int(i0.z);
     if (fi & kFlagBlanked) {
         if (kFused && sub == 0) rigid_heat_blanked(k, K, B);   // one lane per particle
         return;
     }
     const bool tool_i = (fi & kFlagTool) != 0;
-    const float4 i1 = rec[4 * k + 1], i2 = rec[4 * k + 2], i3 = rec[4 * k + 3];
+    const float4 i1 = rec[N + k], i2 = rec_b[k], i3 = rec_b[N + k];
     const float xri = i0.x, yri = i0.y, hi = i0.w;
     const float vix = i1.x, viy = i1.y, rhoi = i1.z, ci = i1.w;
-    const float sAi = i2.x, sBi = i2.y, sCi = i2.z;
-    const float Rxxi = i3.x, Rxyi = i3.y, Ryyi = i3.z, Ti = i3.w;
+    const float sAi = i2.x, sCi = i2.y, sBi = i2.z;
+    const float Rxxi = i3.x, Ryyi = i3.y, Rxyi = i3.z, Ti = i3.w;
     const float thermal_alpha = (!tool_i) ? K.f.alpha_wp : K.f.alpha_tool_sph;
     const bool thermal = thermal_alpha != 0.f && !K.thermal_pse;   // Brookshaw build only
     const bool pse_tool = K.thermal_pse && tool_i;                  // PSE build: tool particles return at once
@@ -376,7 +456,8 @@ __device__ __forceinline__ void interact32_block(int vb, int N, const KConsts &K
     const float kde = -3.f * fac * h1 * h1, kdf = 2.25f * fac * h1 * h1;
     const int hash = B.hash[k];
     const sph_geom_constants &g = K.g;
-    int gi = 0, gj = 0, ii = 0, hi_i = 0, lo_j = 0, hi_j = 0, j = 0, j1 = 0;
+    int gi = 0, gj = 0, ii = 0, hi_i = 0, lo_j = 0, hi_j = 0;
+    int j = 0, j0 = 0, j1 = 0;   // the column's range [j0, j1); j: the next group of four, aligned
     const int R = g.stencil;
     bool done = true;
     if (hash >= 0 && hash < g.num_cell && !pse_tool) {
@@ -386,166 +467,141 @@ __device__ __forceinline__ void interact32_block(int vb, int N, const KConsts &K
         hi_i = min(gi + R + 1, g.nx);
         lo_j = max(gj - R, 0);
         hi_j = min(gj + R + 1, g.ny);
-        j = __ldg(offsets + ii * g.ny + lo_j) + sub;
-        j1 = __ldg(offsets + ii * g.ny + hi_j);
         done = false;
     }
-    // a particle whose stencil lies inside the staged region reads shared memory
-    // (slot = global index + per-column delta); any other uses global loads
+    // a particle whose stencil lies inside the staged region reads its neighbours'
+    // records from shared memory (slot = global index + per-column delta); any other
+    // uses global loads
     bool use_s = false;
-    if constexpr (kStaged) {
+    if constexpr (kStaged)
         use_s = staged && !done && gi == s_hdr.ix && lo_j >= s_hdr.r_lo && hi_j - 1 <= s_hdr.r_hi;
-        if (use_s) {
-            j += s_hdr.delta[ii - s_hdr.c_lo];
-            j1 += s_hdr.delta[ii - s_hdr.c_lo];
-        }
-    }
-    const float4 *__restrict__ nb = use_s ? nrec : rec;
     // Pass 0 sums over the in-support neighbours.  In the reference every active
     // particle of the stencil (this one included) runs the pair body, with zero
     // kernel weights outside the support: exact zeros for finite data, but NaN
     // when one of the factors is NaN or infinite.  So a particle whose stencil
     // holds a record marked non-finite repeats its sums over every active
     // candidate with the reference's zero weights (pass 1).
-    // OR of the candidate flags over the stencil (bit kCandNonFinite is the one
-    // read; blanked candidates carry no mark)
-    int marks = 0;
+    int marks = 0;   // OR of the flags of the candidates that the entries could not decide
+    const float cell8 = 8.f * cell;
+    const F2 cell_2 = pk(cell), x_i = pk(xri, yri), v_i = pk(vix, viy), s_i = pk(sAi, sCi), R_i = pk(Rxxi, Ryyi);
+    const float rhoi_half = 0.5f * rhoi, hi_half = 0.5f * hi, c_i = -0.5f * alpha * ci;
+    // this particle in the entries' frame; one whose own entry could not decide takes all
+    const bool take_all = (fi & (kFlagNonFinite | kFlagFar)) != 0;
+    const float y8 = take_all ? __int_as_float(0x7fffffff) : cand_y8(yri, gj & 7, cell);
+    const int undecided = kFlagNonFinite | kFlagFar;
+    auto column = [&]() {   // the range of column ii
+        j0 = __ldg(offsets + ii * g.ny + lo_j);
+        j1 = __ldg(offsets + ii * g.ny + hi_j);
+        j = (j0 & ~3) + 4 * sub;
+    };
     auto sweep = [&](auto all_tag) {
     constexpr bool all = decltype(all_tag)::value;
-    // the candidate test on (xr, yr), the row difference and the flag bits
-    auto take = [&](int &cnt, int jj, float cx, float cy, int drow, int cf, float dxc) {
-        const float dx = dxc + (xri - cx);
-        const float dy = (float)drow * cell + (yri - cy);
-        const float rr2 = dx * dx + dy * dy;
-        if (!all) marks |= cf;
-        if ((all || (rr2 < fourh2 && rr2 >= 1e-8f)) && !(cf & kCandBlanked))
-            s_list[cnt++][threadIdx.x] = (jj << 3) | (gi - ii + R);
-    };
+    if (!done) column();
     while (!done) {
-        // phase 1: collect the next in-support, active neighbours (column offset packed in 3 bits)
-        // from the 8-byte candidate entries (cand_pack), or from the staged records' first 16
-        // bytes; four candidates per round keep four loads in flight
-        int cnt = 0;
-        while (cnt < kChunk32) {
-            const float dxc = (float)(gi - ii) * cell;
-            if (j + 4 * kSplit - (kSplit - 1) <= j1 && cnt <= kChunk32 - 4) {
-                if (!kStaged || !use_s) {
-                    float2 c[4];
+        // phase 1: collect the next in-support neighbours (column offset packed in 3 bits)
+        // from the 8-byte candidate entries, four in one aligned load.  Every candidate is
+        // stored, and the list grows past it if it is in.
+        int *lp = &s_list[0][threadIdx.x];
+        const int *const list = lp;
+        while (lp <= list + (kChunk32 - 4) * kB) {
+            if (j < j1) {
+                const float xc = fmaf((float)(gi - ii), cell, xri);
+                const int e = (j << 3) | (gi - ii + R), u0 = j - j0;
+                const unsigned len = (unsigned)(j1 - j0);
+                float2 c[4];
+                ld_cand4(cand + j, c);
 #pragma unroll
-                    for (int u = 0; u < 4; u++) c[u] = __ldg(cand + j + u * kSplit);
-#pragma unroll
-                    for (int u = 0; u < 4; u++)
-                        take(cnt, j + u * kSplit, c[u].x, c[u].y, cand_row_diff(gj, c[u].y),
-                             __float_as_int(c[u].x), dxc);
-                } else {
-                    float4 n[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) n[u] = nb[4 * (j + u * kSplit)];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int fj = __float_as_int(n[u].z);
-                        take(cnt, j + u * kSplit, n[u].x, n[u].y, gj - (fj & kRowMask), rec_cand_flags(fj), dxc);
-                    }
+                for (int u = 0; u < 4; u++) {
+                    const float dx = xc - c[u].x, dd = y8 - c[u].y;
+                    const float dy = fminf(fabsf(dd), cell8 - fabsf(dd));
+                    const float rr2 = dx * dx + dy * dy;
+                    *lp = e + 8 * u;
+                    // NaN passes both tests of the distance
+                    const bool in = ((unsigned)(u0 + u) < len) & (all | (!(rr2 >= fourh2) & !(rr2 < 1e-8f)));
+                    lp += in ? kB : 0;
                 }
                 j += 4 * kSplit;
-            } else if (j < j1) {
-                if (!kStaged || !use_s) {
-                    const float2 c = __ldg(cand + j);
-                    take(cnt, j, c.x, c.y, cand_row_diff(gj, c.y), __float_as_int(c.x), dxc);
-                } else {
-                    const float4 n0 = nb[4 * j + 0];
-                    const int fj = __float_as_int(n0.z);
-                    take(cnt, j, n0.x, n0.y, gj - (fj & kRowMask), rec_cand_flags(fj), dxc);
-                }
-                j += kSplit;
             } else {
                 if (++ii >= hi_i) {
                     done = true;
                     break;
                 }
-                j = __ldg(offsets + ii * g.ny + lo_j) + sub;
-                j1 = __ldg(offsets + ii * g.ny + hi_j);
-                if constexpr (kStaged) {
-                    if (use_s) {
-                        j += s_hdr.delta[ii - s_hdr.c_lo];
-                        j1 += s_hdr.delta[ii - s_hdr.c_lo];
-                    }
-                }
+                column();
             }
         }
         // phase 2: the pair body over the collected list, lanes in step.  No
         // software prefetch of the next record: the 32 registers it holds cost
         // more resident warps than it hides latency.
-        for (int t = 0; t < cnt; t++) {
-            const int e = s_list[t][threadIdx.x];
+        for (const int *q0 = list; q0 < lp; q0 += kB) {
+            const int e = *q0;
             const int jn = e >> 3;
-            // the 64-byte record of an in-support neighbour: two 256-bit loads (the
-            // kernel is bound by L1 wavefronts, and one request per 32 bytes halves them)
-            float4 n0, n1, n2, n3;
+            float4 n0, n1, n2, n3;   // the neighbour's 64-byte record
             if (use_s) {
-                n0 = nb[4 * jn + 0];
-                n1 = nb[4 * jn + 1];
-                n2 = nb[4 * jn + 2];
-                n3 = nb[4 * jn + 3];
+                const float4 *r = nrec + (jn + s_hdr.delta[gi + R - (e & 7) - s_hdr.c_lo]);
+                n0 = r[0];
+                n1 = r[cap];
+                n2 = r[2 * cap];
+                n3 = r[3 * cap];
             } else {
-                ld_nc_256(rec + 4 * jn, n0, n1);
-                ld_nc_256(rec + 4 * jn + 2, n2, n3);
+                n0 = __ldg(rec + jn);
+                n1 = __ldg(rec + N + jn);
+                n2 = __ldg(rec_b + jn);
+                n3 = __ldg(rec_b + N + jn);
             }
             const int fj = __float_as_int(n0.z);
-            const float dx = (float)((e & 7) - R) * cell + (xri - n0.x);
-            const float dy = (float)(gj - (fj & kRowMask)) * cell + (yri - n0.y);
+            // the distance vector: cell offset times the cell edge, plus the offsets in the cells
+            const F2 off = pk((float)((e & 7) - R), (float)(gj - (fj & kRowMask)));
+            const F2 d = fma2(off, cell_2, x_i - pk(n0.x, n0.y));
+            const float dx = f2lo(d), dy = f2hi(d);
             const float rr2 = dx * dx + dy * dy;
-            // FP32 form: hardware reciprocal square root instead of sqrt and division
-            const float inv_r = rsqrtf(rr2);
+            // FP32 form: hardware reciprocal square root instead of sqrt and division; both
+            // branches of the spline and a selection, so that the lanes stay together
+            const float inv_r = rsqrt_approx(rr2);
             const float q = rr2 * inv_r * h1;
+            const bool far = q > 1.f;
             // pass 1: cubic_spline's zero weights outside the support (kernels.cuh:37-39)
-            const bool zero_w = all && (rr2 >= fourh2 || rr2 < 1e-8f);
+            bool zero_w = false, conduction_only = false;
+            if (all || ((fj | fi) & (undecided | kFlagTool))) {   // rare
+                const bool out = !(rr2 < fourh2 && rr2 >= 1e-8f);
+                if (all) {
+                    if (fj & kFlagBlanked) continue;
+                    zero_w = out;
+                } else if ((fj | fi) & undecided) {
+                    marks |= fj | fi;
+                    if (out || (fj & kFlagBlanked)) continue;
+                }
+                conduction_only = ((fj | fi) & kFlagTool) != 0;
+            }
             if constexpr (kFused) {
-                float w, dwf;
-                if (q > 1.f) {
-                    const float tq = 2.f - q, t2 = tq * tq;
-                    w = kwa * (t2 * t2 * t2);
-                    dwf = kda * t2 * inv_r;
-                } else {
-                    w = fmaf(q * q, fmaf(kwd, q, kwc), fac);
-                    dwf = fmaf(kdf, q, kde);
-                }
-                if (zero_w) w = dwf = 0.f;
-                const float wx = dwf * dx, wy = dwf * dy;
-                const float volj = n2.w;
-                if (!tool_i && !(fj & kFlagTool)) {
-                    const float dvx = n1.x - vix, dvy = n1.y - viy;
-                    const float tx = wx * volj, ty = wy * volj;
-                    af.vd0.add(dvx * tx);
-                    af.vd1.add(dvx * ty);
-                    af.vd2.add(dvy * tx);
-                    af.vd3.add(dvy * ty);
-                    float fab = w * inv_wdp;
-                    fab *= fab;
-                    fab *= fab;
-                    const float sxx = (sAi + n2.x) + fab * (Rxxi + n3.x);
-                    const float sxy = (sBi + n2.y) + fab * (Rxyi + n3.y);
-                    const float syy = (sCi + n2.z) + fab * (Ryyi + n3.z);
-                    const float vijposij = -(dvx * dx + dvy * dy);
-                    const float irho = __fdividef(2.f, rhoi + n1.z);
-                    float piij = 0.f;
-                    if (vijposij < 0.f) {
-                        const float cij = 0.5f * (ci + n1.w);
-                        const float hij = 0.5f * (hi + n0.w);
-                        const float muij = __fdividef(hij * vijposij, rr2 + eta2 * hij * hij);
-                        piij = (-alpha * cij * muij + beta * muij * muij) * irho;
-                    }
-                    // acceleration / mass: (stress terms - viscosity) . grad W
-                    af.ax.add(fmaf(sxx - piij, wx, sxy * wy));
-                    af.ay.add(fmaf(sxy, wx, (syy - piij) * wy));
-                    const float wr = w * irho;
-                    af.xt0.add(wr * dvx);
-                    af.xt1.add(wr * dvy);
-                }
-                if (thermal && (!zero_w || rr2 > 1e-16f)) af.tl.add(volj * (Ti - n3.w) * dwf);
+                const float u = far ? 2.f - q : q, u2 = u * u;
+                float w = far ? u2 * u2 * (kwa * u2) : fmaf(u2, fmaf(kwd, u, kwc), fac);
+                float dwf = far ? kda * u2 * inv_r : fmaf(kdf, u, kde);
+                if (all && zero_w) w = dwf = 0.f;
+                if (thermal && (!all || !zero_w || rr2 > 1e-16f)) af.tl.add(n2.w * (Ti - n3.w) * dwf);
+                if (conduction_only) continue;
+                const F2 wg = pk(dwf) * d;   // grad W
+                const F2 dv = pk(n1.x, n1.y) - v_i;
+                const F2 tv = wg * pk(n2.w);
+                af.vd01.add_product(pk(f2lo(dv)), tv);
+                af.vd23.add_product(pk(f2hi(dv)), tv);
+                float fab = w * inv_wdp;
+                fab *= fab;
+                fab *= fab;
+                F2 sd = fma2(pk(fab), R_i + pk(n3.x, n3.y), s_i + pk(n2.x, n2.y));
+                const float sxy = fmaf(fab, Rxyi + n3.z, sBi + n2.z);
+                const float vijposij = -(f2lo(dv) * dx + f2hi(dv) * dy);
+                const float irho = rcp_approx(fmaf(0.5f, n1.z, rhoi_half));
+                const float hij = fmaf(0.5f, n0.w, hi_half);
+                const float muij = hij * vijposij * rcp_approx(fmaf(eta2 * hij, hij, rr2));
+                // (-alpha c_ij mu + beta mu^2) / rho_ij of an approaching pair
+                const float pi = fmaf(beta, muij, fmaf(-0.5f * alpha, n1.w, c_i)) * muij * irho;
+                // acceleration / mass: (stress terms - viscosity) . grad W
+                sd = sd - pk(vijposij < 0.f ? pi : 0.f);
+                af.a.add(fma2(sd, wg, pk(sxy) * pk(f2hi(wg), f2lo(wg))));
+                af.xt.add_product(pk(w * irho), dv);
             } else {
                 float val, der;
-                if (q > 1.f) {
+                if (far) {
                     const float t = 2.f - q, t2 = t * t;
                     val = 0.25f * t2 * t2 * t2;
                     der = -0.75f * t2 * h1 * inv_r;
@@ -557,7 +613,7 @@ __device__ __forceinline__ void interact32_block(int vb, int N, const KConsts &K
                 const float dwf = zero_w ? 0.f : der * fac;
                 const float wx = dwf * dx, wy = dwf * dy;
                 const float volj = n2.w;
-                if (!tool_i && !(fj & kFlagTool)) {
+                if (!conduction_only) {
                     const float dvx = n1.x - vix, dvy = n1.y - viy;
                     const float tx = wx * volj, ty = wy * volj;
                     vd0.add(dvx * tx);
@@ -568,8 +624,8 @@ __device__ __forceinline__ void interact32_block(int vb, int N, const KConsts &K
                     fab *= fab;
                     fab *= fab;
                     const float ax = (sAi + n2.x) + fab * (Rxxi + n3.x);
-                    const float ay = (sBi + n2.y) + fab * (Rxyi + n3.y);
-                    const float az = (sCi + n2.z) + fab * (Ryyi + n3.z);
+                    const float ay = (sBi + n2.z) + fab * (Rxyi + n3.z);
+                    const float az = (sCi + n2.y) + fab * (Ryyi + n3.y);
                     sd0.add(ax * wx);
                     sd1.add(ay * wy);
                     sd2.add(ay * wx);
@@ -598,44 +654,30 @@ __device__ __forceinline__ void interact32_block(int vb, int N, const KConsts &K
 #pragma unroll
         for (int o = 1; o < kSplit; o <<= 1) marks |= __shfl_xor_sync(gmask, marks, o);
     }
-    if (marks & kCandNonFinite) {   // rare: the reference's full stencil with zero weights
+    if (marks & kFlagNonFinite) {   // rare: the reference's full stencil with zero weights
         vd0 = vd1 = vd2 = vd3 = sd0 = sd1 = sd2 = sd3 = vt0 = vt1 = xt0 = xt1 = tl = KahanF{};
         af = Acc32Fused{};
         ii = max(gi - R, 0);
-        j = __ldg(offsets + ii * g.ny + lo_j) + sub;
-        j1 = __ldg(offsets + ii * g.ny + hi_j);
-        if constexpr (kStaged) {
-            if (use_s) {
-                j += s_hdr.delta[ii - s_hdr.c_lo];
-                j1 += s_hdr.delta[ii - s_hdr.c_lo];
-            }
-        }
         done = false;
         sweep(std::true_type{});
     }
     if constexpr (kFused) {
+        KahanF f[9] = {af.vd01.first(), af.vd01.second(), af.vd23.first(), af.vd23.second(), af.a.first(),
+                       af.a.second(), af.xt.first(), af.xt.second(), af.tl};
         if constexpr (kSplit > 1) {   // merge the lanes' compensated sums; the first lane goes on
 #pragma unroll
-            for (int o = 1; o < kSplit; o <<= 1) {
-                af.vd0.merge(gmask, o);
-                af.vd1.merge(gmask, o);
-                af.vd2.merge(gmask, o);
-                af.vd3.merge(gmask, o);
-                af.ax.merge(gmask, o);
-                af.ay.merge(gmask, o);
-                af.xt0.merge(gmask, o);
-                af.xt1.merge(gmask, o);
-                af.tl.merge(gmask, o);
-            }
+            for (int o = 1; o < kSplit; o <<= 1)
+#pragma unroll
+                for (int m = 0; m < 9; m++) f[m].merge(gmask, o);
             if (sub != 0) return;
         }
         const float mass = K.f.mass;
         const float xs = K.f.xs_mass;
-        const float4 vd = make_float4(af.vd0.s, af.vd1.s, af.vd2.s, af.vd3.s);
+        const float4 vd = make_float4(f[0].s, f[1].s, f[2].s, f[3].s);
         // the whole acceleration sum rides in sd.x / sd.z (vt zero): the epilogue adds sd.x + sd.y + vt.x
-        const float4 sd = make_float4(mass * af.ax.s, 0.f, mass * af.ay.s, 0.f);
-        const float2 xt = make_float2(xs * af.xt0.s, xs * af.xt1.s);
-        const float T_t = thermal_alpha * (2.0f * af.tl.s);
+        const float4 sd = make_float4(mass * f[4].s, 0.f, mass * f[5].s, 0.f);
+        const float2 xt = make_float2(xs * f[6].s, xs * f[7].s);
+        const float T_t = thermal_alpha * (2.0f * f[8].s);
         // predicted velocity and density from this particle's record
         fused_epilogue32<kMlp>(k, K, B, F, seg, tool, secant_iters, status, tool_i, make_float2(vix, viy), rhoi, vd,
                                sd, make_float2(0.f, 0.f), xt, thermal, T_t, pending);
@@ -677,7 +719,7 @@ static void launch_i32(cudaStream_t s, int N, const KConsts &K, const int32_t *o
                        const MlpDev &mlp = MlpDev{}) {
     size_t smem = 0;
     if (kStaged) {
-        smem = (size_t)cap * 64 + sizeof(int) * kChunk32 * kB;
+        smem = (size_t)cap * 64 + sizeof(int) * (kChunk32 + 1) * kB;
         static bool configured = false;   // opt in above 48 KB of dynamic shared memory, once
         if (!configured) {
             cudaFuncSetAttribute(k_interact32<true, kB, kMinB, kStaged, kMlp, kSplit>,

@@ -31,12 +31,10 @@ namespace sphfem {
 
 // Launch shapes of the fused FP32K neighbour-sum kernel: (threads per block,
 // minimum resident blocks per SM, staged records: 0 = global loads, lanes per
-// particle).  Variant 0 is the default: 6 blocks (24 warps) per SM at 76
-// registers (80 with the learned warm start in the epilogue).  A minimum of 5
-// blocks of 128 (or 10 of 64) lets the compiler keep 80 registers at the same
-// 24 warps; a free choice (91 registers) drops to 20 warps.  On the 4.19 M
-// lattice 64x10, 128x6 and 256x3 lie within 2 % of each other, 128x5 4 % behind;
-// with the warm start 128x5 and 64x10 need 96 registers (20 warps).
+// particle).  Variant 0 is the default: 6 blocks (24 warps) per SM at 79
+// registers.  On the 4.19 M lattice 128x6 and 256x3 are within 0.2 % of each
+// other, 64x12, 64x8 and 128x4 1-2 % behind, 128x5 and 64x10 5 %; on the
+// 12,000-particle cut the shapes with 2 and 4 lanes per particle are ahead.
 const int kInteractVariants[][4] = {{128, 6, 0, 1},   {64, 12, 0, 1},   {64, 8, 0, 1},     {128, 4, 0, 1},
                                     {256, 3, 0, 1},   {256, 1, 0, 1},   {128, 3, 640, 1},  {128, 2, 1024, 1},
                                     {64, 6, 384, 1},  {256, 2, 1024, 1}, {128, 6, 0, 2},    {128, 6, 0, 4},
@@ -144,10 +142,11 @@ __global__ void __launch_bounds__(kBlock) k_heat_pse32(int N, KConsts K, const i
                                                        const int32_t *__restrict__ hashes, TT *__restrict__ T_t) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= N) return;
-    const float4 i0 = rec[4 * k + 0];
+    const float4 *rec_c = rec + 2 * (size_t)N, *rec_d = rec + 3 * (size_t)N;   // the records' last two quarters
+    const float4 i0 = rec[k];
     const int fi = __float_as_int(i0.z);
     if (fi & kFlagBlanked) return;
-    const float xri = i0.x, yri = i0.y, hi = i0.w, Ti = rec[4 * k + 3].w;
+    const float xri = i0.x, yri = i0.y, hi = i0.w, Ti = rec_d[k].w;
     const double alpha = ((fi & kFlagTool) && k < N / 2) ? K.c.trml_tool_sph.alpha : K.c.trml_wp.alpha;
     const float h2 = hi * hi;
     const float c = 4.f / (h2 * h2 * (float)kRigidPi);
@@ -165,11 +164,11 @@ __global__ void __launch_bounds__(kBlock) k_heat_pse32(int N, KConsts K, const i
             const int j1 = __ldg(offsets + ii * g.ny + hi_j);
 #pragma unroll 4   // several neighbours' loads in flight (the kernel waits on loads, not on math)
             for (int j = __ldg(offsets + ii * g.ny + lo_j); j < j1; j++) {
-                const float4 n0 = rec[4 * j + 0];
+                const float4 n0 = rec[j];
                 const float dx = dxc + (xri - n0.x);
                 const float dy = (float)(gj - (__float_as_int(n0.z) & kRowMask)) * cell + (yri - n0.y);
                 const float w2 = c * expf(-(dx * dx + dy * dy) * inv_h2);
-                sum.add((rec[4 * j + 3].w - Ti) * w2 * rec[4 * j + 2].w);
+                sum.add((rec_d[j].w - Ti) * w2 * rec_c[j].w);
             }
         }
     }

@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kPB, kPMinBlocks) k_step_persistent(PersistArg
     if (!grid_barrier(P.bar, status)) return;
     // reorder + predictor + EOS + artificial stress + records
     for (int k = gtid; k < N; k += gstride)
-        gather32_one(k, P.perm[k], K, P.A, P.F32, P.B, P.F32, P.perm, P.X.hash_next, P.W.rec32, P.W.cand32, P.tool);
+        gather32_one(N, k, P.perm[k], K, P.A, P.F32, P.B, P.F32, P.perm, P.X.hash_next, P.W.rec32, P.W.cand32, P.tool);
     if (!grid_barrier(P.bar, status)) return;
     // neighbour sums + epilogue, 128 particles per virtual block
     const int n_vb = (N + kPB - 1) / kPB;

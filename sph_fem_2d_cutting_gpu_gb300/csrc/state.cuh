@@ -74,23 +74,44 @@ constexpr int kRecWords = 16;
 // kFlagNonFinite: a value of an active particle's record is NaN or infinite
 // (its pair terms are NaN even with the zero kernel weights outside the
 // support); never set on blanked records.
-enum : int { kFlagBlanked = 1 << 30, kFlagTool = 1 << 29, kFlagNonFinite = 1 << 28, kRowMask = (1 << 28) - 1 };
+// kFlagFar (FP32 records): the position is so far from its cell's box (moved since
+// the sort) that its candidate entry cannot stand for it.
+enum : int {
+    kFlagFar = (int)0x80000000u, kFlagBlanked = 1 << 30, kFlagTool = 1 << 29, kFlagNonFinite = 1 << 28,
+    kRowMask = (1 << 28) - 1
+};
 
-// FP32K candidate entry, one float2 per record in the same order: the record's
-// (xr, yr) for the in-support test of the candidate scan, 8 bytes instead of
-// the record's first 16.  The flags ride in the low mantissa bits: xr's two
-// lowest bits hold kCandBlanked / kCandNonFinite, yr's three lowest bits the
-// cell row modulo 8 (the row difference to the summing particle is at most the
-// stencil half-width, 3).  Each coordinate moves by at most 7 units in the
-// last place of a value below a cell edge, so the test's support boundary
-// moves by at most 2^-20 of a cell, where the kernel and its gradient vanish to
-// third and second order; the pair terms themselves use the full record.
-enum : int { kCandBlanked = 1, kCandNonFinite = 2 };
-__device__ __forceinline__ float2 cand_pack(float xr, float yr, int flags) {
-    const int bx = (__float_as_int(xr) & ~3) | ((flags & kFlagBlanked) ? kCandBlanked : 0) |
-                   ((flags & kFlagNonFinite) ? kCandNonFinite : 0);
-    const int by = (__float_as_int(yr) & ~7) | (flags & 7);
-    return make_float2(__int_as_float(bx), __int_as_float(by));
+// An FP32 record's four quarters lie in four arrays: the lanes of a warp read
+// neighbours that are mostly near one another in cell order, and with eight quarters
+// to a 128-byte line a pass of the L1 serves more lanes than with two whole records --
+// the neighbour sums are bound by these passes (2,640 a warp with whole records read
+// by 256-bit loads, 2,250 with halves, 2,060 with quarters).
+__device__ __forceinline__ void put_rec32(float4 *__restrict__ rec, int N, int k, float4 r0, float4 r1, float4 r2,
+                                          float4 r3) {
+    rec[k] = r0;
+    rec[(size_t)N + k] = r1;
+    rec[2 * (size_t)N + k] = r2;
+    rec[3 * (size_t)N + k] = r3;
+}
+
+// FP32 candidate entry, one float2 per record in the same order, for the in-support
+// test of the candidate scan: (x - x_cell, y8), 8 bytes instead of the record's first
+// 16.  y8 is the y coordinate in a frame that repeats every 8 cells, (row mod 8) cell +
+// (y - y_cell): rows that a stencil joins are at most 3 apart, so min(|d|, 8 cell -
+// |d|) of two entries' difference d is their distance in y, with no row to decode.  y8
+// is below 8 cells: its rounding moves the test's boundary by less than 2^-19 of a cell,
+// where the kernel and its gradient vanish to third and second order; the pair terms
+// use the full record.  A blanked record's entry fails every test (x infinite); one
+// whose record is marked non-finite or far passes every test (x NaN, in a test that
+// NaN passes), and the record's flags decide.
+__device__ __forceinline__ float cand_y8(float yr, int row, float cell) { return fmaf((float)(row & 7), cell, yr); }
+__device__ __forceinline__ int cand_far(float xr, float yr, float cell) {
+    return fabsf(xr - 0.5f * cell) <= 0.75f * cell && fabsf(yr - 0.5f * cell) <= 0.75f * cell ? 0 : kFlagFar;
+}
+__device__ __forceinline__ float2 cand_pack32(float xr, float yr, int flags, float cell) {
+    const float x = (flags & kFlagBlanked) ? __int_as_float(0x7f800000)
+                    : (flags & (kFlagNonFinite | kFlagFar)) ? __int_as_float(0x7fffffff) : xr;
+    return make_float2(x, cand_y8(yr, flags & 7, cell));
 }
 
 // Per-segment constants of the contact search, rebuilt each step with the
@@ -161,20 +182,25 @@ struct WearDev {
     double A, B, C, D;                   // wear constants (constants_structs.h:113-119)
 };
 
-// The same entries beside the FP64 records, for a test that only sorts out
-// candidates that cannot be in the support: kCandSpecial marks the ones that it
-// may not sort out -- a non-finite record, or coordinates further than 4 cells
-// from the cell (positions moved since the sort), where FP32 is too coarse.
-constexpr int kCandSpecial = kCandNonFinite;
+// Candidate entry beside the FP64 records, for a test that only sorts out candidates
+// that cannot be in the support: (x - x_cell, y - y_cell), the flags in the low
+// mantissa bits: x's two lowest hold kCandBlanked / kCandSpecial, y's three lowest the
+// cell row modulo 8.  kCandSpecial marks the ones that the test may not sort out -- a
+// non-finite record, or coordinates further than 4 cells from the cell (positions
+// moved since the sort), where FP32 is too coarse.
+enum : int { kCandBlanked = 1, kCandSpecial = 2 };
 __device__ __forceinline__ float2 cand_pack64(float xr, float yr, float cell, int flags) {
     const bool near = fabsf(xr) <= 4.f * cell && fabsf(yr) <= 4.f * cell;
-    return cand_pack(xr, yr, near ? flags : flags | kFlagNonFinite);
+    const int bx = (__float_as_int(xr) & ~3) | ((flags & kFlagBlanked) ? kCandBlanked : 0) |
+                   (!near || (flags & kFlagNonFinite) ? kCandSpecial : 0);
+    const int by = (__float_as_int(yr) & ~7) | (flags & 7);
+    return make_float2(__int_as_float(bx), __int_as_float(by));
 }
 
 struct StepScratch {
     dbl4 *rec64;      // [N][4] FP64 records
-    float4 *rec32;       // [N][4] FP32 records
-    float2 *cand32;      // [N] candidate entries of the records (cand_pack, cand_pack64)
+    float4 *rec32;       // [4][N] FP32 records, quarter by quarter (put_rec32)
+    float2 *cand32;      // [N, padded to whole groups of 4] candidate entries of the records (cand_pack32, cand_pack64)
     double2 *pos_init, *vel_init;   // leap_frog snapshots (staged path)
     dbl4 *S_init;
     double *rho_init, *T_init;
