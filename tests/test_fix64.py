@@ -1,10 +1,12 @@
 """Integer model of csrc/fix64.cuh's reciprocals and rounded product, against exact rationals,
-and of csrc/fix64_math.cuh's log2 and exp2 (with the tables read from it), against 60 digits.
+and of csrc/fix64_math.cuh's log2, exp2, atan2, sin and cos (with the tables read from it),
+against 60 digits and against correctly rounded floats.
 
 The device functions restated step by step on Python integers: the third-order Newton
 reciprocal of a 53-bit mantissa stays within the stated 2^5 units of 2^114 / M from every
 FP32 start within two units in the last place, fix_recip_rn gives the correctly rounded
 double 1 / x, and fix_mul_rn the correctly rounded double product with a float."""
+import math
 import random
 import re
 import struct
@@ -148,3 +150,88 @@ def test_log2_exp2():
         F = k if k < 1000 else M64 - k if k < 2000 else rng.getrandbits(64)
         y = exp2_frac(F, E)
         assert (1 << 63) <= y <= M64 and abs(y - two ** (Decimal(F) / (1 << 64)) * two ** 63) < 40
+
+
+def to_float(m, e):
+    m, e = norm(m, e)
+    return math.ldexp((m >> 40) + ((m >> 39) & 1), e + 40)
+
+
+def series(d2, tail, coefficients):
+    d = d2 >> 32
+    h = tail[1] - umulhi(d, tail[0])
+    h = tail[2] - umulhi(d, h)
+    H = h
+    for c in coefficients:
+        H = c - mul_hi(d2, H)
+    return M64 - mul_hi(d2, H)
+
+
+def sincosf(x):
+    b = fbits(abs(x))
+    if b < 0x39000000:
+        return x, 1.0
+    T = ((b & 0x7FFFFF) | 0x800000) << ((b >> 23) - 87)
+    khi, klo = 0xC90FDAA22168C234, 0xC4C6628B80DC1CD1
+    big, neg = T > khi >> 1, T > khi
+    if big:
+        hi, lo = ((T - khi - 1) & M64, -klo & M64) if neg else (khi - T, klo)
+        z = min(64 - (hi | 1).bit_length(), 63)
+        m, e = ((hi << z) | (lo >> (64 - z)) if z else hi) & M64, -63 - z
+    else:
+        m, e = norm(T, -63)
+    dq = m >> min(-64 - e, 63)
+    d2 = mul_hi(dq, dq)
+    S = series(d2, (0xCA96, 0xD73F9F, 0xB092309D),
+               (0x6B99159FD5, 0x2E3BC74AAD8E, 0xD00D00D00D00D, 0x222222222222222, 0x2AAAAAAAAAAAAAAB))
+    C = series(d2, (0xB41, 0xD73FA, 0xC9CBA54),
+               (0x8F76C77FC, 0x49F93EDDE28, 0x1A01A01A01A02, 0x5B05B05B05B05B, 0xAAAAAAAAAAAAAAB, 0x8000000000000000))
+    sd, cd = to_float(mul_hi(m, S), e), to_float(C, -64)
+    return math.copysign(cd if big else sd, x), ((-sd if neg else sd) if big else cd)
+
+
+def atan2f(y, x, A):
+    lo, hi = sorted((abs(y), abs(x)))
+    lb, hb = fbits(lo), fbits(hi)
+    s = (hb >> 23) - (lb >> 23)
+    assert s <= 60
+    ml, mh = (lb & 0x7FFFFF) | 0x800000, (hb & 0x7FFFFF) | 0x800000
+    swap = abs(y) > abs(x)
+    i = int(f32(f32(lo * f32(1.0 / hi)) * f32(63.9999)))
+    den = mh << s if i else mh
+    N, Dn = (64 * ml - i * den, 64 * den + i * ml) if i else (ml, mh)
+    assert 0 <= N <= M64
+    z = 64 - Dn.bit_length()
+    Y = recip_mant(((Dn << z) & M64) >> 11)
+    nm, ne = norm(N, 0 if i else -s) if N else (0, -63)
+    qm, qe = mul_hi(nm, Y << 1), ne + z - 62
+    qm, qe = norm(qm, qe) if qm else (0, qe - 63)
+    z2 = mul_hi(qm, qm) >> min(-(2 * qe + 128), 63)
+    h = 0x24924925 - umulhi(z2 >> 32, 0x1C71C71C)
+    H = 0x3333333333333333 - mul_hi(z2, h << 32)
+    H = 0x5555555555555555 - mul_hi(z2, H)
+    am = mul_hi(qm, M64 - mul_hi(z2, H))
+    if i == 0 and not swap and x > 0:
+        return math.copysign(to_float(am, qe), y)
+    sh = -61 - qe
+    r = (am >> sh if sh < 64 else 0) + (A[i] >> 2)
+    if swap:
+        r = 0x3243F6A8885A308D - r
+    if x < 0:
+        r = 0x6487ED5110B4611A - r
+    return math.copysign(to_float(r, -61), y)
+
+
+def test_angles():
+    A = table("kAtanT")
+    rng = random.Random(13)
+    half_pi = f32(math.pi / 2)
+    for k in range(20000):
+        x = (half_pi, f32(math.pi / 4))[k] if k < 2 else f32(rng.uniform(-1, 1) * half_pi * 2.0 ** -rng.choice((0, 0, 3, 12, 20)))
+        if x:
+            assert sincosf(x) == (f32(math.sin(x)), f32(math.cos(x)))
+        y, x = f32(rng.gauss(0, 1) * 2.0 ** rng.randint(-30, 2)), f32(rng.gauss(0, 1) * 2.0 ** rng.randint(-3, 3))
+        if k % 3 == 0:
+            y = f32(x * rng.choice((1, -1, 1 / 64, 0.5, 63 / 64)))
+        if x and y:
+            assert atan2f(y, x, A) == f32(math.atan2(y, x))
