@@ -9,12 +9,13 @@
 // decoding (cand_pack32), every candidate is stored and the list grows past the ones
 // that are in, the spline and the viscosity are selections instead of branches, sums
 // and vectors use the packed FP32 instructions, and a record's quarters lie in four
-// arrays (put_rec32): 9,010 instructions a warp instead of 10,440 and 1,940 L1 passes
-// instead of 2,640.  4,194,304-particle lattice (2h cells) 1.453 -> 1.237 ms, 640,000-
-// particle cut 257 -> 215 us, 12 cuts of 1.33 M particles 511 -> 423 us, 121,620-particle
-// rigid cut (cells of h) 63 -> 50 us, 12,000-particle cut 39 -> 31 us.  Products with a
-// common factor as scalars instead of packed with the factor doubled, two pairs a
-// turn, or the list entry fetched a turn ahead were 0-2 % slower.
+// arrays (put_rec32): 9,100 instructions a warp instead of 10,440 and 1,940 L1 passes
+// instead of 2,640.  Every pair term is formed in the order that it was in before,
+// so the results are the same bit for bit.  4,194,304-particle lattice (2h cells) 1.453 ->
+// 1.249 ms, 640,000-particle cut 257 -> 217 us, 12 cuts of 1.33 M particles 511 -> 427 us,
+// 121,620-particle rigid cut (cells of h) 63 -> 50 us, 12,000-particle cut 39 -> 32 us.
+// Products with a common factor as scalars instead of packed with the factor doubled,
+// two pairs a turn, or the list entry fetched a turn ahead were 0-2 % slower.
 #pragma once
 
 #include <type_traits>
@@ -484,7 +485,7 @@ __device__ __forceinline__ void interact32_block(int vb, int N, const KConsts &K
     int marks = 0;   // OR of the flags of the candidates that the entries could not decide
     const float cell8 = 8.f * cell;
     const F2 cell_2 = pk(cell), x_i = pk(xri, yri), v_i = pk(vix, viy), s_i = pk(sAi, sCi), R_i = pk(Rxxi, Ryyi);
-    const float rhoi_half = 0.5f * rhoi, hi_half = 0.5f * hi, c_i = -0.5f * alpha * ci;
+    const float rhoi_half = 0.5f * rhoi, hi_half = 0.5f * hi, ci_half = 0.5f * ci;
     // this particle in the entries' frame; one whose own entry could not decide takes all
     const bool take_all = (fi & (kFlagNonFinite | kFlagFar)) != 0;
     const float y8 = take_all ? __int_as_float(0x7fffffff) : cand_y8(yri, gj & 7, cell);
@@ -574,7 +575,7 @@ __device__ __forceinline__ void interact32_block(int vb, int N, const KConsts &K
             }
             if constexpr (kFused) {
                 const float u = far ? 2.f - q : q, u2 = u * u;
-                float w = far ? u2 * u2 * (kwa * u2) : fmaf(u2, fmaf(kwd, u, kwc), fac);
+                float w = far ? kwa * (u2 * u2 * u2) : fmaf(u2, fmaf(kwd, u, kwc), fac);
                 float dwf = far ? kda * u2 * inv_r : fmaf(kdf, u, kde);
                 if (all && zero_w) w = dwf = 0.f;
                 if (thermal && (!all || !zero_w || rr2 > 1e-16f)) af.tl.add(n2.w * (Ti - n3.w) * dwf);
@@ -587,17 +588,16 @@ __device__ __forceinline__ void interact32_block(int vb, int N, const KConsts &K
                 float fab = w * inv_wdp;
                 fab *= fab;
                 fab *= fab;
-                F2 sd = fma2(pk(fab), R_i + pk(n3.x, n3.y), s_i + pk(n2.x, n2.y));
+                const F2 sd = fma2(pk(fab), R_i + pk(n3.x, n3.y), s_i + pk(n2.x, n2.y));
                 const float sxy = fmaf(fab, Rxyi + n3.z, sBi + n2.z);
                 const float vijposij = -(f2lo(dv) * dx + f2hi(dv) * dy);
                 const float irho = rcp_approx(fmaf(0.5f, n1.z, rhoi_half));
                 const float hij = fmaf(0.5f, n0.w, hi_half);
                 const float muij = hij * vijposij * rcp_approx(fmaf(eta2 * hij, hij, rr2));
-                // (-alpha c_ij mu + beta mu^2) / rho_ij of an approaching pair
-                const float pi = fmaf(beta, muij, fmaf(-0.5f * alpha, n1.w, c_i)) * muij * irho;
+                const float pi = (-alpha * fmaf(0.5f, n1.w, ci_half) * muij + beta * muij * muij) * irho;
+                const F2 sp = sd - pk(vijposij < 0.f ? pi : 0.f);   // viscosity of an approaching pair
                 // acceleration / mass: (stress terms - viscosity) . grad W
-                sd = sd - pk(vijposij < 0.f ? pi : 0.f);
-                af.a.add(fma2(sd, wg, pk(sxy) * pk(f2hi(wg), f2lo(wg))));
+                af.a.add(fma2(pk(f2lo(sp), sxy), pk(f2lo(wg)), pk(sxy, f2hi(sp)) * pk(f2hi(wg))));
                 af.xt.add_product(pk(w * irho), dv);
             } else {
                 float val, der;
