@@ -175,6 +175,7 @@ __global__ void __launch_bounds__(kBlock) k_invalidate(int N, SortedFields A, ui
 // ---- rigid (SPH-mode) tool: tool_gpu.cu, actions_gpu.cu:316-343 ----------------------------------
 // tool::update_tool (tool.cpp:202-212) on the device copy of the tool.
 __global__ void k_rigid_move(sph_rigid_tool *t, double dt) {
+    begin_after();
     if (threadIdx.x == 0 && blockIdx.x == 0) rigid_move(*t, dt);
 }
 
@@ -221,6 +222,7 @@ template <bool kNextHash, class SF>
 __global__ void __launch_bounds__(kBlock) k_step_tail_fem(int N, KConsts K, SF A, SegDev seg,
                                                           const ToolDev *__restrict__ tool, SortScratch X,
                                                           uint32_t *status) {
+    begin_after();
     PARTICLE_LOOP_HEAD
     if (!flag_is_one(A.blanked[i]) && contact_probe(i, K, A, seg, tool)) {
         X.slots[histogram_slot(X.counts, K.g.num_cell + 1)] = i;
@@ -234,6 +236,7 @@ template <bool kNextHash, class SF>
 __global__ void __launch_bounds__(128) k_contact_queue(KConsts K, SF A, SegDev seg, const ToolDev *__restrict__ tool,
                                                        const double *__restrict__ T_nodes, SortScratch X,
                                                        uint32_t *status) {
+    begin_after();
     const int count = X.counts[K.g.num_cell + 1], warps = (int)(gridDim.x * 4u);
     for (int q = (int)(blockIdx.x * 4u + (threadIdx.x >> 5)); q < count; q += warps) {
         const int i = X.slots[q];
@@ -248,6 +251,7 @@ __global__ void __launch_bounds__(kBlock) k_step_tail(int N, KConsts K, SF A, Se
                                                       const ToolDev *__restrict__ tool,
                                                       const double *__restrict__ T_nodes, SortScratch X,
                                                       uint32_t *status) {
+    begin_after();
     PARTICLE_LOOP_HEAD
     step_tail_one<kMode, kNextHash>(i, K, A, X, status);
 }
@@ -410,23 +414,21 @@ template <class SF>
 static void step_tail(cudaStream_t s, int N, const KConsts &K, const SF &A, const SegDev &seg, ToolDev *tool,
                       const double *T_nodes, const SortScratch &X, uint32_t *status, bool next_hash) {
     const int tb = fp64_block(N);   // the rigid contact is FP64 work: spread small systems over all SMs
-#undef GRID
-#define GRID div_up(N, tb), tb, 0, s
     if (K.has_tool) {
         const int grid = std::min(2 * 152, div_up(N, 4));   // a queue of any length; two blocks on each SM
         if (next_hash) {
-            k_step_tail_fem<true><<<GRID>>>(N, K, A, seg, tool, X, status);
-            k_contact_queue<true><<<grid, 128, 0, s>>>(K, A, seg, tool, T_nodes, X, status);
+            launch_after(s, k_step_tail_fem<true, SF>, div_up(N, tb), tb, 0, N, K, A, seg, tool, X, status);
+            launch_after(s, k_contact_queue<true, SF>, grid, 128, 0, K, A, seg, tool, T_nodes, X, status);
         } else {
-            k_step_tail_fem<false><<<GRID>>>(N, K, A, seg, tool, X, status);
-            k_contact_queue<false><<<grid, 128, 0, s>>>(K, A, seg, tool, T_nodes, X, status);
+            launch_after(s, k_step_tail_fem<false, SF>, div_up(N, tb), tb, 0, N, K, A, seg, tool, X, status);
+            launch_after(s, k_contact_queue<false, SF>, grid, 128, 0, K, A, seg, tool, T_nodes, X, status);
         }
     } else if (K.rigid) {
-        if (next_hash) k_step_tail<2, true><<<GRID>>>(N, K, A, seg, tool, T_nodes, X, status);
-        else k_step_tail<2, false><<<GRID>>>(N, K, A, seg, tool, T_nodes, X, status);
+        launch_after(s, next_hash ? k_step_tail<2, true, SF> : k_step_tail<2, false, SF>, div_up(N, tb), tb, 0, N, K, A, seg,
+                     tool, T_nodes, X, status);
     } else {
-        if (next_hash) k_step_tail<0, true><<<GRID>>>(N, K, A, seg, tool, T_nodes, X, status);
-        else k_step_tail<0, false><<<GRID>>>(N, K, A, seg, tool, T_nodes, X, status);
+        launch_after(s, next_hash ? k_step_tail<0, true, SF> : k_step_tail<0, false, SF>, div_up(N, tb), tb, 0, N, K, A, seg,
+                     tool, T_nodes, X, status);
     }
 }
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields &A, const SegDev &seg,
@@ -439,9 +441,7 @@ void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedField
                       bool next_hash) {
     step_tail(s, N, K, A, seg, tool, T_nodes, X, status, next_hash);
 }
-#undef GRID
-#define GRID div_up(N, kBlock), kBlock, 0, s
-void launch_rigid_move(cudaStream_t s, sph_rigid_tool *t, double dt) { k_rigid_move<<<1, 32, 0, s>>>(t, dt); }
+void launch_rigid_move(cudaStream_t s, sph_rigid_tool *t, double dt) { launch_after(s, k_rigid_move, 1, 32, 0, t, dt); }
 void launch_rigid_move_particles(cudaStream_t s, int N, const SortedFields &A, const sph_rigid_tool *t, double dt) {
     k_rigid_move_particles<<<GRID>>>(N, A, t, dt);
 }

@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(kBlock) k_hash_count(int N, const double2 *__r
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int32_t *__restrict__ in, int n,
                                                               int32_t *__restrict__ block_sums) {
+    begin_after();
     __shared__ int sw[32];
     int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     int s = 0;
@@ -60,6 +61,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int32_t *__r
 }
 
 __global__ void __launch_bounds__(1024) k_scan_top(int32_t *__restrict__ block_sums, int nb) {
+    begin_after();
     __shared__ int sw[32];
     int carry = 0;
     for (int base = 0; base < nb; base += blockDim.x) {
@@ -85,6 +87,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(int32_t *__restrict_
                                                             int32_t *__restrict__ offsets,
                                                             int32_t *__restrict__ cell_start,
                                                             int32_t *__restrict__ cell_end, int num_cell) {
+    begin_after();
     __shared__ int sw[32];
     int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     int v[kScanItems];
@@ -131,6 +134,7 @@ __global__ void __launch_bounds__(kBlock) k_scatter(int N, const int32_t *__rest
                                                     const int32_t *__restrict__ arrival,
                                                     const int32_t *__restrict__ offsets, int32_t *__restrict__ slots,
                                                     KConsts K, FemDev F, const ToolDev *__restrict__ tool) {
+    begin_after();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) scatter_one(i, key, arrival, offsets, slots);
     else if (i - N < F.n_nodes) fem_half_one(i - N, K, F, tool);
@@ -272,6 +276,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused(int N, SortScratch X, K
                                                          SortedFields A, SortedFields B, FixedFields F,
                                                          dbl4 *__restrict__ rec64, float2 *__restrict__ cand32,
                                                          const ToolDev *__restrict__ tools, uint32_t *status) {
+    begin_after();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= N) return;
     const int i = X.slots[s], k = rank_of(s, i, X.key, X.offsets, X.slots, status);
@@ -338,6 +343,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused32(int N, SortScratch X,
                                                            int32_t *__restrict__ idx, float4 *__restrict__ rec,
                                                            float2 *__restrict__ cand,
                                                            const ToolDev *__restrict__ tools, uint32_t *status) {
+    begin_after();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= N) return;
     const int i = X.slots[s], k = rank_of(s, i, X.key, X.offsets, X.slots, status);
@@ -417,17 +423,17 @@ int launch_sort_slots(cudaStream_t s, int N, const SortScratch &X, const KConsts
     const sph_geom_constants &g = K.g;
     const int n = g.num_cell + 1;
     const int nb = scan_blocks(g.num_cell);
-    k_scan_reduce<<<nb, kScanThreads, 0, s>>>(X.counts, n, X.block_sums);
+    launch_after(s, k_scan_reduce, nb, kScanThreads, 0, X.counts, n, X.block_sums);
     if (nb <= kScanTopTiles) {
-        k_scan_down<true><<<nb, kScanThreads, 0, s>>>(X.counts, n, X.block_sums, X.offsets, X.cell_start, X.cell_end,
-                                                      g.num_cell);
+        launch_after(s, k_scan_down<true>, nb, kScanThreads, 0, X.counts, n, X.block_sums, X.offsets, X.cell_start,
+                     X.cell_end, g.num_cell);
     } else {
-        k_scan_top<<<1, 1024, 0, s>>>(X.block_sums, nb);
-        k_scan_down<false><<<nb, kScanThreads, 0, s>>>(X.counts, n, X.block_sums, X.offsets, X.cell_start, X.cell_end,
-                                                       g.num_cell);
+        launch_after(s, k_scan_top, 1, 1024, 0, X.block_sums, nb);
+        launch_after(s, k_scan_down<false>, nb, kScanThreads, 0, X.counts, n, X.block_sums, X.offsets, X.cell_start,
+                     X.cell_end, g.num_cell);
     }
-    k_scatter<<<div_up((int64_t)N + F.n_nodes, kBlock), kBlock, 0, s>>>(N, X.key, X.arrival, X.offsets, X.slots, K, F,
-                                                                        tool);
+    launch_after(s, k_scatter, div_up((int64_t)N + F.n_nodes, kBlock), kBlock, 0, N, X.key, X.arrival, X.offsets, X.slots,
+                 K, F, tool);
     return nb <= kScanTopTiles ? 3 : 4;
 }
 void launch_rank(cudaStream_t s, int N, const SortScratch &X, int32_t *perm, uint32_t *status) {
@@ -441,7 +447,7 @@ void launch_gather_plain(cudaStream_t s, int N, const int32_t *perm, const Sorte
 void launch_gather_fused(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const SortedFields &A,
                          const SortedFields &B, const FixedFields &F, const StepScratch &W, const ToolDev *tool) {
     const int tb = fp64_block(N);   // EOS and artificial stress per particle: spread small systems
-    k_gather_fused<<<div_up(N, tb), tb, 0, s>>>(N, X, K, A, B, F, W.rec64, W.cand32, tool, W.status);
+    launch_after(s, k_gather_fused, div_up(N, tb), tb, 0, N, X, K, A, B, F, W.rec64, W.cand32, tool, W.status);
 }
 
 void launch_gather_fused32(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const SortedFields *A64,
@@ -449,13 +455,17 @@ void launch_gather_fused32(cudaStream_t s, int N, const SortScratch &X, const KC
                            const SortedFields32 &B, int32_t *idx, const StepScratch &W, const ToolDev *tool) {
     const int tb = fp64_block(N), g = div_up(N, tb);
     if (A32 && pr32)
-        k_gather_fused32<<<g, tb, 0, s>>>(N, X, K, *A32, F32, B, F32, idx, W.rec32, W.cand32, tool, W.status);
+        launch_after(s, k_gather_fused32<SortedFields32, FixedFields32>, g, tb, 0, N, X, K, *A32, F32, B, F32, idx,
+                     W.rec32, W.cand32, tool, W.status);
     else if (A32)
-        k_gather_fused32<<<g, tb, 0, s>>>(N, X, K, *A32, F, B, F32, idx, W.rec32, W.cand32, tool, W.status);
+        launch_after(s, k_gather_fused32<SortedFields32, FixedFields>, g, tb, 0, N, X, K, *A32, F, B, F32, idx, W.rec32,
+                     W.cand32, tool, W.status);
     else if (pr32)
-        k_gather_fused32<<<g, tb, 0, s>>>(N, X, K, *A64, F32, B, F32, idx, W.rec32, W.cand32, tool, W.status);
+        launch_after(s, k_gather_fused32<SortedFields, FixedFields32>, g, tb, 0, N, X, K, *A64, F32, B, F32, idx, W.rec32,
+                     W.cand32, tool, W.status);
     else
-        k_gather_fused32<<<g, tb, 0, s>>>(N, X, K, *A64, F, B, F32, idx, W.rec32, W.cand32, tool, W.status);
+        launch_after(s, k_gather_fused32<SortedFields, FixedFields>, g, tb, 0, N, X, K, *A64, F, B, F32, idx, W.rec32,
+                     W.cand32, tool, W.status);
 }
 
 void launch_state_to64(cudaStream_t s, int N, const SortedFields32 &A, const FixedFields32 &Fa, const SortedFields &B,

@@ -19,6 +19,7 @@ namespace sphfem {
 template <bool kMove>
 __global__ void __launch_bounds__(kBlock) k_fem_rate_update(KConsts K, FemDev F, SegDev seg,
                                                             const ToolDev *__restrict__ tool) {
+    begin_after();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= F.n_nodes) return;
     fem_rate_update_one(i, K, F, seg, tool);
@@ -30,6 +31,7 @@ __global__ void __launch_bounds__(kBlock) k_fem_rate_update(KConsts K, FemDev F,
 
 // One block per case: its segments and tool state move, then its y-bins.
 __global__ void __launch_bounds__(kBlock) k_tool_cases(SegDev seg, ToolDev *tool) {
+    begin_after();
     ToolDev &tc = tool[blockIdx.x];
     for (int q = threadIdx.x; q < tc.seg_count; q += blockDim.x)
         segment_move(seg, tc.seg_first + q, tc.vel, tc.dt, tc.flank_retreat);
@@ -85,11 +87,10 @@ __global__ void __launch_bounds__(kBlock) k_tool_move(KConsts K, SegDev seg, Fem
 void launch_fem_rate_update(cudaStream_t s, const KConsts &K, const FemDev &F, const SegDev &seg,
                             const ToolDev *tool, bool move_nodes) {
     const int grid = div_up(F.n_nodes, kBlock);
-    if (move_nodes) k_fem_rate_update<true><<<grid, kBlock, 0, s>>>(K, F, seg, tool);
-    else k_fem_rate_update<false><<<grid, kBlock, 0, s>>>(K, F, seg, tool);
+    launch_after(s, move_nodes ? k_fem_rate_update<true> : k_fem_rate_update<false>, grid, kBlock, 0, K, F, seg, tool);
 }
 void launch_tool_cases(cudaStream_t s, int n_cases, const SegDev &seg, ToolDev *tool) {
-    k_tool_cases<<<n_cases, kBlock, 0, s>>>(seg, tool);
+    launch_after(s, k_tool_cases, n_cases, kBlock, 0, seg, tool);
 }
 void launch_fem_reset(cudaStream_t s, const FemDev &F, double *T_old, double *f_temp, double *K_temp) {
     k_fem_reset<<<div_up(F.nnz > F.n_nodes ? F.nnz : F.n_nodes, kBlock), kBlock, 0, s>>>(F, T_old, f_temp, K_temp);

@@ -709,6 +709,7 @@ __global__ void __launch_bounds__(kB, kMinB) k_interact32(int N, KConsts K, cons
                                                        const ToolDev *__restrict__ tool,
                                                        int32_t *__restrict__ secant_iters, uint32_t *status,
                                                        int cap, MlpDev mlp) {
+    begin_after();
     interact32_block<kFused, kB, kStaged, kMlp, kSplit>(blockIdx.x, N, K, offsets, rec, cand, B, F, seg, tool,
                                                         secant_iters, status, cap, mlp);
 }
@@ -727,8 +728,8 @@ static void launch_i32(cudaStream_t s, int N, const KConsts &K, const int32_t *o
             configured = true;
         }
     }
-    k_interact32<true, kB, kMinB, kStaged, kMlp, kSplit><<<div_up(N, kB / kSplit), kB, smem, s>>>(
-        N, K, offsets, W.rec32, W.cand32, B, F, seg, tool, W.secant_iters, W.status, cap, mlp);
+    launch_after(s, k_interact32<true, kB, kMinB, kStaged, kMlp, kSplit>, div_up(N, kB / kSplit), kB, smem, N, K, offsets,
+                 W.rec32, W.cand32, B, F, seg, tool, W.secant_iters, W.status, cap, mlp);
 }
 
 // The launch shapes of kInteractVariants (interactions.cu), in its order.

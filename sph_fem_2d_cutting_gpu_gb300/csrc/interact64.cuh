@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(kThreads64, 5) k_interact64(int N, KConsts K, 
                                                               FixedFields F, SegDev seg,
                                                               const ToolDev *__restrict__ tool,
                                                               int32_t *__restrict__ secant_iters, uint32_t *status) {
+    begin_after();
     constexpr int kSums = kFused ? 9 : 13;
     __shared__ int s_list[kParts64 * kListPitch64];
     __shared__ double s_sum[kSums][kThreads64];

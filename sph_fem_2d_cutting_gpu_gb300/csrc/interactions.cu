@@ -85,6 +85,7 @@ static __device__ __noinline__ double pse_weight_general(double rr2, double inv_
 __global__ void __launch_bounds__(128) k_heat_pse64(int N, KConsts K, const int32_t *__restrict__ offsets,
                                                     const dbl4 *__restrict__ rec,
                                                     const int32_t *__restrict__ hashes, double *__restrict__ T_t) {
+    begin_after();
     const int k = (int)(blockIdx.x * 128u + threadIdx.x) / kPseLanes, sub = (int)threadIdx.x % kPseLanes;
     const int kk = min(k, N - 1);
     const dbl4 i0 = rec[4 * kk + 0], i2 = rec[4 * kk + 2], i3 = rec[4 * kk + 3];
@@ -140,6 +141,7 @@ template <class TT>   // T_t: double (staged call, FP64 arrays) or float (the co
 __global__ void __launch_bounds__(kBlock) k_heat_pse32(int N, KConsts K, const int32_t *__restrict__ offsets,
                                                        const float4 *__restrict__ rec,
                                                        const int32_t *__restrict__ hashes, TT *__restrict__ T_t) {
+    begin_after();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= N) return;
     const float4 *rec_c = rec + 2 * (size_t)N, *rec_d = rec + 3 * (size_t)N;   // the records' last two quarters
@@ -178,7 +180,7 @@ __global__ void __launch_bounds__(kBlock) k_heat_pse32(int N, KConsts K, const i
 void launch_heat_pse(cudaStream_t s, int N, const KConsts &K, const int32_t *offsets, const StepScratch &W,
                      const SortedFields32 &B) {
     const int tb = fp64_block(N);
-    k_heat_pse32<<<div_up(N, tb), tb, 0, s>>>(N, K, offsets, W.rec32, B.hash, B.T_t);
+    launch_after(s, k_heat_pse32<float>, div_up(N, tb), tb, 0, N, K, offsets, W.rec32, B.hash, B.T_t);
 }
 
 void launch_heat_pse(cudaStream_t s, int N, const KConsts &K, const int32_t *offsets, const StepScratch &W,
@@ -188,7 +190,7 @@ void launch_heat_pse(cudaStream_t s, int N, const KConsts &K, const int32_t *off
         k_heat_pse32<<<div_up(N, tb), tb, 0, s>>>(N, K, offsets, W.rec32, B.hash, B.T_t);
         return;
     }
-    k_heat_pse64<<<div_up((int64_t)N * kPseLanes, 128), 128, 0, s>>>(N, K, offsets, W.rec64, B.hash, B.T_t);
+    launch_after(s, k_heat_pse64, div_up((int64_t)N * kPseLanes, 128), 128, 0, N, K, offsets, W.rec64, B.hash, B.T_t);
 }
 
 void launch_interactions32_fused(cudaStream_t s, int N, const KConsts &K, const int32_t *offsets,
@@ -208,8 +210,8 @@ void launch_interactions(cudaStream_t s, int N, const KConsts &K, const int32_t 
     } else {
         const int g64 = div_up(N, kParts64);
         if (fused)
-            k_interact64<true><<<g64, kThreads64, 0, s>>>(N, K, offsets, W.rec64, W.cand32, B, F, seg, tool,
-                                                          W.secant_iters, W.status);
+            launch_after(s, k_interact64<true>, g64, kThreads64, 0, N, K, offsets, W.rec64, W.cand32, B, F, seg, tool,
+                         W.secant_iters, W.status);
         else
             k_interact64<false><<<g64, kThreads64, 0, s>>>(N, K, offsets, W.rec64, W.cand32, B, F, seg, tool,
                                                            W.secant_iters, W.status);

@@ -7,6 +7,25 @@
 
 namespace sphfem {
 
+// A launch whose kernel starts with begin_after(): its blocks may take their places while
+// the kernel before it in the stream finishes.  The step is a chain of short kernels on
+// a small system, and launching each only when the last one is done cost it 1-2 us a
+// kernel.
+template <class... P, class... A>
+inline void launch_after(cudaStream_t s, void (*k)(P...), int grid, int block, size_t smem, A &&...a) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, k, P(a)...);
+}
+
 // cells.cu
 void launch_hash(cudaStream_t s, int N, const SortedFields &A, sph_geom_constants g);
 void launch_count(cudaStream_t s, int N, const SortedFields &A, const SortScratch &X, sph_geom_constants g,
