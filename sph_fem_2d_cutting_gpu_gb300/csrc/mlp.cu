@@ -6,9 +6,9 @@
 // The 64x64 hidden layers run on the 5th-generation tensor cores: operands in
 // shared memory in the no-swizzle K-major layout, tcgen05.mma issued by one
 // thread, accumulators in TMEM, completion through tcgen05.commit on an
-// mbarrier.  A tile is 128 samples = 128 threads = the 128 TMEM lanes of an
-// M=128 accumulator, so thread r reads row r with tcgen05.ld 32x32b and keeps
-// its sample's activations in registers between layers.  In training the two
+// mbarrier.  A tile is 128 samples = the 128 TMEM lanes of an M=128 accumulator,
+// read with tcgen05.ld 32x32b: one thread for each sample in inference, four
+// (16 neurons each) in training.  In training the two
 // 64x64 weight gradients of a tile are one M=128, N=128, K=128 MMA
 // ([dZ3^T; dZ2^T] x [A2 | A1]: the two diagonal blocks are dW3 and dW2) that
 // accumulates in TMEM over all tiles of the CTA.
@@ -24,7 +24,7 @@
 namespace sphfem {
 namespace {
 
-constexpr int kTile = 128;                 // samples per tile = threads per CTA
+constexpr int kTile = 128;                 // samples per tile (inference: threads per CTA)
 constexpr uint32_t kTmemCols = 256;        // training: [0,64) layer, [64,192) stacked dW
 constexpr uint32_t kTmemColsFwd = 64;      // inference
 
@@ -103,37 +103,20 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// This thread's row of a 64-column accumulator starting at column `col`.
-__device__ __forceinline__ void tmem_row64(uint32_t tmem, uint32_t col, float *v) {
-    const uint32_t lane = (threadIdx.x >> 5) * 32u;
-    const uint32_t a = tmem + (lane << 16) + col;
-    tmem_ld16(a, v);
-    tmem_ld16(a + 16, v + 16);
-    tmem_ld16(a + 32, v + 32);
-    tmem_ld16(a + 48, v + 48);
-}
+// d silu(z) / dz from the sigmoid s of z.
+__device__ __forceinline__ float dsiluf_(float z, float s) { return s * (1.f + z * (1.f - s)); }
 
-__device__ __forceinline__ float dsiluf_(float z) {
-    float s = sigmoidf_(z);
-    return s * (1.f + z * (1.f - s));
-}
-__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-
-// Row r of a K-major 64-column operand from 64 floats (rounded to BF16).
-__device__ __forceinline__ void store_row64(unsigned char *base, int r, const float *v) {
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-        uint4 q = make_uint4(pack_bf16x2(v[8 * c + 0], v[8 * c + 1]), pack_bf16x2(v[8 * c + 2], v[8 * c + 3]),
-                             pack_bf16x2(v[8 * c + 4], v[8 * c + 5]), pack_bf16x2(v[8 * c + 6], v[8 * c + 7]));
-        *(uint4 *)(base + cm_off(r, 8 * c, 64)) = q;
-    }
-}
-
-// Column k of a K-major 128-column operand, rows row0..row0+63, from 64 floats
-// (the transposed copies that feed the weight-gradient MMA).
-__device__ __forceinline__ void store_col(unsigned char *base, int row0, int k, const float *v) {
-#pragma unroll
-    for (int j = 0; j < 64; j++) *(__nv_bfloat16 *)(base + cm_off(row0 + j, k, 128)) = __float2bfloat16_rn(v[j]);
+// Four 8x8 BF16 core matrices (128 contiguous bytes each) transposed from shared to
+// shared memory by one warp; lane l passes the address of row l & 7 of matrix l >> 3.
+__device__ __forceinline__ void transpose_cores(uint32_t dst, uint32_t src) {
+    uint32_t a, b, c, d;
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(a), "=r"(b), "=r"(c), "=r"(d)
+                 : "r"(src)
+                 : "memory");
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(a), "r"(b), "r"(c),
+                 "r"(d)
+                 : "memory");
 }
 
 // Shared parameter block of a CTA (FP32 values of the BF16 weights of the
@@ -153,32 +136,12 @@ __device__ void load_small(MlpSmall &s, const MlpDev &m) {
     if (threadIdx.x == 0) s.b4 = m.params[kMlpOffB4];
 }
 
-// W [64 out][64 in] as the B operand of X W^T (rows n = out, K = in), or
-// transposed (rows n = in, K = out) as the B operand of dZ W.
-__device__ void load_weight(unsigned char *dst, const uint16_t *w, bool transpose) {
-    if (!transpose) {   // 8 consecutive inputs of one output = one 16-byte core-matrix row
-        for (int i = threadIdx.x; i < kMlpH * kMlpH / 8; i += blockDim.x) {
-            const int o = i >> 3, k8 = (i & 7) * 8;
-            *(uint4 *)(dst + cm_off(o, k8, 64)) = *(const uint4 *)(w + o * kMlpH + k8);
-        }
-        return;
-    }
-    for (int i = threadIdx.x; i < kMlpH * kMlpH; i += blockDim.x) {
-        int o = i >> 6, in = i & 63;
-        int n = transpose ? in : o, k = transpose ? o : in;
-        *(uint16_t *)(dst + cm_off(n, k, 64)) = w[i];
-    }
-}
-
-
-__device__ __forceinline__ void layer1(const MlpSmall &s, const float *xn, float *a, float *z) {
-#pragma unroll
-    for (int j = 0; j < kMlpH; j++) {
-        float acc = s.b1[j];
-#pragma unroll
-        for (int c = 0; c < kMlpIn; c++) acc = fmaf(s.w1[j * kMlpIn + c], xn[c], acc);
-        if (z) z[j] = acc;
-        a[j] = siluf_(acc);
+// W [64 out][64 in] as the B operand of X W^T (rows n = out, K = in): 8 consecutive
+// inputs of one output are one 16-byte core-matrix row.
+__device__ void load_weight(unsigned char *dst, const uint16_t *w) {
+    for (int i = threadIdx.x; i < kMlpH * kMlpH / 8; i += blockDim.x) {
+        const int o = i >> 3, k8 = (i & 7) * 8;
+        *(uint4 *)(dst + cm_off(o, k8, 64)) = *(const uint4 *)(w + o * kMlpH + k8);
     }
 }
 
@@ -193,8 +156,6 @@ struct FwdSmem {
     int fail;
 };
 
-// Forward pass of this CTA's tile; xn = standardised features of this
-// thread's row.  Returns the standardised output, or sets *timeout.
 // 16 columns [c0, c0+16) of row r of a K-major 64-column operand (BF16).
 __device__ __forceinline__ void store_row16(unsigned char *base, int r, int c0, const float *v) {
 #pragma unroll
@@ -272,8 +233,8 @@ __device__ bool fwd_setup(FwdSmem &sh, const MlpDev &m, uint32_t &tmem) {
         sh.fail = 0;
     }
     load_small(sh.small, m);
-    load_weight(sh.w2, m.wb + kMlpWbW2, false);
-    load_weight(sh.w3, m.wb + kMlpWbW3, false);
+    load_weight(sh.w2, m.wb + kMlpWbW2);
+    load_weight(sh.w3, m.wb + kMlpWbW3);
     if (threadIdx.x < 32) tmem_alloc(smem_u32(&sh.tmem_slot), kTmemColsFwd);
     tc_fence_before();
     __syncthreads();
@@ -372,6 +333,8 @@ __global__ void __launch_bounds__(kTile, 1)
 }
 
 // ---- training: gradients of one minibatch ---------------------------------------------------------
+constexpr int kTrainThreads = 512;   // four threads for each sample of a tile, 16 neurons each
+
 struct TrainSmem {
     alignas(128) unsigned char w2f[kMlpH * kMlpH * 2];   // W2 as B of A1 W2^T
     alignas(128) unsigned char w3f[kMlpH * kMlpH * 2];
@@ -380,60 +343,98 @@ struct TrainSmem {
     alignas(128) unsigned char act[kTile * kMlpH * 2];   // A operand of the 64-wide GEMMs
     alignas(128) unsigned char adw[kTile * kTile * 2];   // [dZ3^T; dZ2^T]  (rows: neurons, K: samples)
     alignas(128) unsigned char bdw[kTile * kTile * 2];   // [A2^T; A1^T]
-    float zs[kTile][kMlpH + 1];                          // Z2 of each sample, then dZ1
-    float xn[kTile][kMlpIn];
-    float dw4[4][kMlpH];
+    float zs[kTile][kMlpH + 1];                          // A3 of each sample, then dZ1; at the end the sums to merge
+    alignas(16) float xn[kTile][kMlpIn];
+    float g[kTile];                                      // d loss / dy of each sample
     float db4[4], loss[4];
     MlpSmall small;
-    alignas(8) unsigned long long mbar;
+    alignas(8) unsigned long long mbar, mbar_dw;
     uint32_t tmem_slot;
 };
 
 // Per-CTA partial sums over the samples of its tiles, written to
 // part[blockIdx.x][0..kMlpParams) (gradient of the mean loss) and
 // part[..][kMlpParams] (sum of 0.5 (y - t)^2 in standardised units).
-__global__ void __launch_bounds__(kTile, 1)
+//
+// A tile's chain is five MMAs with the SiLU of 128 x 64 values between them, so it is
+// bound by the latency of that chain and by the sigmoids (three for each sample and
+// neuron, each with its derivative).  With one thread for each sample the 64-wide
+// register rows unrolled into code far larger than the instruction cache and one warp
+// in flight on each scheduler: 50 us a tile.  Four threads for each sample (16 neurons
+// each: straight-line code, four warps on each scheduler), the sigmoids evaluated once,
+// the transposed operands of the weight gradient made from the stored ones by
+// ldmatrix / stmatrix while the layer's MMA runs, and sums over the samples split over
+// all threads: 65,536 samples (512 tiles on 152 SMs) 226 -> 48 us; 8,192 samples 92 -> 19 us.
+__global__ void __launch_bounds__(kTrainThreads, 1)
     k_mlp_grad(MlpDev m, const float *__restrict__ x, const float *__restrict__ tgt, const int32_t *__restrict__ idx,
                int64_t nb, float inv_nb, float *__restrict__ part, uint32_t *status) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     TrainSmem &sh = *(TrainSmem *)smem_raw;
-    const int r = threadIdx.x, warp = r >> 5, lane = r & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int r = tid & (kTile - 1), c0 = 16 * (tid >> 7);   // this thread's sample (TMEM lane) and first neuron
+    const int nj = tid & (kMlpH - 1), ns = 16 * (tid >> 6);  // in sums over samples: its neuron and first sample
     float *out = part + (size_t)blockIdx.x * (kMlpParams + 1);
     const int64_t ntiles = (nb + kTile - 1) / kTile;
     if ((int64_t)blockIdx.x >= ntiles) {
-        for (int i = r; i < kMlpParams + 1; i += kTile) out[i] = 0.f;
+        for (int i = tid; i < kMlpParams + 1; i += kTrainThreads) out[i] = 0.f;
         return;
     }
-    const uint32_t mbar = smem_u32(&sh.mbar);
-    if (r == 0) mbar_init(mbar);
+    const uint32_t mbar = smem_u32(&sh.mbar), mbar_dw = smem_u32(&sh.mbar_dw);
+    const uint32_t act = smem_u32(sh.act), adw = smem_u32(sh.adw), bdw = smem_u32(sh.bdw);
+    if (tid == 0) {
+        mbar_init(mbar);
+        mbar_init(mbar_dw);
+    }
     load_small(sh.small, m);
-    load_weight(sh.w2f, m.wb + kMlpWbW2, false);
-    load_weight(sh.w3f, m.wb + kMlpWbW3, false);
-    load_weight(sh.w2b, m.wb + kMlpWbW2, true);
-    load_weight(sh.w3b, m.wb + kMlpWbW3, true);
-    for (int i = r; i < 4 * kMlpH; i += kTile) (&sh.dw4[0][0])[i] = 0.f;
-    if (r < 4) { sh.db4[r] = 0.f; sh.loss[r] = 0.f; }
+    load_weight(sh.w2f, m.wb + kMlpWbW2);
+    load_weight(sh.w3f, m.wb + kMlpWbW3);
     if (warp == 0) tmem_alloc(smem_u32(&sh.tmem_slot), kTmemCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh.tmem_slot;
-    uint32_t phase = 0;
+    const uint32_t trow = tmem + ((uint32_t)(warp & 3) * 32u << 16) + (uint32_t)c0;
+    {   // the transposed weights: warp w does the 8 outputs of group w / 2 and 32 inputs
+        const uint32_t o = (uint32_t)(warp >> 1), i = (uint32_t)(4 * (warp & 1) + (lane >> 3)), b = 16u * (lane & 7);
+        transpose_cores(smem_u32(sh.w2b) + i * 1024 + o * 128 + b, smem_u32(sh.w2f) + o * 1024 + i * 128 + b);
+        transpose_cores(smem_u32(sh.w3b) + i * 1024 + o * 128 + b, smem_u32(sh.w3f) + o * 1024 + i * 128 + b);
+    }
+    uint32_t phase = 0, phase_dw = 0;
     bool timeout = false;
-    // per-thread accumulators: thread j < 64 owns dW1[j][:], db1[j], db3[j]; thread 64 + j owns db2[j]
-    float acc_w1[kMlpIn] = {0.f, 0.f, 0.f, 0.f}, acc_b1 = 0.f, acc_b23 = 0.f;
+    // sums of this thread: dW1[nj][:], db1[nj], dW4[nj] over its samples; db3 / db2 of row r of
+    // adw over its quarter of the samples; threads of the first 16 neurons: db4 and the loss
+    float acc_w1[kMlpIn] = {0.f, 0.f, 0.f, 0.f}, acc_b1 = 0.f, acc_w4 = 0.f, acc_b23 = 0.f, acc_b4 = 0.f, acc_loss = 0.f;
     int tiles_done = 0;
-    float v[kMlpH];
+    float v[16], d1[16], d2[16];
 
-    auto mma_wait = [&]() -> bool {
-        bool ok = mbar_wait(mbar, phase);
-        phase ^= 1u;
-        return !__syncthreads_or(!ok);
+    auto mma_wait = [&](uint32_t bar, uint32_t &ph) -> bool {
+        bool ok = mbar_wait(bar, ph);
+        ph ^= 1u;
+        const bool all = !__syncthreads_or(!ok);
+        tc_fence_after();
+        return all;
     };
     auto sync_for_mma = [&]() {
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
+    };
+    auto issue = [&](const unsigned char *w) {   // layer accumulator = act w^T
+        if (tid == 0) {
+            tc_fence_after();
+            gemm_issue(tmem, act, smem_u32(w), 64, 64, false);
+            mma_commit(mbar);
+        }
+    };
+    // act^T (64 neurons x 128 samples) into rows row0.. of an operand of the weight gradient:
+    // a warp does 8 samples
+    auto transpose_act = [&](uint32_t dst, int row0) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t ng = (uint32_t)(4 * h + (lane >> 3)), b = 16u * (lane & 7);
+            transpose_cores(dst + ((uint32_t)(row0 >> 3) + ng) * 2048u + (uint32_t)warp * 128u + b,
+                            act + (uint32_t)warp * 1024u + ng * 128u + b);
+        }
     };
 
     for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -444,128 +445,105 @@ __global__ void __launch_bounds__(kTile, 1)
             const int64_t i = idx ? idx[e] : e;
             float4 q = *(const float4 *)(x + 4 * i);
             xr[0] = q.x; xr[1] = q.y; xr[2] = q.z; xr[3] = q.w;
-            tn = (tgt[i] - m.y_mean) / m.y_std;
+            if (c0 == 0) tn = (tgt[i] - m.y_mean) / m.y_std;
         }
         normalise(m, xr, xn);
+        if (c0 == 0) *(float4 *)sh.xn[r] = make_float4(xn[0], xn[1], xn[2], xn[3]);
+        // layer 1 (CUDA cores)
 #pragma unroll
-        for (int c = 0; c < kMlpIn; c++) sh.xn[r][c] = xn[c];
-        // layer 1 (CUDA cores): A1 -> act and bdw rows 64..127
-        layer1(sh.small, xn, v, nullptr);
+        for (int q = 0; q < 16; q++) {
+            float z = sh.small.b1[c0 + q];
 #pragma unroll
-        for (int jj = 0; jj < kMlpH; jj++) v[jj] = bf16_round(v[jj]);
-        store_row64(sh.act, r, v);
-        store_col(sh.bdw, 64, r, v);
+            for (int c = 0; c < kMlpIn; c++) z = fmaf(sh.small.w1[(c0 + q) * kMlpIn + c], xn[c], z);
+            const float s = sigmoidf_(z);
+            d1[q] = dsiluf_(z, s);
+            v[q] = z * s;
+        }
+        store_row16(sh.act, r, c0, v);
         // layer 2: Z2 = A1 W2^T + b2
         sync_for_mma();
-        if (r == 0) {
-            tc_fence_after();
-            gemm_issue(tmem, smem_u32(sh.act), smem_u32(sh.w2f), 64, 64, false);
-            mma_commit(mbar);
-        }
-        if (!mma_wait()) { timeout = true; break; }
-        tc_fence_after();
-        tmem_row64(tmem, 0, v);
+        issue(sh.w2f);
+        transpose_act(bdw, 64);   // A1^T
+        if (!mma_wait(mbar, phase)) { timeout = true; break; }
+        tmem_ld16(trow, v);
 #pragma unroll
-        for (int jj = 0; jj < kMlpH; jj++) {
-            v[jj] += sh.small.b2[jj];
-            sh.zs[r][jj] = v[jj];
-            v[jj] = bf16_round(siluf_(v[jj]));
+        for (int q = 0; q < 16; q++) {
+            const float z = v[q] + sh.small.b2[c0 + q], s = sigmoidf_(z);
+            d2[q] = dsiluf_(z, s);
+            v[q] = z * s;
         }
-        tc_fence_before();
-        __syncthreads();
-        store_row64(sh.act, r, v);
-        store_col(sh.bdw, 0, r, v);
+        store_row16(sh.act, r, c0, v);
         // layer 3: Z3 = A2 W3^T + b3, output, dZ3
         sync_for_mma();
-        if (r == 0) {
+        issue(sh.w3f);
+        transpose_act(bdw, 0);   // A2^T
+        if (!mma_wait(mbar, phase)) { timeout = true; break; }
+        tmem_ld16(trow, v);
+#pragma unroll
+        for (int q = 0; q < 16; q++) {
+            const float z = v[q] + sh.small.b3[c0 + q], s = sigmoidf_(z);
+            sh.zs[r][c0 + q] = z * s;
+            v[q] = dsiluf_(z, s);
+        }
+        __syncthreads();
+        if (c0 == 0) {   // the output: one thread for each sample
+            float y = sh.small.b4;
+#pragma unroll 16
+            for (int j = 0; j < kMlpH; j++) y = fmaf(sh.small.w4[j], sh.zs[r][j], y);
+            const float err = valid ? (y - tn) : 0.f;
+            const float g = err * inv_nb;
+            sh.g[r] = g;
+            acc_b4 += g;
+            acc_loss = fmaf(0.5f * err, err, acc_loss);
+        }
+        __syncthreads();
+        {
+            const float g = sh.g[r];
+#pragma unroll
+            for (int q = 0; q < 16; q++) v[q] = g * sh.small.w4[c0 + q] * v[q];
+        }
+        store_row16(sh.act, r, c0, v);   // dZ3 as A of dA2 = dZ3 W3
+        sync_for_mma();
+        issue(sh.w3b);
+        transpose_act(adw, 0);           // dZ3^T
+#pragma unroll
+        for (int s = 0; s < 16; s++) acc_w4 = fmaf(sh.g[ns + s], sh.zs[ns + s][nj], acc_w4);
+        if (!mma_wait(mbar, phase)) { timeout = true; break; }
+        tmem_ld16(trow, v);
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = v[q] * d2[q];
+        store_row16(sh.act, r, c0, v);   // dZ2 as A of dA1 = dZ2 W2
+        sync_for_mma();
+        issue(sh.w2b);
+        transpose_act(adw, 64);          // dZ2^T
+        // [dW3 | . ; . | dW2] += [dZ3^T; dZ2^T] [A2 | A1] over this tile's samples
+        sync_for_mma();
+        if (tid == 0) {
             tc_fence_after();
-            gemm_issue(tmem, smem_u32(sh.act), smem_u32(sh.w3f), 64, 64, false);
-            mma_commit(mbar);
+            gemm_issue(tmem + 64, adw, bdw, 128, 128, tiles_done > 0);
+            mma_commit(mbar_dw);
         }
-        if (!mma_wait()) { timeout = true; break; }
-        tc_fence_after();
-        tmem_row64(tmem, 0, v);
-        float y = sh.small.b4;
+        if (!mma_wait(mbar, phase)) { timeout = true; break; }
+        tmem_ld16(trow, v);
 #pragma unroll
-        for (int jj = 0; jj < kMlpH; jj++) {
-            v[jj] += sh.small.b3[jj];
-            y = fmaf(sh.small.w4[jj], siluf_(v[jj]), y);
-        }
-        const float err = valid ? (y - tn) : 0.f;
-        const float g = err * inv_nb;
-        // dW4 = sum g a3, db4 = sum g (warp sums, then per-warp slots)
+        for (int q = 0; q < 16; q++) sh.zs[r][c0 + q] = v[q] * d1[q];   // dZ1 (FP32)
+        tc_fence_before();
+        __syncthreads();
 #pragma unroll
-        for (int jj = 0; jj < kMlpH; jj++) {
-            float c = g * siluf_(v[jj]);
-            for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-            if (lane == 0) sh.dw4[warp][jj] += c;
+        for (int s = 0; s < 16; s++) {
+            const float d = sh.zs[ns + s][nj];
+            const float4 xs = *(const float4 *)sh.xn[ns + s];
+            acc_b1 += d;
+            acc_w1[0] = fmaf(d, xs.x, acc_w1[0]);
+            acc_w1[1] = fmaf(d, xs.y, acc_w1[1]);
+            acc_w1[2] = fmaf(d, xs.z, acc_w1[2]);
+            acc_w1[3] = fmaf(d, xs.w, acc_w1[3]);
         }
         {
-            float c = g, l = 0.5f * err * err;
-            for (int o = 16; o > 0; o >>= 1) {
-                c += __shfl_xor_sync(0xffffffffu, c, o);
-                l += __shfl_xor_sync(0xffffffffu, l, o);
-            }
-            if (lane == 0) { sh.db4[warp] += c; sh.loss[warp] += l; }
-        }
-#pragma unroll
-        for (int jj = 0; jj < kMlpH; jj++) v[jj] = bf16_round(g * sh.small.w4[jj] * dsiluf_(v[jj]));
-        tc_fence_before();
-        __syncthreads();
-        store_row64(sh.act, r, v);   // dZ3 as A of dA2 = dZ3 W3
-        store_col(sh.adw, 0, r, v);  // dZ3^T
-        sync_for_mma();
-        if (r == 0) {
-            tc_fence_after();
-            gemm_issue(tmem, smem_u32(sh.act), smem_u32(sh.w3b), 64, 64, false);
-            mma_commit(mbar);
-        }
-        if (!mma_wait()) { timeout = true; break; }
-        tc_fence_after();
-        tmem_row64(tmem, 0, v);
-#pragma unroll
-        for (int jj = 0; jj < kMlpH; jj++) v[jj] = bf16_round(v[jj] * dsiluf_(sh.zs[r][jj]));
-        tc_fence_before();
-        __syncthreads();
-        store_row64(sh.act, r, v);    // dZ2 as A of dA1 = dZ2 W2
-        store_col(sh.adw, 64, r, v);  // dZ2^T
-        // [dW3 | . ; . | dW2] += [dZ3^T; dZ2^T] [A2 | A1] over this tile's samples, and dA1
-        sync_for_mma();
-        if (r == 0) {
-            tc_fence_after();
-            gemm_issue(tmem + 64, smem_u32(sh.adw), smem_u32(sh.bdw), 128, 128, tiles_done > 0);
-            gemm_issue(tmem, smem_u32(sh.act), smem_u32(sh.w2b), 64, 64, false);
-            mma_commit(mbar);
-        }
-        if (!mma_wait()) { timeout = true; break; }
-        tc_fence_after();
-        tmem_row64(tmem, 0, v);
-#pragma unroll
-        for (int jj = 0; jj < kMlpH; jj++) {   // dZ1 = dA1 * silu'(Z1) (FP32), Z1 recomputed
-            float z = sh.small.b1[jj];
-#pragma unroll
-            for (int c = 0; c < kMlpIn; c++) z = fmaf(sh.small.w1[jj * kMlpIn + c], xn[c], z);
-            v[jj] *= dsiluf_(z);
-        }
-        tc_fence_before();
-        __syncthreads();   // zs (Z2) no longer needed by any thread
-#pragma unroll
-        for (int jj = 0; jj < kMlpH; jj++) sh.zs[r][jj] = v[jj];
-        __syncthreads();
-        if (r < kMlpH) {
-            // dW1 row r, db1[r]; db3[r] = sum over samples of dZ3[:, r] (row r of adw)
-            for (int s2 = 0; s2 < kTile; s2++) {
-                const float d = sh.zs[s2][r];
-                acc_b1 += d;
-#pragma unroll
-                for (int c = 0; c < kMlpIn; c++) acc_w1[c] = fmaf(d, sh.xn[s2][c], acc_w1[c]);
-            }
-        }
-        {
-            // db3 (threads < 64) or db2 (threads >= 64): sum of row r of adw
             float sum = 0.f;
-            for (int k8 = 0; k8 < kTile; k8 += 8) {
-                uint4 q = *(const uint4 *)(sh.adw + cm_off(r, k8, 128));
+#pragma unroll
+            for (int k8 = 0; k8 < 32; k8 += 8) {
+                const uint4 q = *(const uint4 *)(sh.adw + cm_off(r, 2 * c0 + k8, 128));   // 2 c0: the quarter's samples
                 const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
                 for (int h = 0; h < 4; h++)
@@ -574,29 +552,46 @@ __global__ void __launch_bounds__(kTile, 1)
             acc_b23 += sum;
         }
         tiles_done++;
-        __syncthreads();
+        if (!mma_wait(mbar_dw, phase_dw)) { timeout = true; break; }   // act, adw, bdw, zs free again
     }
     if (timeout) {
-        if (r == 0) set_status(status, SPH_STATUS_MMA_TIMEOUT);
-        for (int i = r; i < kMlpParams + 1; i += kTile) out[i] = 0.f;
+        if (tid == 0) set_status(status, SPH_STATUS_MMA_TIMEOUT);
+        for (int i = tid; i < kMlpParams + 1; i += kTrainThreads) out[i] = 0.f;
     } else {
         // weight gradients from TMEM: rows < 64 hold dW3 (columns 64..127), rows >= 64 dW2 (columns 128..191)
-        tc_fence_after();
         const bool upper = r < kMlpH;
-        tmem_row64(tmem, upper ? 64u : 128u, v);
-        float *dst = out + (upper ? kMlpOffW3 + r * kMlpH : kMlpOffW2 + (r - kMlpH) * kMlpH);
+        tmem_ld16(trow + (upper ? 64u : 128u), v);
+        float *dst = out + (upper ? kMlpOffW3 + r * kMlpH : kMlpOffW2 + (r - kMlpH) * kMlpH) + c0;
 #pragma unroll
-        for (int jj = 0; jj < kMlpH; jj++) dst[jj] = v[jj];
-        if (upper) {
-#pragma unroll
-            for (int c = 0; c < kMlpIn; c++) out[kMlpOffW1 + r * kMlpIn + c] = acc_w1[c];
-            out[kMlpOffB1 + r] = acc_b1;
-            out[kMlpOffB3 + r] = acc_b23;
-            out[kMlpOffW4 + r] = sh.dw4[0][r] + sh.dw4[1][r] + sh.dw4[2][r] + sh.dw4[3][r];
-        } else {
-            out[kMlpOffB2 + (r - kMlpH)] = acc_b23;
+        for (int q = 0; q < 16; q += 2) *(float2 *)(dst + q) = make_float2(v[q], v[q + 1]);
+        float(&red)[7][kTrainThreads] = *(float(*)[7][kTrainThreads]) & sh.zs[0][0];
+        red[0][tid] = acc_w1[0];
+        red[1][tid] = acc_w1[1];
+        red[2][tid] = acc_w1[2];
+        red[3][tid] = acc_w1[3];
+        red[4][tid] = acc_b1;
+        red[5][tid] = acc_w4;
+        red[6][tid] = acc_b23;
+        if (c0 == 0) {
+            for (int o = 16; o > 0; o >>= 1) {
+                acc_b4 += __shfl_xor_sync(0xffffffffu, acc_b4, o);
+                acc_loss += __shfl_xor_sync(0xffffffffu, acc_loss, o);
+            }
+            if (lane == 0) { sh.db4[warp] = acc_b4; sh.loss[warp] = acc_loss; }
         }
-        if (r == 0) {
+        __syncthreads();
+        if (tid < 6 * kMlpH) {   // sum m of neuron nj over the 8 groups of samples
+            const int mm = tid >> 6;
+            float s = 0.f;
+#pragma unroll
+            for (int h = 0; h < 8; h++) s += red[mm][h * kMlpH + nj];
+            out[mm < 4 ? kMlpOffW1 + nj * kMlpIn + mm : (mm == 4 ? kMlpOffB1 : kMlpOffW4) + nj] = s;
+        } else {                 // rows nj and 64 + nj of adw over the four quarters
+            const int row = tid - 6 * kMlpH;
+            const float s = (red[6][row] + red[6][kTile + row]) + (red[6][2 * kTile + row] + red[6][3 * kTile + row]);
+            out[(row < kMlpH ? kMlpOffB3 : kMlpOffB2 - kMlpH) + row] = s;
+        }
+        if (tid == 0) {
             out[kMlpOffB4] = sh.db4[0] + sh.db4[1] + sh.db4[2] + sh.db4[3];
             out[kMlpParams] = sh.loss[0] + sh.loss[1] + sh.loss[2] + sh.loss[3];
         }
@@ -619,16 +614,28 @@ __device__ __forceinline__ void store_wb(uint16_t *__restrict__ wb, int p, float
     if (q >= 0) wb[q] = __bfloat16_as_ushort(__float2bfloat16_rn(w));
 }
 
-// Sum of the per-CTA partials in CTA order (deterministic); with `adam`, one
-// Adam step on the FP32 parameters and refreshed BF16 weight copies.
-__global__ void k_mlp_reduce_adam(const float *__restrict__ part, int nparts, float *__restrict__ grad_out,
-                                  float *__restrict__ loss_out, float *__restrict__ params, float *__restrict__ m1,
-                                  float *__restrict__ m2, uint16_t *__restrict__ wb, float lr, float beta1, float beta2,
-                                  float eps, float c1, float c2, int adam) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p > kMlpParams) return;
+// Sum of the per-CTA partials in a fixed order (deterministic); with `adam`, one
+// Adam step on the FP32 parameters and refreshed BF16 weight copies.  A block has 32
+// parameters and eight groups of CTAs: one thread for each parameter walked up to 304
+// partials in turn on 35 SMs, 15 us of exposed latency; now 6 us.
+__global__ void __launch_bounds__(256)
+    k_mlp_reduce_adam(const float *__restrict__ part, int nparts, float *__restrict__ grad_out,
+                      float *__restrict__ loss_out, float *__restrict__ params, float *__restrict__ m1,
+                      float *__restrict__ m2, uint16_t *__restrict__ wb, float lr, float beta1, float beta2, float eps,
+                      float c1, float c2, int adam) {
+    __shared__ float s_g[8][32];
+    const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
+    const int p = blockIdx.x * 32 + lane;
     float g = 0.f;
-    for (int c = 0; c < nparts; c++) g += part[(size_t)c * (kMlpParams + 1) + p];
+    if (p <= kMlpParams) {
+#pragma unroll 8
+        for (int c = group; c < nparts; c += 8) g += part[(size_t)c * (kMlpParams + 1) + p];
+    }
+    s_g[group][lane] = g;
+    __syncthreads();
+    if (group != 0 || p > kMlpParams) return;
+#pragma unroll
+    for (int h = 1; h < 8; h++) g += s_g[h][lane];
     if (grad_out) grad_out[p] = g;
     if (p == kMlpParams) {
         if (loss_out) *loss_out = g;
@@ -680,13 +687,13 @@ void launch_jc_warm(cudaStream_t s, int grid, const KConsts &K, const SortedFiel
 
 void launch_mlp_grad(cudaStream_t s, int grid, const MlpDev &m, const float *x, const float *t, const int32_t *idx,
                      int64_t nb, float *part, uint32_t *status) {
-    k_mlp_grad<<<grid, kTile, sizeof(TrainSmem), s>>>(m, x, t, idx, nb, 1.f / (float)nb, part, status);
+    k_mlp_grad<<<grid, kTrainThreads, sizeof(TrainSmem), s>>>(m, x, t, idx, nb, 1.f / (float)nb, part, status);
 }
 
 void launch_mlp_reduce_adam(cudaStream_t s, const float *part, int nparts, float *grad_out, float *loss_out,
                             float *params, float *m1, float *m2, uint16_t *wb, float lr, float beta1, float beta2,
                             float eps, float c1, float c2, bool adam) {
-    k_mlp_reduce_adam<<<div_up(kMlpParams + 1, 256), 256, 0, s>>>(part, nparts, grad_out, loss_out, params, m1, m2,
+    k_mlp_reduce_adam<<<div_up(kMlpParams + 1, 32), 256, 0, s>>>(part, nparts, grad_out, loss_out, params, m1, m2,
                                                                   wb, lr, beta1, beta2, eps, c1, c2, adam ? 1 : 0);
 }
 

@@ -81,7 +81,7 @@ int ensure_part(sph_mlp *m, int rows) {
 
 int grad_grid(const sph_mlp *m, int64_t nb) {
     int64_t tiles = (nb + 127) / 128;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, 2 * (int64_t)m->num_sms));
+    return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, m->num_sms));
 }
 
 // Gradient (and loss) of the mean loss over samples idx[0..nb) (or 0..nb) into
