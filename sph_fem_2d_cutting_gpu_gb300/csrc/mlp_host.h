@@ -2,6 +2,7 @@
 // points and the context's warm-start attachment.
 #pragma once
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -15,10 +16,17 @@ struct sph_mlp {
     uint16_t *wb = nullptr;                                  // BF16 weight copies
     float *part = nullptr;                                   // per-CTA gradient partials
     int part_rows = 0;
-    float *grad = nullptr;                                   // [kMlpParams + 1]
+    float *grad = nullptr;                                   // [kMlpParams + 1], then the status word
     float *loss = nullptr;                                   // per-step losses of a training run
     int64_t loss_cap = 0;
     uint32_t *status = nullptr;
+    // Scratch kept for the next call: a batch's features and targets on the device (up to
+    // kKeepSamples), and a page-locked copy of gradient, loss and status.  One call at a
+    // time uses it and the stream (busy).
+    float *batch = nullptr;
+    int64_t batch_cap = 0;
+    float *result = nullptr;
+    std::mutex busy;
     sph_mlp_norm norm{};
     int64_t adam_t = 0;
     std::vector<void *> allocs;

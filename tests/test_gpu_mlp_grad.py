@@ -30,3 +30,24 @@ def test_gradient_tiles(lib, n):
     for name, (a, b) in BLOCKS.items():
         assert rel(g[a:b], ref[a:b]) < 2e-2, name
     assert abs(loss - l_ref) <= 1e-3 * l_ref
+
+
+def test_kept_scratch(lib):
+    """One object called from several threads with batches that grow, shrink and exceed what it
+    keeps (2^20 samples): each call's result is that of the call made alone."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    p, norm = random_net(23)
+    sizes = [40_000, 3, 5_000, 100_000, 129, (1 << 20) + 1]
+    batches = [data(n, 30 + n) for n in sizes]
+    alone = []
+    for x, t in batches:
+        m = net_with(p, norm)
+        alone.append((m.gradients(x, t), m.predict(x)))
+        m.close()
+    m = net_with(p, norm)
+    with ThreadPoolExecutor(4) as pool:
+        got = list(pool.map(lambda b: (m.gradients(*b), m.predict(b[0])), batches * 2))
+    m.close()
+    for (a, ya), (b, yb) in zip(alone * 2, got):
+        assert np.array_equal(a[0], b[0]) and a[1] == b[1] and np.array_equal(ya, yb)
