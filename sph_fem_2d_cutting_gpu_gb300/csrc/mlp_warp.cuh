@@ -21,7 +21,16 @@
 
 namespace sphfem {
 
-__device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + expf(-z)); }
+// 1 / x for x >= 1 (or NaN) without the branch of a division, which keeps the evaluations
+// of a thread's neurons from overlapping: one Newton step with an exact residual from the
+// hardware's approximation, correctly rounded (Markstein 1990: all but, possibly, a
+// mantissa of ones); the approximation itself where the result is subnormal or zero.
+__device__ __forceinline__ float recip_ge1(float x) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return x < 0x1p126f ? fmaf(r, fmaf(-x, r, 1.f), r) : r;
+}
+__device__ __forceinline__ float sigmoidf_(float z) { return recip_ge1(1.f + expf(-z)); }
 __device__ __forceinline__ float siluf_(float z) { return z * sigmoidf_(z); }
 __device__ __forceinline__ float bf16_bits_to_f(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
