@@ -3,6 +3,7 @@
 // the fused contact / boundary-condition / invalidate kernel of the step.
 #include <algorithm>
 
+#include "fem.cuh"
 #include "tail.cuh"
 
 namespace sphfem {
@@ -173,10 +174,11 @@ __global__ void __launch_bounds__(kBlock) k_invalidate(int N, SortedFields A, ui
 }
 
 // ---- rigid (SPH-mode) tool: tool_gpu.cu, actions_gpu.cu:316-343 ----------------------------------
-// tool::update_tool (tool.cpp:202-212) on the device copy of the tool.
-__global__ void k_rigid_move(sph_rigid_tool *t, double dt) {
+// tool::update_tool (tool.cpp:202-212) on the device copy of the tool: a thread for
+// each segment.  The fused step's motion is in k_scatter.
+__global__ void __launch_bounds__(32) k_rigid_move(sph_rigid_tool *t, double dt) {
     begin_after();
-    if (threadIdx.x == 0 && blockIdx.x == 0) rigid_move(*t, dt);
+    for (int i = threadIdx.x; i <= t->n_seg; i += 32) rigid_move_part(*t, i, dt);
 }
 
 // tool_gpu.cu:205-216 update_tool_particles
@@ -218,12 +220,25 @@ __global__ void __launch_bounds__(kBlock) k_fric_heat_rigid(int N, KConsts K, So
 // the warp of each particle at the tool, by the warps at the tool's tip that held
 // most of them.  y-bins, contact and tail: 12,000-particle cut 64 -> 37 us, 640,000
 // particles 73 -> 53 us, 12 cuts of 1.33 M particles 90 -> 77 us.
-template <bool kNextHash, class SF>
-__global__ void __launch_bounds__(kBlock) k_step_tail_fem(int N, KConsts K, SF A, SegDev seg,
+// kNodes (tail_takes_nodes): the first blocks take the tool's nodes, their thermal update
+// from the segments' kept Robin terms and their motion; neither needs the tail or is
+// needed by it.
+template <bool kNodes, bool kNextHash, class SF>
+__global__ void __launch_bounds__(kBlock, 8) k_step_tail_fem(int N, KConsts K, SF A, SegDev seg, FemDev F,
                                                           const ToolDev *__restrict__ tool, SortScratch X,
                                                           uint32_t *status) {
     begin_after();
-    PARTICLE_LOOP_HEAD
+    const int node_blocks = kNodes ? div_up(F.n_nodes, blockDim.x) : 0;
+    if (kNodes && (int)blockIdx.x < node_blocks) {
+        const int i = blockIdx.x * blockDim.x + threadIdx.x;
+        if (i >= F.n_nodes) return;
+        const ToolDev &tc = node_case(K, tool, i);
+        fem_rate_update_one<true>(i, K, F, seg, tool);
+        node_move(F, i, tc.vel, tc.dt, tc.flank_retreat);
+        return;
+    }
+    const int i = (blockIdx.x - node_blocks) * blockDim.x + threadIdx.x;
+    if (i >= N) return;
     if (!flag_is_one(A.blanked[i]) && contact_probe(i, K, A, seg, tool)) {
         X.slots[histogram_slot(X.counts, K.g.num_cell + 1)] = i;
         return;
@@ -411,18 +426,18 @@ void launch_invalidate(cudaStream_t s, int N, const SortedFields &A, uint32_t *s
     k_invalidate<<<GRID>>>(N, A, status);
 }
 template <class SF>
-static void step_tail(cudaStream_t s, int N, const KConsts &K, const SF &A, const SegDev &seg, ToolDev *tool,
-                      const double *T_nodes, const SortScratch &X, uint32_t *status, bool next_hash) {
+static void step_tail(cudaStream_t s, int N, const KConsts &K, const SF &A, const SegDev &seg, const FemDev &F,
+                      ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status, bool next_hash) {
     const int tb = fp64_block(N);   // the rigid contact is FP64 work: spread small systems over all SMs
     if (K.has_tool) {
         const int grid = std::min(2 * 152, div_up(N, 4));   // a queue of any length; two blocks on each SM
-        if (next_hash) {
-            launch_after(s, k_step_tail_fem<true, SF>, div_up(N, tb), tb, 0, N, K, A, seg, tool, X, status);
-            launch_after(s, k_contact_queue<true, SF>, grid, 128, 0, K, A, seg, tool, T_nodes, X, status);
-        } else {
-            launch_after(s, k_step_tail_fem<false, SF>, div_up(N, tb), tb, 0, N, K, A, seg, tool, X, status);
-            launch_after(s, k_contact_queue<false, SF>, grid, 128, 0, K, A, seg, tool, T_nodes, X, status);
-        }
+        const int nodes = div_up(F.n_nodes, tb);
+        launch_after(s,
+                     next_hash ? (nodes ? k_step_tail_fem<true, true, SF> : k_step_tail_fem<false, true, SF>)
+                               : (nodes ? k_step_tail_fem<true, false, SF> : k_step_tail_fem<false, false, SF>),
+                     div_up(N, tb) + nodes, tb, 0, N, K, A, seg, F, tool, X, status);
+        launch_after(s, next_hash ? k_contact_queue<true, SF> : k_contact_queue<false, SF>, grid, 128, 0, K, A, seg,
+                     tool, T_nodes, X, status);
     } else if (K.rigid) {
         launch_after(s, next_hash ? k_step_tail<2, true, SF> : k_step_tail<2, false, SF>, div_up(N, tb), tb, 0, N, K, A, seg,
                      tool, T_nodes, X, status);
@@ -432,14 +447,14 @@ static void step_tail(cudaStream_t s, int N, const KConsts &K, const SF &A, cons
     }
 }
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields &A, const SegDev &seg,
-                      ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
+                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
                       bool next_hash) {
-    step_tail(s, N, K, A, seg, tool, T_nodes, X, status, next_hash);
+    step_tail(s, N, K, A, seg, F, tool, T_nodes, X, status, next_hash);
 }
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields32 &A, const SegDev &seg,
-                      ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
+                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
                       bool next_hash) {
-    step_tail(s, N, K, A, seg, tool, T_nodes, X, status, next_hash);
+    step_tail(s, N, K, A, seg, F, tool, T_nodes, X, status, next_hash);
 }
 void launch_rigid_move(cudaStream_t s, sph_rigid_tool *t, double dt) { launch_after(s, k_rigid_move, 1, 32, 0, t, dt); }
 void launch_rigid_move_particles(cudaStream_t s, int N, const SortedFields &A, const sph_rigid_tool *t, double dt) {

@@ -10,6 +10,7 @@
 // cell_end directly.
 #include "cells.cuh"
 #include "fem.cuh"
+#include "rigid.cuh"
 
 namespace sphfem {
 
@@ -129,14 +130,18 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(int32_t *__restrict_
 
 // ---- scatter into the cell's slot range (arbitrary order inside the cell) -------------
 // With a FEM tool the threads after the particles' run the nodes' half step
-// (calculate_temp(0.5 dt), independent of the sort).
+// (calculate_temp(0.5 dt), independent of the sort).  A rigid tool, whose segments and
+// fillet the tail is the next to read, moves there too (in a launch of its own before the
+// tail, by one thread: 10 us of a step).
 __global__ void __launch_bounds__(kBlock) k_scatter(int N, const int32_t *__restrict__ key,
                                                     const int32_t *__restrict__ arrival,
                                                     const int32_t *__restrict__ offsets, int32_t *__restrict__ slots,
-                                                    KConsts K, FemDev F, const ToolDev *__restrict__ tool) {
+                                                    KConsts K, FemDev F, const ToolDev *__restrict__ tool,
+                                                    sph_rigid_tool *rigid) {
     begin_after();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) scatter_one(i, key, arrival, offsets, slots);
+    else if (rigid) rigid_move_part(*rigid, i - N, K.dt);
     else if (i - N < F.n_nodes) fem_half_one(i - N, K, F, tool);
 }
 
@@ -419,7 +424,7 @@ int scan_blocks(int num_cell) { return div_up(num_cell + 1, kScanTile); }
 // (up to 1,024 tiles = 2.1 M cells the saved launch is worth more: 2.7 us).
 constexpr int kScanTopTiles = 1024;
 int launch_sort_slots(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const FemDev &F,
-                      const ToolDev *tool) {
+                      const ToolDev *tool, sph_rigid_tool *rigid) {
     const sph_geom_constants &g = K.g;
     const int n = g.num_cell + 1;
     const int nb = scan_blocks(g.num_cell);
@@ -432,8 +437,9 @@ int launch_sort_slots(cudaStream_t s, int N, const SortScratch &X, const KConsts
         launch_after(s, k_scan_down<false>, nb, kScanThreads, 0, X.counts, n, X.block_sums, X.offsets, X.cell_start,
                      X.cell_end, g.num_cell);
     }
-    launch_after(s, k_scatter, div_up((int64_t)N + F.n_nodes, kBlock), kBlock, 0, N, X.key, X.arrival, X.offsets, X.slots,
-                 K, F, tool);
+    const int64_t tool_parts = rigid ? SPH_RIGID_MAX_SEG + 1 : F.n_nodes;
+    launch_after(s, k_scatter, div_up(N + tool_parts, kBlock), kBlock, 0, N, X.key, X.arrival, X.offsets, X.slots, K, F,
+                 tool, rigid);
     return nb <= kScanTopTiles ? 3 : 4;
 }
 void launch_rank(cudaStream_t s, int N, const SortScratch &X, int32_t *perm, uint32_t *status) {

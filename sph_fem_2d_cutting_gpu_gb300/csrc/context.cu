@@ -460,7 +460,7 @@ int issue_fused_body(sph_ctx *ctx, int64_t &n, int w, cudaEvent_t *ev = nullptr)
         CK_LAUNCH();
         return SPH_OK;
     }
-    n += launch_sort_slots(s, N, ctx->X, ctx->K, ctx->has_tool ? ctx->fem : FemDev{}, ctx->tool_dev);
+    n += launch_sort_slots(s, N, ctx->X, ctx->K, ctx->has_tool ? ctx->fem : FemDev{}, ctx->tool_dev, ctx->K.rigid);
     if (ev) CK(cudaEventRecord(ev[0], s));
     if (f32)
         launch_gather_fused32(s, N, ctx->X, ctx->K, ctx->v32[ctx->cur] ? nullptr : &A,
@@ -499,24 +499,29 @@ int issue_fused_body(sph_ctx *ctx, int64_t &n, int w, cudaEvent_t *ev = nullptr)
         n += 1;
     }
     if (ev) CK(cudaEventRecord(ev[3], s));
+    FemDev tail_fem{};
     if (ctx->has_tool) {
         const bool shift = ctx->wear_mode == SPH_WEAR_SHIFT;
-        launch_fem_rate_update(s, ctx->K, ctx->fem, ctx->seg, ctx->tool_dev, !shift);
-        n += 2;
+        const bool with_tail = !shift && tail_takes_nodes(N);
+        if (with_tail) {
+            tail_fem = ctx->fem;
+        } else {
+            launch_fem_rate_update(s, ctx->K, ctx->fem, ctx->seg, ctx->tool_dev, !shift);
+            n += 1;
+        }
         if (shift) {   // wear_adjustment (leap_frog.cu:224-229), then the nodes with its flank retreat
             launch_wear_adjustment(s, ctx->K, ctx->fem, ctx->seg, ctx->wear, ctx->tool_dev, ctx->K.dt);
             launch_tool_move(s, ctx->K, ctx->seg, ctx->fem, ctx->tool_dev, ctx->K.dt, 4, true);
             n += 7;
         }
-        launch_tool_cases(s, ctx->K.n_cases, ctx->seg, ctx->tool_dev);
-    }
-    if (ctx->K.rigid) {
-        launch_rigid_move(s, ctx->K.rigid, ctx->K.dt);
+        launch_tool_cases(s, ctx->K, ctx->seg, ctx->tool_dev, with_tail);
         n += 1;
     }
     if (ev) CK(cudaEventRecord(ev[4], s));
-    if (f32) launch_step_tail(s, N, ctx->K, B32, ctx->seg, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status, true);
-    else launch_step_tail(s, N, ctx->K, B, ctx->seg, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status, true);
+    if (f32)
+        launch_step_tail(s, N, ctx->K, B32, ctx->seg, tail_fem, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status, true);
+    else
+        launch_step_tail(s, N, ctx->K, B, ctx->seg, tail_fem, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status, true);
     n += ctx->has_tool ? 2 : 1;   // with the FEM tool: the tail and the contact queue
     if (ev) CK(cudaEventRecord(ev[5], s));
     CK_LAUNCH();
@@ -776,7 +781,7 @@ int ctx_upload_tool(sph_ctx *ctx, bool with_model, const std::vector<ToolDev> &t
         SegDev &S = ctx->seg;
         S.n = M.n_seg;
         DALLOC(S.left, M.n_seg); DALLOC(S.right, M.n_seg); DALLOC(S.normal, M.n_seg); DALLOC(S.marks, M.n_seg);
-        DALLOC(S.heat_exchange, M.n_seg); DALLOC(S.fric_heat, M.n_seg);
+        DALLOC(S.heat_exchange, M.n_seg); DALLOC(S.fric_heat, M.n_seg); DALLOC(S.robin, M.n_seg);
         DALLOC(S.bin_count, (size_t)kSegBins * tds.size());
         DALLOC(S.bin_list, (size_t)kSegBins * kSegBinCap * tds.size());
         DALLOC(S.geo, M.n_seg);
@@ -1168,7 +1173,7 @@ int sph_sort(sph_ctx *ctx) {
     REQUIRE_STATE(true);
     const int N = ctx->N;
     launch_count(ctx->stream, N, CUR(ctx), ctx->X, ctx->K.g, ctx->W.status, false);
-    const int sort_launches = launch_sort_slots(ctx->stream, N, ctx->X, ctx->K, FemDev{}, ctx->tool_dev);
+    const int sort_launches = launch_sort_slots(ctx->stream, N, ctx->X, ctx->K, FemDev{}, ctx->tool_dev, nullptr);
     launch_rank(ctx->stream, N, ctx->X, ctx->F.idx, ctx->W.status);
     const int w = pick_out(ctx);
     launch_gather_plain(ctx->stream, N, ctx->F.idx, CUR(ctx), ctx->buf[w]);

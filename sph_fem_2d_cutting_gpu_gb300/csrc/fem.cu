@@ -15,7 +15,7 @@
 namespace sphfem {
 
 // kMove: the nodes move with the tool in the same pass (the Robin terms read the
-// segments' end points, not the nodes).
+// segments' end points, not the nodes).  Small systems: in the tail's launch.
 template <bool kMove>
 __global__ void __launch_bounds__(kBlock) k_fem_rate_update(KConsts K, FemDev F, SegDev seg,
                                                             const ToolDev *__restrict__ tool) {
@@ -29,14 +29,19 @@ __global__ void __launch_bounds__(kBlock) k_fem_rate_update(KConsts K, FemDev F,
     }
 }
 
-// One block per case: its segments and tool state move, then its y-bins.
-__global__ void __launch_bounds__(kBlock) k_tool_cases(SegDev seg, ToolDev *tool) {
+// One block per case: its segments and tool state move, then its y-bins.  kRobin: the
+// segments' Robin terms, which the motion ends, are kept for the nodes' update.
+template <bool kRobin>
+__global__ void __launch_bounds__(kBlock) k_tool_cases(KConsts K, SegDev seg, ToolDev *tool) {
     begin_after();
     ToolDev &tc = tool[blockIdx.x];
-    for (int q = threadIdx.x; q < tc.seg_count; q += blockDim.x)
-        segment_move(seg, tc.seg_first + q, tc.vel, tc.dt, tc.flank_retreat);
-    __syncthreads();
-    if (threadIdx.x == 0) tool_case_move(tc, tc.dt);
+    // no field that the segments read changes with the case's state
+    if (threadIdx.x == blockDim.x - 1) tool_case_move(tc, tc.dt);
+    for (int q = threadIdx.x; q < tc.seg_count; q += blockDim.x) {
+        const int s = tc.seg_first + q;
+        if (kRobin) seg.robin[s] = robin_segment(K, seg, s);
+        segment_move(seg, s, tc.vel, tc.dt, tc.flank_retreat);
+    }
     __syncthreads();
     seg_bins_block(blockIdx.x, seg, tool);
 }
@@ -89,8 +94,8 @@ void launch_fem_rate_update(cudaStream_t s, const KConsts &K, const FemDev &F, c
     const int grid = div_up(F.n_nodes, kBlock);
     launch_after(s, move_nodes ? k_fem_rate_update<true> : k_fem_rate_update<false>, grid, kBlock, 0, K, F, seg, tool);
 }
-void launch_tool_cases(cudaStream_t s, int n_cases, const SegDev &seg, ToolDev *tool) {
-    launch_after(s, k_tool_cases, n_cases, kBlock, 0, seg, tool);
+void launch_tool_cases(cudaStream_t s, const KConsts &K, const SegDev &seg, ToolDev *tool, bool robin) {
+    launch_after(s, robin ? k_tool_cases<true> : k_tool_cases<false>, K.n_cases, kBlock, 0, K, seg, tool);
 }
 void launch_fem_reset(cudaStream_t s, const FemDev &F, double *T_old, double *f_temp, double *K_temp) {
     k_fem_reset<<<div_up(F.nnz > F.n_nodes ? F.nnz : F.n_nodes, kBlock), kBlock, 0, s>>>(F, T_old, f_temp, K_temp);

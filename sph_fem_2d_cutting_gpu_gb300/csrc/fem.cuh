@@ -7,22 +7,29 @@
 
 namespace sphfem {
 
-// Robin terms of node i (FEM_thermal_gpu.cu:342-386): rhs and diagonal additions.
+// Robin terms of segment s for each of its two nodes (FEM_thermal_gpu.cu:342-386): rhs and
+// diagonal additions.
+__device__ __forceinline__ double2 robin_segment(const KConsts &K, const SegDev &seg, int s) {
+    const double2 hx = seg.heat_exchange[s];
+    if (hx.y == 0) return make_double2(0., 0.);
+    const double T_cont_particle = hx.x / hx.y;
+    const double2 l = seg.left[s], r = seg.right[s];
+    const double ddx = l.x - r.x, ddy = l.y - r.y;
+    const double dist = sqrtf_d(ddx * ddx + ddy * ddy);
+    return make_double2(__fma_rn(0.5 * K.c.tool.h * dist, T_cont_particle, 0.5 * seg.fric_heat[s]),
+                        __dmul_rn(K.c.tool.h, 0.5 * dist));
+}
+// ... and their sums over the segments of node i.  kStored: seg.robin holds them.
+template <bool kStored = false>
 __device__ __forceinline__ void robin_terms(const KConsts &K, const FemDev &F, const SegDev &seg, int i, double &df,
                                             double &dk) {
     df = 0.;
     dk = 0.;
     for (int t = F.node_seg_ptr[i]; t < F.node_seg_ptr[i + 1]; t++) {
-        int s = F.node_seg[t];
-        double2 hx = seg.heat_exchange[s];
-        if (hx.y == 0) continue;
-        double T_cont_particle = hx.x / hx.y;
-        double fric_eng = seg.fric_heat[s];
-        double2 l = seg.left[s], r = seg.right[s];
-        double ddx = l.x - r.x, ddy = l.y - r.y;
-        double dist = sqrtf_d(ddx * ddx + ddy * ddy);
-        df += 0.5 * K.c.tool.h * dist * T_cont_particle + 0.5 * fric_eng;
-        dk += K.c.tool.h * (0.5 * dist);
+        const int s = F.node_seg[t];
+        const double2 r = kStored ? seg.robin[s] : robin_segment(K, seg, s);
+        df = __dadd_rn(df, r.x);
+        dk = __dadd_rn(dk, r.y);
     }
 }
 
@@ -40,11 +47,12 @@ __device__ __forceinline__ void fem_half_one(int i, const KConsts &K, const FemD
 
 // apply_robin_bdc + calculate_temp_rate + calculate_temp(dt), one row per
 // thread (FEM_thermal_gpu.cu:342-386,443-468).  Reads T_half, writes k and T.
+template <bool kStored = false>
 __device__ __forceinline__ void fem_rate_update_one(int i, const KConsts &K, const FemDev &F, const SegDev &seg,
                                                     const ToolDev *__restrict__ tool) {
     const double dt = node_case(K, tool, i).dt;
     double df, dk;
-    robin_terms(K, F, seg, i, df, dk);
+    robin_terms<kStored>(K, F, seg, i, df, dk);
     double buffer = 0.;
     for (int t = F.row_ptr[i]; t < F.row_ptr[i + 1]; t++) {
         int c = F.col_ind[t];

@@ -36,7 +36,7 @@ int scan_blocks(int num_cell);
 // the scan of the histogram (which it leaves zeroed) and the scatter into the cells'
 // slots, with the half step of F's nodes (none: n_nodes 0); returns the launches
 int launch_sort_slots(cudaStream_t s, int N, const SortScratch &X, const KConsts &K, const FemDev &F,
-                      const ToolDev *tool);
+                      const ToolDev *tool, sph_rigid_tool *rigid);
 // perm from the slots (the staged sort; the fused gathers rank as they go)
 void launch_rank(cudaStream_t s, int N, const SortScratch &X, int32_t *perm, uint32_t *status);
 void launch_gather_plain(cudaStream_t s, int N, const int32_t *perm, const SortedFields &A, const SortedFields &B);
@@ -95,12 +95,18 @@ void launch_contact(cudaStream_t s, int N, const KConsts &K, const SortedFields 
 void launch_bc(cudaStream_t s, int N, const SortedFields &A);
 void launch_bc_thermal(cudaStream_t s, int N, const KConsts &K, const SortedFields &A);
 void launch_invalidate(cudaStream_t s, int N, const SortedFields &A, uint32_t *status);
-// with the FEM tool (its y-bins built): the contact queue after it (one more launch)
+// Whether the tool's nodes are updated in the tail's launch: on a tail of at most one wave
+// (8 blocks an SM), where a launch less counts -- 12,000 particles 5 us of a step of 76.
+// On a longer one the nodes' part, which needs more registers, costs more than a launch:
+// 1.33 M particles 625 us a step against 621, 640,000 particles 329 against 327.
+constexpr bool tail_takes_nodes(int N) { return N <= 8 * 152 * 256; }
+// with the FEM tool (its y-bins built): the contact queue after it (one more launch).  F:
+// the nodes whose thermal update (from seg.robin) and motion go with it; none: n_nodes 0.
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields &A, const SegDev &seg,
-                      ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
+                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
                       bool next_hash);
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields32 &A, const SegDev &seg,
-                      ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
+                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
                       bool next_hash);
 void launch_rigid_move(cudaStream_t s, sph_rigid_tool *t, double dt);
 void launch_rigid_move_particles(cudaStream_t s, int N, const SortedFields &A, const sph_rigid_tool *t, double dt);
@@ -117,8 +123,9 @@ void launch_reduce_cases(cudaStream_t s, int n_cases, const SortedFields &A, con
 // move_nodes: the nodes move with the tool in the same pass (tool_update_FEM_gpu)
 void launch_fem_rate_update(cudaStream_t s, const KConsts &K, const FemDev &F, const SegDev &seg,
                             const ToolDev *tool, bool move_nodes);
-// every case's segments and tool state moved, then the segment y-bins (one block a case)
-void launch_tool_cases(cudaStream_t s, int n_cases, const SegDev &seg, ToolDev *tool);
+// every case's segments and tool state moved, then the segment y-bins (one block a case);
+// robin: the segments' Robin terms go to seg.robin first
+void launch_tool_cases(cudaStream_t s, const KConsts &K, const SegDev &seg, ToolDev *tool, bool robin);
 void launch_fem_reset(cudaStream_t s, const FemDev &F, double *T_old, double *f_temp, double *K_temp);
 void launch_fem_robin(cudaStream_t s, const KConsts &K, const FemDev &F, const SegDev &seg, double *f_temp,
                       double *K_temp);

@@ -29,17 +29,19 @@ __device__ __forceinline__ void rigid_line(double p1x, double p1y, double p2x, d
 }
 
 // tool.cpp update_tool: every segment end and the fillet centre move by dt * vel,
-// the segment lines are rebuilt, the normals stay.
-__device__ __forceinline__ void rigid_move(sph_rigid_tool &t, double dt) {
+// the segment lines are rebuilt, the normals stay.  Part i of n_seg + 1: a segment, or
+// the fillet.
+__device__ __forceinline__ void rigid_move_part(sph_rigid_tool &t, int i, double dt) {
     const double dx = __dmul_rn(dt, t.vel[0]), dy = __dmul_rn(dt, t.vel[1]);
-    for (int i = 0; i < t.n_seg; i++) {
-        t.left[i][0] = __dadd_rn(t.left[i][0], dx);
-        t.left[i][1] = __dadd_rn(t.left[i][1], dy);
-        t.right[i][0] = __dadd_rn(t.right[i][0], dx);
-        t.right[i][1] = __dadd_rn(t.right[i][1], dy);
-        rigid_line(t.left[i][0], t.left[i][1], t.right[i][0], t.right[i][1], t.la[i], t.lb[i], t.vertical[i]);
-    }
-    if (t.has_fillet) {
+    if (i < t.n_seg) {
+        const double lx = __dadd_rn(t.left[i][0], dx), ly = __dadd_rn(t.left[i][1], dy);
+        const double rx = __dadd_rn(t.right[i][0], dx), ry = __dadd_rn(t.right[i][1], dy);
+        t.left[i][0] = lx;
+        t.left[i][1] = ly;
+        t.right[i][0] = rx;
+        t.right[i][1] = ry;
+        rigid_line(lx, ly, rx, ry, t.la[i], t.lb[i], t.vertical[i]);
+    } else if (i == t.n_seg && t.has_fillet) {
         t.fillet_p[0] = __dadd_rn(t.fillet_p[0], dx);
         t.fillet_p[1] = __dadd_rn(t.fillet_p[1], dy);
     }

@@ -133,6 +133,7 @@ struct SegDev {
     int4 *marks;              // element, colour, node left, node right
     double2 *heat_exchange;   // (sum T*length, sum length)
     double *fric_heat;
+    double2 *robin;           // fused step: each segment's Robin terms (rhs, diagonal) for its two nodes
     WearAcc wear;             // wear statistics (pp == NULL: off)
     double *wear_rate;        // wear_nodes: per-segment wear rate of the last nodal shift
     // y-bins of each case's segments for the contact's ray casting (k_seg_bins):

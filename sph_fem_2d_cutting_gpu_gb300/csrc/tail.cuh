@@ -61,11 +61,7 @@ __device__ __forceinline__ void seg_bins_block(int c, const SegDev &seg, ToolDev
             if (slot < kSegBinCap) list[b * kSegBinCap + slot] = i;
             if (seg.bin_xkey) atomicMax(&xkey[b], kx);
         }
-    }
-    // the per-segment constants of the contact search (SegGeo)
-    if (seg.geo) {
-        for (int i = threadIdx.x; i < t.seg_count; i += blockDim.x) {
-            const double2 L = seg.left[t.seg_first + i], R = seg.right[t.seg_first + i];
+        if (seg.geo) {   // the segment's constants of the contact search (SegGeo)
             SegGeo g;
             g.ymin_f = fminf_d(L.y, R.y);
             g.ymax_f = fmaxf_d(L.y, R.y);
