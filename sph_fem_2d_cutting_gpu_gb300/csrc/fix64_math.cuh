@@ -180,6 +180,21 @@ __device__ __forceinline__ double fix_log_above_1(double x) {
     return fix_double(l * Fix64{0xb17217f7d1cf79acull, -64});
 }
 
+// pow(x, n), or for lanes with `lg` log(x) of x > 1: fix_pow and fix_log_above_1 with their
+// common part formed once, for lanes that need either to stay together.
+__device__ __forceinline__ double fix_pow_or_log(double x, double n, bool lg) {
+    const uint32_t xh = (uint32_t)__double2hiint(x), nh = (uint32_t)__double2hiint(n);
+    bool neg;
+    const Fix64 l = fix_log2(x, neg);
+    if (lg) return xh >= 0x7ff00000u ? log_general(x) : fix_double(l * Fix64{0xb17217f7d1cf79acull, -64});
+    const Fix64 y = fix_norm(l * fix_abs(n));
+    if (nh - 0x3f600000u >= 0x00a00000u || xh - 0x00100000u >= 0x7fe00000u || y.e + 63 >= 9) {
+        if (nh - 0x3f600000u < 0x00a00000u && (xh | (uint32_t)__double2loint(x)) == 0u) return 0.;
+        return pow_general(x, n);
+    }
+    return fix_double(fix_exp2(y, neg));
+}
+
 // ---- atan2, sin and cos of floats ------------------------------------------------------------
 // The reference's atan2f, sinf and cosf, formed to 2^-57 and rounded once to float (the
 // CPU restatement rounds its double functions once, too).  atan by one step to the

@@ -112,7 +112,8 @@ static __device__ __noinline__ void sums64_plain(Sums64 &out, int k, int sub, co
 
 // ---- per-particle epilogue (fused mode) -----------------------------------------------------------
 // vd (= v_der), acc (stress divergence and viscosity, an acceleration), xt (= pos_t from XSPH), T_t.
-__device__ __forceinline__ void fused_epilogue(int k, const KConsts &K, const SortedFields &B, const FixedFields &F,
+// Returns whether the particle may yield: return_map then finishes it.
+__device__ __forceinline__ bool fused_epilogue(int k, const KConsts &K, const SortedFields &B, const FixedFields &F,
                                                const SegDev &seg, const ToolDev *__restrict__ tool,
                                                int32_t *__restrict__ secant_iters, uint32_t *status, bool is_tool,
                                                double2 vel_pred, double rho_pred, dbl4 vd, double2 acc, double2 xt,
@@ -168,15 +169,42 @@ __device__ __forceinline__ void fused_epilogue(int k, const KConsts &K, const So
                                         seg.n, T, blanked, seg.fric_heat, seg.wear);
     else if (K.rigid && !is_tool && K.c.trml_wp.eta != 0.)   // actions_gpu.cu:316-343
         rigid_fric_heat_one(K, dt, K.rigid->vel, vel, B.ft[k], B.n[k], T);
-    // return mapping (actions_gpu.cu:689-754)
-    if (K.c.plastic && !is_tool && blanked != 1.) {
-        double eps_pl = B.eps_pl[k], eps_pl_dot = B.eps_pl_dot[k];
-        int it = 0;
-        st |= plasticity_one<false>(K, dt, S, F.p[k], rho, eps_pl, eps_pl_dot, T, blanked, &it);
-        B.eps_pl[k] = eps_pl;
-        B.eps_pl_dot[k] = eps_pl_dot;
-        if (secant_iters) secant_iters[k] = it;
+    bool yields = false;
+    if (K.c.plastic && !is_tool && blanked != 1.) {   // return mapping (actions_gpu.cu:689-754)
+        yields = !surely_elastic(K, S, F.p[k], B.eps_pl[k], B.eps_pl_dot[k], T);
+        if (!yields) {
+            B.eps_pl_dot[k] = 0.;
+            if (secant_iters) secant_iters[k] = 0;
+        }
     }
+    B.S[k] = S;
+    B.T[k] = T;
+    if (blanked == 1.) B.blanked[k] = 1.;
+    if (st) set_status(status, st);
+    return yields;
+}
+
+// The return mapping of a particle that may yield, from its stored state, by one lane or
+// four (return_mapping).  Not inlined: with its code in the kernel's own the sums of
+// 1,048,576 particles take 2,917 us, so 2,883.
+template <bool kQuad>
+static __device__ __noinline__ void return_map(int k, const KConsts &K, const SortedFields &B, const double *p,
+                                               const ToolDev *tool, int32_t *secant_iters, uint32_t *status) {
+    dbl4 S = B.S[k];
+    double T = B.T[k], blanked = 0.;
+    Mapping64 y;
+    y.eps_pl = B.eps_pl[k];
+    y.eps_pl_dot = B.eps_pl_dot[k];
+    y.T = T;
+    y.dt = tool[case_of_hash(K, B.hash[k])].dt;
+    trial_norms(S, p[k], y.norm, y.svm);
+    const Mapped64 m = return_mapping<kQuad>(K, y);
+    if (kQuad && (threadIdx.x & 3u)) return;
+    B.eps_pl_dot[k] = m.eps_pl_dot;
+    if (secant_iters) secant_iters[k] = abs(m.iters);
+    if (m.iters == 0) return;   // elastic after all
+    B.eps_pl[k] = m.eps_pl;
+    const uint32_t st = apply_mapping(K, y, m, B.rho[k], S, T, blanked);
     B.S[k] = S;
     B.T[k] = T;
     if (blanked == 1.) B.blanked[k] = 1.;
@@ -187,7 +215,16 @@ __device__ __forceinline__ void fused_epilogue(int k, const KConsts &K, const So
 // alternate between the integer and the FP64 pipe, and 4 blocks at 128 registers
 // were 5 % slower on the 1,048,576-particle lattice, 3 blocks 13 %.
 // ---- the kernel --------------------------------------------------------------------------------------
-template <bool kFused>
+// kMapNone: the staged sums.  kMapLane, kMapQuads: the fused step, its return mappings in
+// the epilogue's lanes or in groups of four lanes of the whole block.  The groups cut a
+// small system's step, whose last block waits for one chain (12,000 particles, 74 of them
+// yielding, sums stage 81 -> 72 us), but keep the block's other warps, and their registers,
+// until the epilogue's end: on systems of many waves, where the next block's warps would
+// start in their place, 2 % slower (1,048,576 particles 2,891 -> 2,949 us).  So: groups on
+// grids of up to one wave (map_by_quads).
+enum Map64 { kMapNone, kMapLane, kMapQuads };
+inline bool map_by_quads(int N) { return div_up(N, kParts64) <= 5 * 152; }
+template <Map64 kMap>
 __global__ void __launch_bounds__(kThreads64, 5) k_interact64(int N, KConsts K, const int32_t *__restrict__ offsets,
                                                               const dbl4 *__restrict__ rec,
                                                               const float2 *__restrict__ cand, SortedFields B,
@@ -195,6 +232,7 @@ __global__ void __launch_bounds__(kThreads64, 5) k_interact64(int N, KConsts K, 
                                                               const ToolDev *__restrict__ tool,
                                                               int32_t *__restrict__ secant_iters, uint32_t *status) {
     begin_after();
+    constexpr bool kFused = kMap != kMapNone;
     constexpr int kSums = kFused ? 9 : 13;
     __shared__ int s_list[kParts64 * kListPitch64];
     __shared__ double s_sum[kSums][kThreads64];
@@ -395,39 +433,59 @@ __global__ void __launch_bounds__(kThreads64, 5) k_interact64(int N, KConsts K, 
         put_sum(xt0); put_sum(xt1); put_sum(tl);
     }
     __syncthreads();
-    // the epilogue, one thread per particle: full warps for its FP64 work
-    if (threadIdx.x >= kParts64) return;
+    // the epilogue, one thread per particle: a full warp for its FP64 work
+    if (kMap != kMapQuads && threadIdx.x >= kParts64) return;
     const int e = (int)blockIdx.x * kParts64 + (int)threadIdx.x;
-    if (e >= N) return;
-    const dbl4 e0 = rec[4 * e + 0], e2 = rec[4 * e + 2], e3 = rec[4 * e + 3];
-    const int fe = (int)__double_as_longlong(e3.w);
-    if (fe & kFlagBlanked) {
-        if (kFused) rigid_heat_blanked(e, K, B);
-        return;
-    }
-    double v[kSums];
+    auto particle = [&]() -> bool {
+        if (e >= N) return false;
+        const dbl4 e0 = rec[4 * e + 0], e2 = rec[4 * e + 2], e3 = rec[4 * e + 3];
+        const int fe = (int)__double_as_longlong(e3.w);
+        if (fe & kFlagBlanked) {
+            if (kFused) rigid_heat_blanked(e, K, B);
+            return false;
+        }
+        double v[kSums];
 #pragma unroll
-    for (int f = 0; f < kSums; f++) {
-        const double *s = &s_sum[f][threadIdx.x * kLanes64];
-        v[f] = (s[0] + s[1]) + (s[2] + s[3]);
-    }
-    const bool tool_e = (fe & kFlagTool) != 0;
-    const double alpha_e = (!tool_e) ? K.c.trml_wp.alpha : K.c.trml_tool_sph.alpha;
-    const bool thermal_e = flag_nonzero(alpha_e) && !K.thermal_pse;
-    const double mass = K.c.phys.mass, xs = K.c.corr.xspheps * mass;
-    const dbl4 vd = mk4(v[0], v[1], v[2], v[3]);
-    const double2 xt = make_double2(xs * v[kSums - 3], xs * v[kSums - 2]);
-    const double T_t = alpha_e * (2.0 * v[kSums - 1]);
-    if constexpr (kFused) {
-        fused_epilogue(e, K, B, F, seg, tool, secant_iters, status, tool_e, make_double2(e0.z, e0.w), e2.w, vd,
-                       make_double2(mass * v[4], mass * v[5]), xt, thermal_e, T_t);
+        for (int f = 0; f < kSums; f++) {
+            const double *s = &s_sum[f][threadIdx.x * kLanes64];
+            v[f] = (s[0] + s[1]) + (s[2] + s[3]);
+        }
+        const bool tool_e = (fe & kFlagTool) != 0;
+        const double alpha_e = (!tool_e) ? K.c.trml_wp.alpha : K.c.trml_tool_sph.alpha;
+        const bool thermal_e = flag_nonzero(alpha_e) && !K.thermal_pse;
+        const double mass = K.c.phys.mass, xs = K.c.corr.xspheps * mass;
+        const dbl4 vd = mk4(v[0], v[1], v[2], v[3]);
+        const double2 xt = make_double2(xs * v[kSums - 3], xs * v[kSums - 2]);
+        const double T_t = alpha_e * (2.0 * v[kSums - 1]);
+        if constexpr (kFused) {
+            return fused_epilogue(e, K, B, F, seg, tool, secant_iters, status, tool_e, make_double2(e0.z, e0.w), e2.w,
+                                  vd, make_double2(mass * v[4], mass * v[5]), xt, thermal_e, T_t);
+        } else {
+            if (K.thermal_pse && tool_e) return false;
+            F.S_der[e] = mk4(mass * v[4], mass * v[5], mass * v[6], mass * v[7]);
+            F.v_der[e] = vd;
+            B.pos_t[e] = xt;
+            B.vel_t[e] = make_double2(-mass * v[8], -mass * v[9]);
+            if (thermal_e) B.T_t[e] = T_t;
+            return false;
+        }
+    };
+    static_assert(kParts64 == 32, "one warp");
+    if constexpr (kMap == kMapLane) {
+        if (particle()) return_map<false>(e, K, B, F.p, tool, secant_iters, status);
+    } else if constexpr (kMap == kMapQuads) {
+        int &count = s_list[kParts64];
+        if (threadIdx.x < kParts64) {
+            const bool yields = particle();
+            const unsigned all = __ballot_sync(0xffffffffu, yields);
+            if (yields) s_list[__popc(all & ((1u << threadIdx.x) - 1u))] = e;
+            if (threadIdx.x == 0) count = __popc(all);
+        }
+        __syncthreads();
+        const int q = (int)threadIdx.x / 4;
+        if (q < count) return_map<true>(s_list[q], K, B, F.p, tool, secant_iters, status);
     } else {
-        if (K.thermal_pse && tool_e) return;
-        F.S_der[e] = mk4(mass * v[4], mass * v[5], mass * v[6], mass * v[7]);
-        F.v_der[e] = vd;
-        B.pos_t[e] = xt;
-        B.vel_t[e] = make_double2(-mass * v[8], -mass * v[9]);
-        if (thermal_e) B.T_t[e] = T_t;
+        particle();
     }
 }
 

@@ -43,22 +43,7 @@ __device__ __forceinline__ double jc_term_c(const sph_joco_constants &jc, double
     return 1.0 - fix_pow(theta, jc.m);
 }
 
-// eps_dot = eps_pl_dot / eps_dot_ref
-__device__ __forceinline__ double sigma_yield_rate(const sph_joco_constants &jc, double eps_pl, double eps_dot,
-                                                   double term_c) {
-    const double Term_A = jc.A + jc.B * fix_pow(eps_pl, jc.n);
-    double Term_B = 1.;
-    if (eps_dot > 1.0) Term_B = 1.0 + jc.C * fix_log_above_1(eps_dot);
-    else if (flag_nonzero(eps_dot)) Term_B = pow_general(1.0 + eps_dot, jc.C);
-    return Term_A * Term_B * term_c;
-}
-
-__device__ __forceinline__ double sigma_yield_tc(const sph_joco_constants &jc, double eps_pl, double eps_pl_dot,
-                                                 double term_c) {
-    return sigma_yield_rate(jc, eps_pl, fix_div(eps_pl_dot, jc.eps_dot_ref), term_c);
-}
-
-// Same flow stress with the rate/strain terms in FP32 (powf/logf).  Used by the
+// The flow stress with the rate/strain terms in FP32 (powf/logf).  Used by the
 // FP32-compensated mode, where only the secant residual stays in FP64.
 __device__ __forceinline__ double sigma_yield_tc_f32(const sph_joco_constants &jc, double eps_pl, double eps_pl_dot,
                                                      double term_c) {
@@ -73,17 +58,15 @@ __device__ __forceinline__ double sigma_yield_tc_f32(const sph_joco_constants &j
 // ---- plasticity.cuh:117-162 opt_fun + solve_secant ----------------------------
 // Returns delta_lambda; *iters = iterations used, negative when the 100
 // iteration cap was hit (plasticity.cuh:155-158).
-template <bool kF32Yield>
 __device__ __forceinline__ double solve_secant(const sph_joco_constants &jc, double init, double tol,
                                               double norm_Strial, double eps_pl_init, double term_c, double delta_t,
                                               double mu, int *iters, int max_iter = 100) {
     const double s23 = sqrt(2.0 / 3.0);
-    const double rate = s23 / delta_t, rate_rel = rate / jc.eps_dot_ref;
+    const double rate = s23 / delta_t;
     auto opt_fun = [&](double dl) {
         const double dlp = fmax(dl, 0.);
         double eq = eps_pl_init + s23 * dlp;
-        double sY = kF32Yield ? sigma_yield_tc_f32(jc, eq, rate * dlp, term_c)
-                              : sigma_yield_rate(jc, eq, rate_rel * dlp, term_c);
+        double sY = sigma_yield_tc_f32(jc, eq, rate * dlp, term_c);
         return norm_Strial - 2 * mu * dl - s23 * sY;
     };
     double delta_lambda = init;
@@ -129,6 +112,140 @@ __device__ __forceinline__ bool surely_elastic(const KConsts &K, dbl4 S, double 
     return term_a > 0.f && term_b > 0.f && term_c > 0.f && svm * 1.0001f < term_a * term_b * term_c * 0.9999f;
 }
 
+// Norm of the trial stress and its von Mises stress.
+__device__ __forceinline__ void trial_norms(dbl4 S, double p, double &norm, double &svm) {
+    const double Sxx = S.x, Syy = S.z, Szz = S.w, Sxy = S.y;
+    norm = sqrtf_d(Sxx * Sxx + Syy * Syy + Szz * Szz + 2. * Sxy * Sxy);
+    const double cxx = Sxx - p, cyy = Syy - p, czz = Szz - p, cxy = Sxy;
+    svm = sqrtf_d((cxx * cxx + cyy * cyy + czz * czz) - cxx * cyy - cxx * czz - cyy * czz + 3.0 * cxy * cxy);
+}
+
+// The return mapping of the FP64 step.  The flow stress is a product of a strain, a rate
+// and a temperature term, each a logarithm or a power of 100 or so integer operations and
+// a few on the FP64 pipe, 64 cycles each whatever the number of lanes; a particle at its
+// yield point asks for eleven of them in a row (2.6 secant iterations, two points each).
+// kQuad: lanes 4i .. 4i + 3 of a warp, all of which call it with the same arguments, share
+// them -- lanes 0 and 1 form the strain term of the two points of an iteration, lanes 2
+// and 3 the rate term, lane 1 at first the temperature term -- and ask for four in a row.
+// The arithmetic is the same, rounding for rounding.
+struct Mapping64 {
+    double svm, norm, eps_pl, eps_pl_dot, T, dt;
+};
+struct Mapped64 {
+    double delta_lambda, eps_pl, eps_pl_dot, sY;
+    int iters;   // 0: elastic; negative: the iteration cap
+};
+template <bool kQuad>
+__device__ __forceinline__ Mapped64 return_mapping(const KConsts &K, const Mapping64 &y) {
+    const sph_joco_constants &jc = K.c.joco;
+    const int q = kQuad ? (int)threadIdx.x & 3 : 0;
+    const unsigned mask = 0xfu << (threadIdx.x & 28u);
+    auto from = [&](double v, int lane) { return __shfl_sync(mask, v, lane, 4); };
+    auto power = [&](double x, double n, double c0, double c1) { return __fma_rn(c1, fix_pow(x, n), c0); };
+    auto rate_term = [&](double x) {
+        if (!(x > 1.0)) return flag_nonzero(x) ? pow_general(1.0 + x, jc.C) : 1.;
+        return __fma_rn(jc.C, fix_log_above_1(x), 1.);
+    };
+    // c0 + c1 x^n for lanes 0 and 1, the rate term of x for lanes 2 and 3
+    const bool rate = (q & 2) != 0;
+    auto term = [&](double x, double n, double c0, double c1) {
+        if (rate && !(x > 1.0)) return rate_term(x);
+        return __fma_rn(c1, fix_pow_or_log(x, n, rate), c0);
+    };
+    const double c0 = rate ? 1. : jc.A, c1 = rate ? jc.C : jc.B;
+    Mapped64 out = {0., y.eps_pl, 0., 0., 0};
+    double theta = fix_div(y.T - jc.Tref, jc.Tmelt - jc.Tref);
+    if (theta > 1.) theta = 1.;
+    const double rate0 = fix_div(y.eps_pl_dot, jc.eps_dot_ref);
+    double term_c, sY0;
+    if (kQuad) {
+        const bool temp = q == 1;
+        const double t0 =
+            term(rate ? rate0 : (temp ? theta : y.eps_pl), temp ? jc.m : jc.n, temp ? 1. : c0, temp ? -1. : c1);
+        term_c = from(t0, 1);
+        sY0 = __dmul_rn(__dmul_rn(from(t0, 0), from(t0, 2)), term_c);
+    } else {
+        term_c = power(theta, jc.m, 1., -1.);
+        sY0 = __dmul_rn(__dmul_rn(power(y.eps_pl, jc.n, jc.A, jc.B), rate_term(rate0)), term_c);
+    }
+    if (y.svm < sY0) return out;
+    const double s23 = sqrt(2.0 / 3.0), two_mu = 2 * K.c.phys.G;
+    const double rate_rel = fix_div(fix_div(s23, y.dt), jc.eps_dot_ref);
+    auto residual = [&](double at, double sY) { return __fma_rn(-s23, sY, __fma_rn(-two_mu, at, y.norm)); };
+    double dl = fmax(__dmul_rn(__dmul_rn(y.eps_pl_dot, y.dt), s23), 1e-8);
+    int iter = 0;
+    while (true) {   // plasticity.cuh:117-162
+        const double dl_1 = __dmul_rn(dl, 1.01);
+        double g, g_1;
+        if (kQuad) {
+            const double at = (q & 1) ? dl_1 : dl, atp = fmax(at, 0.);
+            const double t = term(rate ? __dmul_rn(rate_rel, atp) : __fma_rn(s23, atp, y.eps_pl), jc.n, c0, c1);
+            const double gx = residual(at, __dmul_rn(__dmul_rn(t, __shfl_xor_sync(mask, t, 2)), term_c));
+            g = from(gx, 0);
+            g_1 = from(gx, 1);
+        } else {
+            auto at_point = [&](double at) {
+                const double atp = fmax(at, 0.);
+                const double sY = __dmul_rn(power(__fma_rn(s23, atp, y.eps_pl), jc.n, jc.A, jc.B),
+                                            rate_term(__dmul_rn(rate_rel, atp)));
+                return residual(at, __dmul_rn(sY, term_c));
+            };
+            g = at_point(dl);
+            g_1 = at_point(dl_1);
+        }
+        const double old = dl;
+        dl = __dsub_rn(dl, fix_div(__dmul_rn(g, __dsub_rn(dl, dl_1)), __dsub_rn(g, g_1)));
+        if (dl < 0.) dl = __dmul_rn(-0.1, dl);
+        if (fabs(__dsub_rn(dl, old)) < 1e-6) {
+            out.iters = iter + 1;
+            break;
+        }
+        if (iter > K.secant_cap) {
+            out.iters = -(iter + 1);
+            break;
+        }
+        iter++;
+    }
+    out.delta_lambda = dl;
+    // sqrtf(2.0/3.0) * fmaxf(delta_lambda, 0.): both calls return float, so the
+    // reference multiplies in float (actions_gpu.cu:728-729)
+    const float inc = sqrtf((float)(2.0 / 3.0)) * fmaxf((float)dl, 0.f);
+    out.eps_pl = y.eps_pl + (double)inc;
+    out.eps_pl_dot = fix_div((double)inc, y.dt);
+    if (K.c.trml_wp.tq != 0.) {
+        const double rate1 = fix_div(out.eps_pl_dot, jc.eps_dot_ref);
+        if (kQuad) {
+            const double t = term(rate ? rate1 : out.eps_pl, jc.n, c0, c1);
+            out.sY = __dmul_rn(__dmul_rn(t, __shfl_xor_sync(mask, t, 2)), term_c);
+        } else {
+            out.sY = __dmul_rn(__dmul_rn(power(out.eps_pl, jc.n, jc.A, jc.B), rate_term(rate1)), term_c);
+        }
+    }
+    return out;
+}
+
+// The particle's state after its mapping (plasticity_one's last part); returns status bits.
+__device__ __forceinline__ uint32_t apply_mapping(const KConsts &K, const Mapping64 &y, const Mapped64 &m, double rho,
+                                                  dbl4 &S, double &T, double &blanked) {
+    uint32_t st = 0;
+    int it = m.iters;
+    if (it < 0) { st |= SPH_STATUS_SECANT_MAXITER; it = -it; }
+    jc_log_record(K, (float)y.svm, (float)y.eps_pl, (float)y.eps_pl_dot, (float)T, (float)y.norm,
+                  (float)m.delta_lambda, it, (float)y.dt);
+    jc_count(K, it);
+    const double back = fix_div(2. * K.c.phys.G * m.delta_lambda, y.norm);
+    S = mk4(__fma_rn(-S.x, back, S.x), __fma_rn(-S.y, back, S.y), __fma_rn(-S.z, back, S.z),
+            __fma_rn(-S.w, back, S.w));
+    if (K.c.trml_wp.tq != 0.)
+        T = __dadd_rn(T, fix_div(K.c.trml_wp.tq * (m.eps_pl - y.eps_pl) * m.sY, K.c.trml_wp.cp * rho));
+    if (T > K.c.joco.Tmelt) {
+        T = K.c.joco.Tmelt;
+        blanked = 1.;
+        st |= SPH_STATUS_MELT_BLANKED;
+    }
+    return st;
+}
+
 // ---- actions_gpu.cu:689-754 do_plasticity_johnson_cook (one particle) --------
 // Reads/writes the particle's S, eps_pl, eps_pl_dot, T, blanked.  Returns
 // status bits.  `iters_out` receives the secant iteration count (0 if elastic).
@@ -140,24 +257,32 @@ __device__ __forceinline__ uint32_t plasticity_one(const KConsts &K, double dt, 
     const sph_joco_constants &jc = K.c.joco;
     const double mu = K.c.phys.G;
     *iters_out = 0;
-    if (!kF32Yield && surely_elastic(K, S, p, eps_pl, eps_pl_dot, T)) {
-        eps_pl_dot = 0.;
-        return 0u;
+    if constexpr (!kF32Yield) {
+        if (surely_elastic(K, S, p, eps_pl, eps_pl_dot, T)) {
+            eps_pl_dot = 0.;
+            return 0u;
+        }
+        Mapping64 y = {0., 0., eps_pl, eps_pl_dot, T, dt};
+        trial_norms(S, p, y.norm, y.svm);
+        const Mapped64 m = return_mapping<false>(K, y);
+        eps_pl_dot = m.eps_pl_dot;
+        if (m.iters == 0) return 0u;
+        *iters_out = abs(m.iters);
+        eps_pl = m.eps_pl;
+        return apply_mapping(K, y, m, rho, S, T, blanked);
     }
     double Sxx = S.x, Syy = S.z, Szz = S.w, Sxy = S.y;
-    double norm_Strial = sqrtf_d(Sxx * Sxx + Syy * Syy + Szz * Szz + 2. * Sxy * Sxy);
-    double cxx = Sxx - p, cyy = Syy - p, czz = Szz - p, cxy = Sxy;
-    double svm = sqrtf_d((cxx * cxx + cyy * cyy + czz * czz) - cxx * cyy - cxx * czz - cyy * czz + 3.0 * cxy * cxy);
+    double norm_Strial, svm;
+    trial_norms(S, p, norm_Strial, svm);
     double term_c = jc_term_c(jc, T);
-    double sigma_Y = kF32Yield ? sigma_yield_tc_f32(jc, eps_pl, eps_pl_dot, term_c)
-                               : sigma_yield_tc(jc, eps_pl, eps_pl_dot, term_c);
+    double sigma_Y = sigma_yield_tc_f32(jc, eps_pl, eps_pl_dot, term_c);
     if (svm < sigma_Y) {
         eps_pl_dot = 0.;
         return 0u;
     }
     int it = 0;
-    double delta_lambda = solve_secant<kF32Yield>(jc, fmax(eps_pl_dot * dt * sqrt(2. / 3.), 1e-8), 1e-6, norm_Strial,
-                                                  eps_pl, term_c, dt, mu, &it, K.secant_cap);
+    double delta_lambda = solve_secant(jc, fmax(eps_pl_dot * dt * sqrt(2. / 3.), 1e-8), 1e-6, norm_Strial, eps_pl, term_c,
+                                       dt, mu, &it, K.secant_cap);
     uint32_t st = 0;
     if (it < 0) { st |= SPH_STATUS_SECANT_MAXITER; it = -it; }
     *iters_out = it;
@@ -179,8 +304,7 @@ __device__ __forceinline__ uint32_t plasticity_one(const KConsts &K, double dt, 
     S.y = Sxy - Sxy * back;
     if (K.c.trml_wp.tq != 0.) {
         double delta_eps_pl = eps_pl_new - eps_old;
-        double sY = kF32Yield ? sigma_yield_tc_f32(jc, eps_pl_new, eps_pl_dot_new, term_c)
-                              : sigma_yield_tc(jc, eps_pl_new, eps_pl_dot_new, term_c);
+        double sY = sigma_yield_tc_f32(jc, eps_pl_new, eps_pl_dot_new, term_c);
         T += fix_div(K.c.trml_wp.tq * delta_eps_pl * sY, K.c.trml_wp.cp * rho);
     }
     if (T > jc.Tmelt) {
