@@ -732,6 +732,13 @@ static void launch_i32(cudaStream_t s, int N, const KConsts &K, const int32_t *o
                  W.rec32, W.cand32, B, F, seg, tool, W.secant_iters, W.status, cap, mlp);
 }
 
+// The default shape up to three waves of five blocks an SM: no bound on the registers (95
+// instead of 79, five blocks instead of six), so that the loads of a pair and of the
+// epilogue are issued further ahead.  A small system has too few warps for the sixth block
+// to matter: step of 12,000 particles (cut) 71.1 -> 68.9 us, 90,000 (lattice) 62.7 -> 59.6,
+// 250,000 128.0 -> 124.4; but 422,500 194.6 -> 197.5.  Results do not depend on it.
+constexpr bool few_waves32(int N) { return N <= 3 * 5 * 152 * 128; }
+
 // The launch shapes of kInteractVariants (interactions.cu), in its order.
 template <bool kMlp>
 void launch_i32_variant(cudaStream_t s, int N, const KConsts &K, const int32_t *offsets, const SortedFields32 &B,
@@ -751,7 +758,10 @@ void launch_i32_variant(cudaStream_t s, int N, const KConsts &K, const int32_t *
         case 11: launch_i32<128, 6, false, kMlp, 4>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp); break;
         case 12: launch_i32<128, 5, false, kMlp>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp); break;
         case 13: launch_i32<64, 10, false, kMlp>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp); break;
-        default: launch_i32<128, 6, false, kMlp>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp); break;
+        default:
+            if (few_waves32(N)) launch_i32<128, 1, false, kMlp>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp);
+            else launch_i32<128, 6, false, kMlp>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp);
+            break;
     }
 }
 
