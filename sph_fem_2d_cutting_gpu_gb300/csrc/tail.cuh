@@ -529,29 +529,62 @@ __device__ __forceinline__ void contact_fem_warp(int i, const KConsts &K, const 
     double gN = 0.;
     double2 n_ = make_double2(0., 0.);
     if (inside) seg_no = shortest_distance_lanes(pos, gN, n_, cs, lane);
-    if (lane != 0) return;
-    double2 fc = d2(A.fc[i]), ft = d2(A.ft[i]), nrm = d2(A.n[i]);
-    int on = A.on_seg[i];
-    double bl = 0.;
+    double2 fc = make_double2(0., 0.), ft = fc, nrm = fc;
+    int on = -1;
+    bool blanked = false;
     uint32_t st = 0;
-    if (inside == 0) {
-        fc = make_double2(0., 0.); ft = make_double2(0., 0.); nrm = make_double2(0., 0.);
-        on = -1;
-    } else {
-        st = contact_s1_forces(K, tc.dt, tc, d2(A.vel[i]), seg_no, gN, n_, fc, ft, nrm, on, bl);
+    // contact_s1_forces and contact_s2_one, whose eleven divisions and roots -- a dozen
+    // operations on the FP64 pipe each, 64 cycles an operation whatever the number of
+    // lanes -- are taken by different lanes in four rounds.
+    if (inside != 0 && seg_no == -1) {
+        st = SPH_STATUS_CONTACT_NOSEG;
+    } else if (inside != 0 && gN < -0.00025) {
+        blanked = true;
+        st = SPH_STATUS_CONTACT_DEEP;
+    } else if (inside != 0) {
+        const double dt = tc.dt, dt2 = dt * dt, rho = A.rho[i];
+        const double2 vel = d2(A.vel[i]), ft0 = d2(A.ft[i]);
+        const double s1 = -K.c.tool.slave_mass * gN;
+        const double vx = vel.x - tc.vel[0], vy = vel.y - tc.vel[1];
+        const double vdn = vx * n_.x + vy * n_.y;
+        const double vrx = vx - n_.x * vdn, vry = vy - n_.y * vdn;
+        const double am = K.c.tool.contact_alpha * K.c.tool.slave_mass;
+        auto from = [&](double v, int l) { return __shfl_sync(kFullMask, v, l); };
+        const double num = lane == 0 ? s1 * n_.x : lane == 1 ? s1 * n_.y : lane == 2 ? am * vrx
+                         : lane == 3 ? am * vry : K.c.tool.slave_mass;
+        const double q1 = num / (lane < 2 ? dt2 : lane < 4 ? dt : rho);
+        fc = make_double2(from(q1, 0) * K.c.tool.contact_alpha, from(q1, 1) * K.c.tool.contact_alpha);
+        const double fsx = ft0.x - from(q1, 2), fsy = ft0.y - from(q1, 3);
+        const double px = lane == 0 ? fc.x : fsx, py = lane == 0 ? fc.y : fsy;
+        const double root = sqrt(px * px + py * py);
+        const double fy = K.c.tool.mu * from(root, 0), lfs = from(root, 1);
+        const double length = sqrtf_d(from(q1, 4));
+        on = seg_no + tc.seg_first;   // global segment id
+        const bool heat = on < seg.n;
+        double T = 0., delta_T = 0.;
+        if (heat) {
+            const int4 mk = seg.marks[on];
+            T = A.T[i];
+            delta_T = 0.5 * (T_nodes[mk.z] + T_nodes[mk.w]) - T;
+        }
+        const double q2 = (lane == 0 ? fy * fsx : lane == 1 ? fy * fsy : delta_T * K.c.tool.h * length) /
+                          (lane < 2 ? lfs : K.c.trml_wp.cp);
+        ft = lfs > fy ? make_double2(from(q2, 0), from(q2, 1)) : make_double2(fsx, fsy);
+        nrm = n_;
+        const double part = from(q2, 2) / K.c.tool.slave_mass * dt;
+        if (heat && lane == 0) {
+            atomicAdd(&seg.heat_exchange[on].x, T * length);
+            atomicAdd(&seg.heat_exchange[on].y, length);
+            T += part < 0 ? fmax(part, delta_T) : fmin(part, delta_T);
+            put(A.T[i], T);
+        }
     }
-    if (on >= 0) on += tc.seg_first;   // global segment id
-    const bool blanked = flag_is_one(bl);
+    if (lane != 0) return;
     if (blanked) put(A.blanked[i], 1.);
     put(A.ft[i], ft);
     put(A.n[i], nrm);
     A.on_seg[i] = on;
     put(A.fc[i], fc);
-    if (!blanked && on >= 0 && on < seg.n) {
-        double T = A.T[i];
-        contact_s2_one(K, tc.dt, seg, T_nodes, on, A.rho[i], T);
-        put(A.T[i], T);
-    }
     if (st) set_status(status, st);
 }
 
