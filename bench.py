@@ -59,10 +59,11 @@ ALGO_BYTES = {
 # 4,194,304 particles, k_interact32<fused, 128x6>; one-pass capture).
 NCU_TRAFFIC_PER_PARTICLE = {"fp32k": (723_139_584 + 398_211_584) / 4_194_304}
 # Floating-point work per particle of the fused neighbour sums, from ncu's SASS
-# instruction counters (dadd + dmul + 2 dfma; fadd + fmul + 2 ffma) on the
-# 512x512 micro workload with 2h cells (262,144 particles): k_interact64 executes
-# 1,401,475,197 FP64 flops, k_interact32 (compact state, 128x6) 1,402,179,265 FP32 flops.
-NCU_FLOPS_PER_PARTICLE = {"fp64": 1_401_475_197 / 262_144, "fp32k": 1_402_179_265 / 262_144}
+# instruction counters (dadd + dmul + 2 dfma; fadd + fmul + 2 ffma + 2 (fadd2 + fmul2) +
+# 4 ffma2, packed pairs counted as two) on the 512x512 micro workload with 2h cells
+# (262,144 particles): k_interact64 executes 540,407,316 FP64 flops (its products and
+# quotients are integer work), k_interact32 (compact state) 1,367,097,721 FP32 flops.
+NCU_FLOPS_PER_PARTICLE = {"fp64": 540_407_316 / 262_144, "fp32k": 1_367_097_721 / 262_144}
 # Nominal GB300 rates (no measured figure exists for these pipes): FP64 1.25 TFLOP/s;
 # FP32 152 SMs x 128 lanes x 2 flops x 2.07 GHz = 80.5 TFLOP/s.
 NOMINAL_TFLOPS = {"fp64": 1.25, "fp32k": 80.5}

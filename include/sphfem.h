@@ -541,11 +541,11 @@ int sph_set_test_faults(sph_ctx *ctx, uint32_t faults, int32_t secant_cap);
  * Runs `nsteps` fused steps without the CUDA graph, with CUDA events on the
  * context stream between the stages; stage_ms[k] receives the summed device
  * time of stage k over the steps: 0 histogram/hash (previous step's tail when
- * chained), 1 scan+scatter (+ FEM half step), 2 in-cell rank and reorder gather
+ * chained), 1 scan+scatter (+ FEM half step or rigid tool move), 2 in-cell rank and reorder gather
  * (+predict, EOS, artificial stress, records), 3 PSE conduction, 4 neighbour sums +
  * fused epilogue (+ wear statistics reset, warm-started return mapping),
- * 5 FEM rate/update (+ wear adjustment) + tool move (+ rigid tool move),
- * 6 contact/BC/invalidate tail (+ next histogram).  The steps are the same
+ * 5 FEM rate/update (+ wear adjustment) + tool move, 6 contact/BC/invalidate tail
+ * (+ next histogram; on small systems the FEM rate/update and the nodes' move).  The steps are the same
  * as those of sph_step_fused.  n_stages receives 7. */
 int sph_profile_steps(sph_ctx *ctx, int32_t nsteps, float *stage_ms, int32_t *n_stages);
 

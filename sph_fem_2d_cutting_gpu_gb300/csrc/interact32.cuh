@@ -736,7 +736,8 @@ static void launch_i32(cudaStream_t s, int N, const KConsts &K, const int32_t *o
 // instead of 79, five blocks instead of six), so that the loads of a pair and of the
 // epilogue are issued further ahead.  A small system has too few warps for the sixth block
 // to matter: step of 12,000 particles (cut) 71.1 -> 68.9 us, 90,000 (lattice) 62.7 -> 59.6,
-// 250,000 128.0 -> 124.4; but 422,500 194.6 -> 197.5.  Results do not depend on it.
+// 250,000 128.0 -> 124.4; but 422,500 194.6 -> 197.5.  The sums are the same; as between
+// all shapes, the compiler may fuse a multiply-add of the epilogue differently.
 constexpr bool few_waves32(int N) { return N <= 3 * 5 * 152 * 128; }
 
 // The launch shapes of kInteractVariants (interactions.cu), in its order.

