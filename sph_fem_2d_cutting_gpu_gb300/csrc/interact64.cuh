@@ -224,8 +224,13 @@ static __device__ __noinline__ void return_map(int k, const KConsts &K, const So
 // grids of up to one wave (map_by_quads).
 enum Map64 { kMapNone, kMapLane, kMapQuads };
 inline bool map_by_quads(int N) { return div_up(N, kParts64) <= 5 * 152; }
-template <Map64 kMap>
-__global__ void __launch_bounds__(kThreads64, 5) k_interact64(int N, KConsts K, const int32_t *__restrict__ offsets,
+// kBlocks: blocks an SM that the registers must leave room for -- 5 on a grid of many
+// waves (below); 3, with 162 registers and nothing spilled, on one that needs no more
+// (three_blocks): step of 12,000 particles (cut) 112.2 -> 107.4 us, of 7,355 (rigid, PSE)
+// 93.2 -> 89.4, of 1,600 (lattice) 58.5 -> 53.3; but of 19,600 99.6 -> 117.4.
+inline bool three_blocks(int N) { return div_up(N, kParts64) <= 3 * 152; }
+template <Map64 kMap, int kBlocks = 5>
+__global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KConsts K, const int32_t *__restrict__ offsets,
                                                               const dbl4 *__restrict__ rec,
                                                               const float2 *__restrict__ cand, SortedFields B,
                                                               FixedFields F, SegDev seg,

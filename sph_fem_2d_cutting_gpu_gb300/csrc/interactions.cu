@@ -210,7 +210,11 @@ void launch_interactions(cudaStream_t s, int N, const KConsts &K, const int32_t 
     } else {
         const int g64 = div_up(N, kParts64);
         if (fused)
-            launch_after(s, map_by_quads(N) ? k_interact64<kMapQuads> : k_interact64<kMapLane>, g64, kThreads64, 0, N, K, offsets, W.rec64, W.cand32, B, F, seg, tool,
+            launch_after(s,
+                         three_blocks(N)   ? k_interact64<kMapQuads, 3>
+                         : map_by_quads(N) ? k_interact64<kMapQuads>
+                                           : k_interact64<kMapLane>,
+                         g64, kThreads64, 0, N, K, offsets, W.rec64, W.cand32, B, F, seg, tool,
                          W.secant_iters, W.status);
         else
             k_interact64<kMapNone><<<g64, kThreads64, 0, s>>>(N, K, offsets, W.rec64, W.cand32, B, F, seg, tool,

@@ -1,7 +1,8 @@
 """FP64 return mapping: a case small enough for groups of four lanes (one wave of the sums'
-blocks, 5 * 152 * 32 particles) and the same case first in a batch too large for them, where
-each lane maps its own particle.  The two share their arithmetic rounding for rounding, so the
-case ends with the same bits, yielding particles included."""
+blocks; with the registers of three blocks an SM up to 3 * 152 * 32 particles, of five up to
+5 * 152 * 32) and the same case first in a batch too large for them, where each lane maps its
+own particle.  They share their arithmetic rounding for rounding, so the case ends with the same
+bits, yielding particles included."""
 import numpy as np
 import pytest
 
@@ -22,13 +23,14 @@ def cut(speed):
 @pytest.mark.parametrize("steps", [1, 40])
 def test_lanes_and_groups_map_alike(lib, steps):
     out = []
-    for n_cases in (1, 5):
+    for n_cases in (1, 3, 5):
         b = Batch([cut(300.0)] + [cut(120.0 + 10 * k) for k in range(n_cases - 1)], abi.SPH_PREC_FP64)
-        assert (b.N <= 5 * 152 * 32) == (n_cases == 1)
+        assert (b.N <= 3 * 152 * 32) == (n_cases == 1) and (b.N <= 5 * 152 * 32) == (n_cases <= 3)
         b.step(steps)
         out.append(b.download_cases(FIELDS)[0])
         b.close()
     for f in FIELDS:
         assert np.array_equal(out[0][f], out[1][f], equal_nan=True), f
+        assert np.array_equal(out[0][f], out[2][f], equal_nan=True), f
     if steps == 40:
         assert np.count_nonzero(out[0]["eps_pl_dot"]) > 20   # particles on the yield surface
