@@ -16,7 +16,7 @@
 //    runs once per particle in full warps from partial sums in shared memory.
 // Neighbour stage, before and after: 1,048,576-particle lattice (2h cells) 9.40 ->
 // 2.88 ms; 640,000-particle cut (cells of h) 5.53 -> 1.78 ms; 12,000-particle cut
-// 0.247 -> 0.072 ms, the return mapping of the yielding particles (return_map) included.
+// 0.247 -> 0.068 ms, the return mapping of the yielding particles (return_map) included.
 // A particle with anything the mantissa forms do not take (a candidate marked
 // non-finite, a smoothing length, density or volume outside 2^+-64) repeats its
 // sums in plain FP64 over every active candidate, with the reference's zero
@@ -211,9 +211,6 @@ static __device__ __noinline__ void return_map(int k, const KConsts &K, const So
     if (st) set_status(status, st);
 }
 
-// 5 blocks (20 warps) an SM at 96 registers, with 140 bytes spilled: the warps
-// alternate between the integer and the FP64 pipe, and 4 blocks at 128 registers
-// were 5 % slower on the 1,048,576-particle lattice, 3 blocks 13 %.
 // ---- the kernel --------------------------------------------------------------------------------------
 // kMapNone: the staged sums.  kMapLane, kMapQuads: the fused step, its return mappings in
 // the epilogue's lanes or in groups of four lanes of the whole block.  The groups cut a
@@ -224,10 +221,13 @@ static __device__ __noinline__ void return_map(int k, const KConsts &K, const So
 // grids of up to one wave (map_by_quads).
 enum Map64 { kMapNone, kMapLane, kMapQuads };
 inline bool map_by_quads(int N) { return div_up(N, kParts64) <= 5 * 152; }
-// kBlocks: blocks an SM that the registers must leave room for -- 5 on a grid of many
-// waves (below); 3, with 162 registers and nothing spilled, on one that needs no more
-// (three_blocks): step of 12,000 particles (cut) 112.2 -> 107.4 us, of 7,355 (rigid, PSE)
-// 93.2 -> 89.4, of 1,600 (lattice) 58.5 -> 53.3; but of 19,600 99.6 -> 117.4.
+// kBlocks: blocks an SM that the registers must leave room for.  5 (20 warps, 96
+// registers, 164 bytes spilled) on a grid of many waves, where warps alternate between the
+// integer and the FP64 pipe: 4 blocks at 128 registers were 5 % slower on the
+// 1,048,576-particle lattice, 3 blocks 13 %.  3, with 162 registers and nothing spilled, on
+// a grid that needs no more (three_blocks): step of 12,000 particles (cut) 112.2 -> 107.4 us,
+// of 7,355 (rigid, PSE) 93.2 -> 89.4, of 1,600 (lattice) 58.5 -> 53.3; but of 19,600 99.6 ->
+// 117.4.
 inline bool three_blocks(int N) { return div_up(N, kParts64) <= 3 * 152; }
 template <Map64 kMap, int kBlocks = 5>
 __global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KConsts K, const int32_t *__restrict__ offsets,
