@@ -479,6 +479,7 @@ int issue_fused_body(sph_ctx *ctx, int64_t &n, int w, cudaEvent_t *ev = nullptr)
     SegDev sw = ctx->seg;
     if (ctx->wear_mode != SPH_WEAR_OFF) {   // segments_wear_rate_reset (leap_frog.cu:183-186)
         launch_wear_reset(s, ctx->seg);
+        n += 1;
         sw.wear.T_nodes = ctx->fem.T_half;  // the friction heat sees the half-step FEM temperature
     }
     const bool mlp_tensor = ctx->mlp_on && ctx->mlp_mode == SPH_MLP_TENSOR;

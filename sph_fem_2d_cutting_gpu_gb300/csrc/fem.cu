@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(kBlock) k_fem_temp(FemDev F, const double *__r
 
 __global__ void __launch_bounds__(kBlock) k_tool_move(KConsts K, SegDev seg, FemDev F, ToolDev *tool, double dt,
                                                       int what, int per_case) {
+    begin_after();
     tool_move_one(blockIdx.x * blockDim.x + threadIdx.x, K, seg, F, tool, dt, what, per_case);
 }
 
@@ -115,7 +116,7 @@ void launch_tool_move(cudaStream_t s, const KConsts &K, const SegDev &seg, const
     int n = per_case ? K.n_cases : 1;
     if ((what & 1) && seg.n > n) n = seg.n;
     if ((what & 6) && F.n_nodes > n) n = F.n_nodes;
-    k_tool_move<<<div_up(n, kBlock), kBlock, 0, s>>>(K, seg, F, tool, dt, what, per_case ? 1 : 0);
+    launch_after(s, k_tool_move, div_up(n, kBlock), kBlock, 0, K, seg, F, tool, dt, what, per_case ? 1 : 0);
 }
 
 // ---- set-up of the thermal system on the device (FEM_thermal_gpu.cu:126-332) ----------

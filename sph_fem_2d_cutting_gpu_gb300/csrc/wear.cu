@@ -17,6 +17,7 @@ namespace sphfem {
 // positions (do_mass_ele_matrix_construction_p1q3 /
 // do_stiffness_ele_matrix_construction_p1q3), one element per thread.
 __global__ void __launch_bounds__(kBlock) k_wear_elements(KConsts K, FemDev F, WearDev W, double *__restrict__ out) {
+    begin_after();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= W.n_elem) return;
     const int4 el = W.elements[W.elem[k]];
@@ -35,6 +36,7 @@ __global__ void __launch_bounds__(kBlock) k_wear_elements(KConsts K, FemDev F, W
 // positions, and rebuilds its lumped inverse mass (do_inverse_mass_matrix_lumped,
 // FEM_thermal_gpu.cu:326-331; the other nodes' entries do not change).
 __global__ void __launch_bounds__(kBlock) k_wear_layers(FemDev F, WearDev W) {
+    begin_after();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= W.n_nodes) return;
     const int i = W.node[idx];
@@ -64,6 +66,7 @@ __global__ void __launch_bounds__(kBlock) k_wear_layers(FemDev F, WearDev W) {
 // temperatures, and the shift along the segment normal (nodal_shift,
 // tool_FEM.cu:49-55).  The shift is applied by k_wear_node_shift.
 __global__ void __launch_bounds__(kBlock) k_wear_segment_shift(FemDev F, SegDev seg, WearDev W, double dt) {
+    begin_after();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= seg.n) return;
     W.seg_delta[s] = mk4(0., 0., 0., 0.);
@@ -93,6 +96,7 @@ __global__ void __launch_bounds__(kBlock) k_wear_segment_shift(FemDev F, SegDev 
 
 // Each node adds the shifts of the segments ending on it, in segment order.
 __global__ void __launch_bounds__(kBlock) k_wear_node_shift(FemDev F, SegDev seg, WearDev W) {
+    begin_after();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= F.n_nodes) return;
     const int t0 = F.node_seg_ptr[i], t1 = F.node_seg_ptr[i + 1];
@@ -122,6 +126,7 @@ __global__ void __launch_bounds__(kBlock) k_wear_node_shift(FemDev F, SegDev seg
 constexpr int kFlankSegments = 512;
 constexpr int kFlankThreads = 256;
 __global__ void __launch_bounds__(kFlankThreads) k_wear_segments_flank(FemDev F, SegDev seg, ToolDev *tool) {
+    begin_after();
     __shared__ double s_min[kFlankThreads], s_ymin[kFlankThreads], s_ymax[kFlankThreads], s_xmax[kFlankThreads],
         s_dxdy[kFlankThreads];
     double mn = 3.402823466385288598e38, ymin = INFINITY, ymax = -INFINITY, xmax = -INFINITY, dxdy = 0.;
@@ -162,10 +167,17 @@ __global__ void __launch_bounds__(kFlankThreads) k_wear_segments_flank(FemDev F,
 }
 
 // ---- host launchers -------------------------------------------------------------------------------
+// segments_wear_rate_reset: one launch of the chain instead of three memsets in it.
+__global__ void __launch_bounds__(kBlock) k_wear_reset(SegDev seg) {
+    begin_after();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= seg.n) return;
+    seg.wear.pp[i] = mk4(0., 0., 0., 0.);
+    seg.wear.sf[i] = 0.;
+    seg.wear_rate[i] = 0.;
+}
 void launch_wear_reset(cudaStream_t s, const SegDev &seg) {
-    cudaMemsetAsync(seg.wear.pp, 0, sizeof(dbl4) * (size_t)seg.n, s);
-    cudaMemsetAsync(seg.wear.sf, 0, sizeof(double) * (size_t)seg.n, s);
-    cudaMemsetAsync(seg.wear_rate, 0, sizeof(double) * (size_t)seg.n, s);
+    if (seg.n > 0) launch_after(s, k_wear_reset, div_up(seg.n, kBlock), kBlock, 0, seg);
 }
 
 // Few hundred threads of FP64 element work: blocks as small as needed to
@@ -174,12 +186,12 @@ void launch_wear_adjustment(cudaStream_t s, const KConsts &K, const FemDev &F, c
                             ToolDev *tool, double dt) {
     const int ne = W.n_elem > 0 ? W.n_elem : 1, nl = W.n_nodes > 0 ? W.n_nodes : 1, ns = seg.n > 0 ? seg.n : 1;
     const int be = fp64_block(ne), bl = fp64_block(nl), bs = fp64_block(ns), bn = fp64_block(F.n_nodes);
-    k_wear_elements<<<div_up(ne, be), be, 0, s>>>(K, F, W, W.mat_old);
-    k_wear_segment_shift<<<div_up(ns, bs), bs, 0, s>>>(F, seg, W, dt);
-    k_wear_node_shift<<<div_up(F.n_nodes, bn), bn, 0, s>>>(F, seg, W);
-    k_wear_elements<<<div_up(ne, be), be, 0, s>>>(K, F, W, W.mat_new);
-    k_wear_layers<<<div_up(nl, bl), bl, 0, s>>>(F, W);
-    k_wear_segments_flank<<<1, kFlankThreads, 0, s>>>(F, seg, tool);
+    launch_after(s, k_wear_elements, div_up(ne, be), be, 0, K, F, W, W.mat_old);
+    launch_after(s, k_wear_segment_shift, div_up(ns, bs), bs, 0, F, seg, W, dt);
+    launch_after(s, k_wear_node_shift, div_up(F.n_nodes, bn), bn, 0, F, seg, W);
+    launch_after(s, k_wear_elements, div_up(ne, be), be, 0, K, F, W, W.mat_new);
+    launch_after(s, k_wear_layers, div_up(nl, bl), bl, 0, F, W);
+    launch_after(s, k_wear_segments_flank, 1, kFlankThreads, 0, F, seg, tool);
 }
 
 // ---- remesh_low_level (tool_FEM.cu:1696-1705) -----------------------------------------------
