@@ -80,8 +80,9 @@ __global__ void __launch_bounds__(1024) k_scan_top(int32_t *__restrict__ block_s
 // = one past the last slot, left untouched for empty cells (stale, as the
 // reference leaves it).  kTop: block_sums holds the tiles' sums, which every block
 // adds up to its own start; otherwise k_scan_top has scanned them.  The counts,
-// read here for the last time, go back to zero for the next histogram (and with
-// them counts[n], the contact queue's length).
+// read here for the last time, go back to zero for the next histogram, and with
+// them counts[n], the contact queue's length: by a thread of its own, as the tiles
+// end at n - 1 when n is a multiple of kScanTile.
 template <bool kTop>
 __global__ void __launch_bounds__(kScanThreads) k_scan_down(int32_t *__restrict__ counts, int n,
                                                             const int32_t *__restrict__ block_sums,
@@ -97,8 +98,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(int32_t *__restrict_
     for (int k = 0; k < kScanItems; k++) {
         v[k] = (base + k < n) ? counts[base + k] : 0;
         s += v[k];
-        if (base + k <= n) counts[base + k] = 0;
+        if (base + k < n) counts[base + k] = 0;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) counts[n] = 0;
     int start = 0;
     if (kTop) {
         int p = 0;
@@ -400,7 +402,7 @@ void launch_hash(cudaStream_t s, int N, const SortedFields &A, sph_geom_constant
 template <class SF>
 static void count(cudaStream_t s, int N, const SF &A, const SortScratch &X, sph_geom_constants g, uint32_t *status,
                   bool with_hash) {
-    cudaMemsetAsync(X.counts, 0, sizeof(int32_t) * (size_t)(g.num_cell + 1), s);
+    cudaMemsetAsync(X.counts, 0, sizeof(int32_t) * ((size_t)g.num_cell + 2), s);   // and the queue's length
     if (with_hash)
         k_hash_count<true, true><<<div_up(N, kBlock), kBlock, 0, s>>>(N, A.pos, A.blanked, A.hash, X.key, X.arrival,
                                                                        X.counts, X.hash_next, g, (float)(1.0 / g.dx), status);
