@@ -92,16 +92,20 @@ __device__ __forceinline__ double solve_secant(const sph_joco_constants &jc, dou
 // false): an elastic particle then needs nothing else of the three pow() calls
 // that the yield stress costs on the FP64 pipe.  The von Mises stress is formed
 // from the deviatoric differences, which the pressure does not enter; `pf`
-// bounds the reference's own cancellation.  The flow stress is discontinuous at
-// eps_dot = 1 (plasticity.cuh:29-33).
+// bounds the reference's own cancellation, and a state so nearly hydrostatic that its
+// sum of squares may cancel to below zero (a few 1e-15 of the largest)
+// is not decided here: its NaN goes through the return mapping, as in the reference.
+// The flow stress is discontinuous at eps_dot = 1 (plasticity.cuh:29-33).
 __device__ __forceinline__ bool surely_elastic(const KConsts &K, dbl4 S, double p, double eps_pl, double eps_pl_dot,
                                                double T) {
     const JcF32 &j = K.f.jc;
     const float a = float_trunc(S.x), b = float_trunc(S.z), c = float_trunc(S.w), d = float_trunc(S.y);
     const float pf = float_trunc(p);
     const float ab = a - b, bc = b - c, ca = c - a;
-    const float svm = sqrtf(0.5f * (ab * ab + bc * bc + ca * ca) + 3.f * d * d + 1e-12f * pf * pf) +
-                      1e-5f * (fabsf(a) + fabsf(b) + fabsf(c) + fabsf(d));
+    const float dev2 = 0.5f * (ab * ab + bc * bc + ca * ca) + 3.f * d * d;
+    const float size = fabsf(a) + fabsf(b) + fabsf(c) + fabsf(d), all = size + fabsf(pf);
+    if (!(dev2 >= 1e-12f * all * all)) return false;
+    const float svm = sqrtf(dev2 + 1e-12f * pf * pf) + 1e-5f * size;
     const float theta = fminf(float_trunc(T - K.c.joco.Tref) * j.inv_dT, 1.f);
     const float term_c = 1.f - powf(theta, j.m) - 1e-5f;
     const float eps_dot = float_trunc(eps_pl_dot) * j.inv_epsdot_ref;
