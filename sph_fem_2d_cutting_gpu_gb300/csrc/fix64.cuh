@@ -46,16 +46,29 @@ __device__ __forceinline__ Fix64 fix_norm(Fix64 a) {
     return {a.m << z, a.e - z};
 }
 
-// The double nearest to m * 2^e (ties away from zero); below 2^-1022: 0.
+// The bits of the double nearest to m 2^(biased - 1086) for an exponent field that no normal
+// double has: infinity, or a subnormal (ties away from zero) or zero.
+__device__ __forceinline__ uint64_t fix_ends(uint64_t m, int biased) {
+    if (biased > 0) return 0x7ff0000000000000ull;
+    const int s = min(12 - biased, 65);
+    return s > 64 ? 0ull : ((m >> (s - 1)) >> 1) + ((m >> (s - 1)) & 1ull);
+}
+
+// The double nearest to m * 2^e (ties away from zero).  kEnds false, for results that are
+// below 2^1024 by the ranges of what they are formed from: 0 below 2^-1022.
+template <bool kEnds = true>
 __device__ __forceinline__ double fix_double(Fix64 a) {
     a = fix_norm(a);
     const int biased = a.e + 1086;
     const uint64_t r = (a.m >> 11) + ((a.m >> 10) & 1ull);   // the implicit bit adds 1 to the exponent field
-    const uint64_t b = ((uint64_t)(uint32_t)(biased - 1) << 52) + r;
-    return (biased <= 0 || (long long)a.m >= 0) ? 0. : __longlong_as_double((long long)b);
+    uint64_t b = ((uint64_t)(uint32_t)(biased - 1) << 52) + r;
+    if (kEnds && (uint32_t)(biased - 1) >= 2046u) b = fix_ends(a.m, biased);
+    return ((!kEnds && biased <= 0) || (long long)a.m >= 0) ? 0. : __longlong_as_double((long long)b);
 }
 
-// The double nearest to a * x * (-1)^negative for a with its top bit set; 0 for x = 0.
+// The double nearest to a * x * (-1)^negative for a with its top bit set (or 0) and a normal
+// x (or 0); kEnds as above.
+template <bool kEnds = true>
 __device__ __forceinline__ double fix_scale(Fix64 a, double x, bool negative = false) {
     const uint64_t b = (uint64_t)__double_as_longlong(x);
     uint64_t m = mul_hi(a.m, (b << 11) | 0x8000000000000000ull);   // [2^62, 2^64)
@@ -66,8 +79,10 @@ __device__ __forceinline__ double fix_scale(Fix64 a, double x, bool negative = f
     }
     const uint64_t r = (m >> 11) + ((m >> 10) & 1ull);
     const uint64_t sign = ((b >> 32) & 0x80000000ull) ^ (negative ? 0x80000000ull : 0ull);
-    const uint64_t v = (sign << 32) + ((uint64_t)(uint32_t)(biased - 1) << 52) + r;
-    return (biased <= 0 || !flag_nonzero(x)) ? 0. : __longlong_as_double((long long)v);
+    uint64_t v = ((uint64_t)(uint32_t)(biased - 1) << 52) + r;
+    if (kEnds && (uint32_t)(biased - 1) >= 2046u) v = fix_ends(m, biased);
+    const bool zero = (!kEnds && biased <= 0) || !flag_nonzero(x) || (kEnds && (long long)m >= 0);
+    return zero ? 0. : __longlong_as_double((long long)((sign << 32) + v));
 }
 
 // 2^114 / M for M in [2^52, 2^53): (2^61, 2^62], error below 2^5 units.

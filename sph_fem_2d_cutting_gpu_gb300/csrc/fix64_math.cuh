@@ -129,7 +129,7 @@ __device__ __forceinline__ Fix64 fix_log2(double x, bool &negative) {
     return fix_norm({b ? ((uint64_t)(uint32_t)E << (64 - b)) | (f >> b) : f, b - 64});
 }
 
-// 2^(+-y) for y < 2^10 with its top bit set (or 0).
+// 2^(+-y) for y < 2^11 with its top bit set (or 0).
 __device__ __forceinline__ Fix64 fix_exp2(Fix64 y, bool negative) {
     int n = 0;
     uint64_t F;

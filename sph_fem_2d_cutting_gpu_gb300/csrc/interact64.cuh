@@ -18,7 +18,8 @@
 // 2.88 ms; 640,000-particle cut (cells of h) 5.53 -> 1.78 ms; 12,000-particle cut
 // 0.247 -> 0.068 ms, the return mapping of the yielding particles (return_map) included.
 // A particle with anything the mantissa forms do not take (a candidate marked
-// non-finite, a smoothing length, density or volume outside 2^+-64) repeats its
+// non-finite, a smoothing length, density or volume outside 2^+-64, a product of
+// relative velocity and distance that is subnormal or 2^300 and more) repeats its
 // sums in plain FP64 over every active candidate, with the reference's zero
 // weights outside the support (interactions_gpu.cu:230-337).
 #pragma once
@@ -32,6 +33,9 @@ constexpr int kLanes64 = 4;                            // lanes per particle
 constexpr int kThreads64 = 128;                        // threads per block
 constexpr int kParts64 = kThreads64 / kLanes64;        // particles per block
 constexpr int kList64 = 64, kListPitch64 = kList64 + 4;   // neighbours per pass; the pitch spreads a warp's lists over the banks
+
+// |x| < 2^500: with such viscosity constants and (v, x) below 2^300 no product overflows.
+__device__ __forceinline__ bool below_2_500(double x) { return ((uint32_t)__double2hiint(x) & 0x7fffffffu) < 0x5f300000u; }
 
 // v_der, S_der / mass, vel_t / (-mass), pos_t / (eps mass), T_lapl / 2
 struct Sums64 {
@@ -266,7 +270,7 @@ __global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KCons
     // q > 1: w = (2-q)^6 / 4, dW/(r dr) = -3/4 fac h1 (2-q)^2 / r;
     // q <= 1: w = 1 - 3/2 q^2 + 3/4 q^3, dW/(r dr) = -3 fac h1^2 (1 - 3/4 q).
     bool plain = !fix_range(hi) || !fix_range(K.inv_wdeltap) || !fix_range(fourh2 + eta2h2) ||
-                 (fi & kFlagNonFinite);
+                 !below_2_500(K.c.corr.alpha) || !below_2_500(K.c.corr.beta) || (fi & kFlagNonFinite);
     const double h_safe = plain ? 1. : hi;
     const Fix64 h1 = fix_recip_rn(h_safe), hm = fix_of(h_safe);
     const Fix64 fac = fix_norm(fix_of(kPiFac) * (h1 * h1));
@@ -355,26 +359,29 @@ __global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KCons
             dw = dw * Fix64{far ? u2.m : (1ull << 63) - q1 + (q1 >> 2), far ? u2.e : -63};
             dw = fix_norm(dw);   // |dW/dr| / r
             const Fix64 g = fix_norm(dw * fix_of(n3.y));
-            if (thermal) tl += (n3.z - i3.z) * fix_double(g);
+            if (thermal) tl += (n3.z - i3.z) * fix_double<false>(g);
             if (tool_i || (fj & kFlagTool)) continue;
             const Fix64 w = fix_norm(val) * fac;
             const Fix64 irho = fix_recip(sum_rho);
-            const double wx = fix_scale(dw, ex), wy = fix_scale(dw, ey);
-            const double tx = fix_scale(g, ex), ty = fix_scale(g, ey);
+            const double wx = fix_scale<false>(dw, ex), wy = fix_scale<false>(dw, ey);
+            const double tx = fix_scale<false>(g, ex), ty = fix_scale<false>(g, ey);
             const double dvx = n0.z - i0.z, dvy = n0.w - i0.w;
             vd0 += dvx * tx;
             vd1 += dvx * ty;
             vd2 += dvy * tx;
             vd3 += dvy * ty;
             const Fix64 f1 = fix_norm(w * iwdp), f2 = f1 * f1;
-            const double fab = fix_double(f2 * f2);
+            const double fab = fix_double<false>(f2 * f2);
             const Fix64 wr2 = w * irho;
-            const double wr = fix_double({wr2.m, wr2.e + 1});   // W / (0.5 (rho_i + rho_j))
+            const double wr = fix_double<false>({wr2.m, wr2.e + 1});   // W / (0.5 (rho_i + rho_j))
             const double vijposij = dvx * ex + dvy * ey;
             double sxx = i1.x + n1.x, syy = i1.z + n1.z;
             const double sxy = (i1.y + n1.y) + fab * (i2.x + n2.x);
             // viscosity, for approaching pairs: mu < 0, Pi = mu (-alpha c + beta mu) / (0.5 (rho_i + rho_j))
-            const bool approach = __double2hiint(vijposij) < 0 && flag_nonzero(vijposij);
+            // -2^-1022 >= (v, x) > -2^300; a subnormal product and a diverging state's in plain FP64
+            const uint32_t vh = (uint32_t)__double2hiint(vijposij);
+            const bool approach = vh - 0x80100000u < 0x52a00000u;
+            if (!approach && (int)vh < 0 && flag_nonzero(vijposij)) plain = true;
             Fix64 hd = hm * fix_recip(rr2 + eta2h2);   // h_ij / (r^2 + eta^2 h_ij^2)
             if (__double_as_longlong(n2.z) != __double_as_longlong(hi)) {
                 // the division keeps this a branch: predicated, its FP64 operations would
@@ -384,7 +391,7 @@ __global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KCons
                 hd = fix_of(x);
             }
             const Fix64 mu = fix_norm(fix_norm(hd) * fix_abs(vijposij));
-            const double cmu = (i3.x + n3.x) - K.c.corr.beta * fix_double(mu);
+            const double cmu = (i3.x + n3.x) - K.c.corr.beta * fix_double<false>(mu);
             const Fix64 s1 = fix_norm(mu * irho);
             double piij = fix_scale({s1.m, s1.e + 1}, cmu, true);
             if (!approach) piij = 0.;

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(128) k_heat_pse64(int N, KConsts K, const int3
             if (plain || !fix_range(n3.y) || (uint32_t)__double2hiint(rr2) >= 0x7ff00000u) {
                 w = pse_weight_general(rr2, 1. / h2, n3.y);
             } else {
-                w = y.e + 63 > 9 ? 0. : fix_double(fix_exp2(y, true) * fix_of(n3.y));
+                w = y.e + 63 > 10 ? 0. : fix_double(fix_exp2(y, true) * fix_of(n3.y));
             }
             sum += (n3.z - Ti) * w;
             j += kPseLanes;

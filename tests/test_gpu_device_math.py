@@ -1,0 +1,96 @@
+"""The arithmetic on 64-bit mantissas (csrc/fix64.cuh) as compiled: its functions evaluated on the
+GPU element by element (device_math.cu), against exact rationals and correctly rounded doubles,
+over random arguments and over the ends of their ranges."""
+import ctypes as C
+import math
+import subprocess
+from fractions import Fraction
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+from sph_fem_2d_cutting_gpu_gb300 import build
+
+pytestmark = pytest.mark.gpu
+
+OPS = ("fix_double", "fix_scale")
+
+
+@pytest.fixture(scope="module")
+def evaluate(tmp_path_factory):
+    so = tmp_path_factory.mktemp("device_math") / "device_math.so"
+    subprocess.run([build.nvcc(), *build.NVCC_FLAGS, "-I", str(build.CSRC), "-shared", str(Path(__file__).with_name("device_math.cu")),
+                    "-o", str(so)], check=True)
+    lib = C.CDLL(str(so))
+
+    def call(op, a, b=None, e=None):
+        a = np.ascontiguousarray(a, np.uint64)
+        b = np.zeros_like(a) if b is None else np.ascontiguousarray(b, np.uint64)
+        e = np.zeros(len(a), np.int32) if e is None else np.ascontiguousarray(e, np.int32)
+        out = np.empty_like(a)
+        r = lib.device_math(OPS.index(op), len(a), *(v.ctypes.data_as(C.c_void_p) for v in (a, b, e, out)))
+        assert r == 0, f"{op}: CUDA error {r}"
+        return out
+
+    return call
+
+
+def bits(x):
+    return np.asarray(x, np.float64).view(np.uint64)
+
+
+def nearest(f):
+    """The double nearest to a rational, infinity beyond the largest."""
+    try:
+        return float(f)
+    except OverflowError:
+        return math.inf if f > 0 else -math.inf
+
+
+def random_words(rng, n):
+    return rng.integers(0, 1 << 64, n, dtype=np.uint64, endpoint=False)
+
+
+def test_double_of_a_mantissa(evaluate):
+    """Every exponent from below the subnormals to beyond the largest double."""
+    rng = np.random.default_rng(1)
+    e = np.concatenate([np.arange(-1200, 1100), rng.integers(-1145, -1070, 2000), rng.integers(955, 966, 200)])
+    m = random_words(rng, len(e)) | np.uint64(1 << 63)
+    m[::3] >>= np.uint64(7)   # not normalised
+    m[1::97] = np.uint64((1 << 64) - 1)
+    m[2::97] = np.uint64(1 << 63)
+    m[5::97] = 0
+    got = evaluate("fix_double", m, e=e).view(np.float64)
+    for g, mi, ei in zip(got.tolist(), m.tolist(), e.tolist()):
+        f = Fraction(mi) * Fraction(2) ** ei
+        want = nearest(f)
+        # ties go away from zero, to the neighbour of equal distance
+        assert g == want or abs(Fraction(g) - f) == abs(Fraction(want) - f) and g > want, (mi, ei)
+        assert math.copysign(1.0, g) == 1.0
+
+
+def test_scaled_double(evaluate):
+    """a * x with the product at and beyond both ends of the doubles; the mantissa product is short
+    by less than 3 units of 2^-64 of its leading word, so the result is within 0.51 units."""
+    rng = np.random.default_rng(2)
+    n = 6000
+    m = random_words(rng, n) | np.uint64(1 << 63)
+    x = rng.choice([-1.0, 1.0], n) * rng.uniform(1.0, 2.0, n) * 2.0 ** rng.integers(-1000, 1000, n).astype(np.float64)
+    target = np.concatenate([rng.integers(-1090, -1010, n // 3), rng.integers(1010, 1030, n // 3),
+                             rng.integers(-1200, 1200, n - 2 * (n // 3))])
+    e = (target - 64 - np.frexp(x)[1]).astype(np.int32)
+    x[::50] = 0.0
+    x[7::50] = -0.0
+    m[3::50] = 0
+    got = evaluate("fix_scale", m, bits(x), e).view(np.float64)
+    for g, mi, xi, ei in zip(got.tolist(), m.tolist(), x.tolist(), e.tolist()):
+        f = Fraction(mi) * Fraction(xi) * Fraction(2) ** ei * (-1 if ei & 1 else 1)
+        want = nearest(f)
+        if math.isinf(g) or math.isinf(want) or f == 0:
+            # beyond the largest double plus half a unit: infinity, with the product's sign
+            assert g == want or abs(f) > Fraction(2) ** 1024 * (1 - Fraction(1, 1 << 53)), (mi, xi, ei)
+        else:
+            unit = Fraction(math.ulp(want))
+            assert abs(Fraction(g) - f) <= Fraction(51, 100) * unit, (mi, xi, ei)
+            assert g == 0.0 or (g > 0) == (f > 0)

@@ -3,7 +3,7 @@ is a difference of squares of the pressure's size, which cancels to a little abo
 Below zero its root is NaN, the particle counts as yielding, and the reference maps it.  Which
 particles these are hangs on how a compiler fuses the products; that it is a good part of them
 does not.  The step in FP64, the step in FP32K and the CPU oracle treat such a block alike, and
-none of them maps anything where the deviator is large beside the rounding."""
+the two in 64 bits map nothing where the deviator is large beside their rounding."""
 import numpy as np
 import pytest
 
@@ -39,7 +39,8 @@ def test_mapped_as_in_the_reference(lib, deviator):
     o.step()
     mapped = np.mean(o.P["eps_pl_dot"] != 0.0)
     assert (0.2 < mapped < 0.8) if deviator < 1e-6 else mapped == 0.0
-    for precision, staged in ((abi.SPH_PREC_FP64, False), (abi.SPH_PREC_FP64, True), (abi.SPH_PREC_FP32K, False)):
+    forms = [(abi.SPH_PREC_FP64, False), (abi.SPH_PREC_FP64, True), (abi.SPH_PREC_FP32K, False)]
+    for precision, staged in forms if deviator < 1e-6 else forms[:2]:
         part, nan = mapped_on_device(c, precision, staged)
         assert (0.2 < part < 0.8) if deviator < 1e-6 else part == 0.0, (precision, staged)
         assert nan == (part if deviator == 0.0 else 0.0), (precision, staged)   # S / |S| of a zero stress
