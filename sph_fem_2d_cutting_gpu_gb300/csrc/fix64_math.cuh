@@ -146,14 +146,24 @@ __device__ __forceinline__ Fix64 fix_exp2(Fix64 y, bool negative) {
     return {exp2_frac(F), n - 63};
 }
 
-// a / b, within 0.51 units in the last place; arguments beyond 2^+-64 (b) and
-// 2^+-511 (a) divide on the FP64 pipe.
+// a / b, correctly rounded: the 53-bit quotient of the mantissas from the reciprocal is
+// within one unit, and the sign of its exact remainder settles it, as in fix_recip_rn;
+// arguments beyond 2^+-64 (b) and 2^+-511 (a) divide on the FP64 pipe.
 static __device__ __noinline__ double div_general(double a, double b) { return a / b; }
 __device__ __forceinline__ double fix_div(double a, double b) {
-    const uint32_t ah = (uint32_t)__double2hiint(a) & 0x7fffffffu, bh = (uint32_t)__double2hiint(b) & 0x7fffffffu;
+    const uint64_t ab = (uint64_t)__double_as_longlong(a), bb = (uint64_t)__double_as_longlong(b);
+    const uint32_t ah = (uint32_t)(ab >> 32) & 0x7fffffffu, bh = (uint32_t)(bb >> 32) & 0x7fffffffu;
     if (bh - 0x3bf00000u >= 0x08000000u || (ah - 0x20000000u >= 0x40000000u && flag_nonzero(a)))
         return div_general(a, b);
-    return fix_scale(fix_norm(fix_recip(__hiloint2double((int)bh, __double2loint(b)))), a, __double2hiint(b) < 0);
+    const uint64_t A = (ab & 0xfffffffffffffull) | 0x10000000000000ull;
+    const uint64_t B = (bb & 0xfffffffffffffull) | 0x10000000000000ull;
+    const bool less = A < B;                             // a quotient in [1/2, 1), else in [1, 2)
+    uint64_t q = (mul_hi(recip_mant(B) << (less ? 2 : 1), A << 11) + 512) >> 10;   // [2^52, 2^53]
+    const long long rem = (long long)((A << (less ? 53 : 52)) - q * B);
+    q += 2 * rem > (long long)B ? 1 : 2 * rem < -(long long)B ? -1 : 0;
+    const uint64_t sign = (ab ^ bb) & 0x8000000000000000ull;
+    const int e = (int)(ah >> 20) - (int)(bh >> 20) + (less ? 1022 : 1023);
+    return __longlong_as_double((long long)(flag_nonzero(a) ? sign + ((uint64_t)(uint32_t)(e - 1) << 52) + q : sign));
 }
 
 // pow(x, n) for x > 0 and n in [2^-9, 2), within 0.6 units in the last place; other

@@ -1,4 +1,4 @@
-// The device functions of csrc/fix64.cuh, element by element, for tests/test_gpu_device_math.py.
+// The device functions of csrc/fix64.cuh and csrc/fix64_math.cuh, element by element, for tests/test_gpu_device_math.py.
 // One launch evaluates function `op` for n elements: operands in a and b (bit patterns of
 // doubles, or of floats in the low words; 64-bit mantissas with their exponent), the result's
 // bits in out.
@@ -7,13 +7,15 @@
 namespace sphfem {
 namespace {
 
-enum Op { kFixDouble, kFixScale };
+enum Op { kFixDouble, kFixScale, kFixDiv, kDiv };
 
 __device__ uint64_t evaluate(int op, uint64_t a, uint64_t b, int e) {
-    const double y = __longlong_as_double((long long)b);
+    const double x = __longlong_as_double((long long)a), y = __longlong_as_double((long long)b);
     switch (op) {
         case kFixDouble: return (uint64_t)__double_as_longlong(fix_double({a, e}));
         case kFixScale: return (uint64_t)__double_as_longlong(fix_scale({a, e}, y, (e & 1) != 0));
+        case kFixDiv: return (uint64_t)__double_as_longlong(fix_div(x, y));
+        case kDiv: return (uint64_t)__double_as_longlong(x / y);
     }
     return 0;
 }

@@ -1,4 +1,4 @@
-"""The arithmetic on 64-bit mantissas (csrc/fix64.cuh) as compiled: its functions evaluated on the
+"""The arithmetic on 64-bit mantissas (csrc/fix64.cuh, csrc/fix64_math.cuh) as compiled: its functions evaluated on the
 GPU element by element (device_math.cu), against exact rationals and correctly rounded doubles,
 over random arguments and over the ends of their ranges."""
 import ctypes as C
@@ -14,7 +14,7 @@ from sph_fem_2d_cutting_gpu_gb300 import build
 
 pytestmark = pytest.mark.gpu
 
-OPS = ("fix_double", "fix_scale")
+OPS = ("fix_double", "fix_scale", "fix_div", "div")
 
 
 @pytest.fixture(scope="module")
@@ -94,3 +94,33 @@ def test_scaled_double(evaluate):
             unit = Fraction(math.ulp(want))
             assert abs(Fraction(g) - f) <= Fraction(51, 100) * unit, (mi, xi, ei)
             assert g == 0.0 or (g > 0) == (f > 0)
+
+
+EDGES = [0.0, -0.0, 5e-324, 2.0 ** -1022, -(2.0 ** -1023), 1.0, -1.0, 1.0 + 2.0 ** -52, 2.0 - 2.0 ** -52, 3.0, 0.1,
+         1.7976931348623157e308, math.inf, -math.inf, math.nan] + \
+        [s * 2.0 ** e * f for s in (1, -1) for e in (-512, -511, -64, -63, 63, 64, 511, 512) for f in (1.0, 1.0 - 2.0 ** -53)]
+
+
+def same(a, b):
+    """Equal bits, or both NaN."""
+    return (a == b) | (np.isnan(a.view(np.float64)) & np.isnan(b.view(np.float64)))
+
+
+def test_division(evaluate):
+    """fix_div against IEEE division, bit for bit: within the ranges of its own path, where
+    mantissas are equal or neighbours, and at and beyond their ends."""
+    rng = np.random.default_rng(3)
+    n = 2_000_000
+    a, b = (rng.choice([-1.0, 1.0], n) * rng.uniform(1.0, 2.0, n) * 2.0 ** rng.integers(-k, k, n).astype(np.float64)
+            for k in (530, 66))
+    near = rng.random(n) < 0.2
+    a[near] = np.abs(b[near]) * 2.0 ** rng.integers(-20, 20, near.sum())
+    a = (bits(a).astype(np.int64) + np.where(near, rng.integers(-2, 3, n), 0)).view(np.float64)
+    few = rng.random(n) < 0.2   # short mantissas: exact quotients and ones beside them
+    a[few], b[few] = np.rint(a[few] / 2.0 ** 500) + 1.0, np.float64(1.0) + rng.integers(0, 1000, few.sum())
+    pairs = [(x, y) for x in EDGES for y in EDGES]
+    a = np.concatenate([a, [p[0] for p in pairs]])
+    b = np.concatenate([b, [p[1] for p in pairs]])
+    got, want = evaluate("fix_div", bits(a), bits(b)), evaluate("div", bits(a), bits(b))
+    bad = np.flatnonzero(~same(got, want))
+    assert len(bad) == 0, [(a[i].hex(), b[i].hex(), hex(int(got[i])), hex(int(want[i]))) for i in bad[:5]]
