@@ -246,7 +246,8 @@ __device__ __forceinline__ float fix_atan2f(float y, float x) {
     const uint32_t ab = (uint32_t)__float_as_int(y) & 0x7fffffffu, bb = (uint32_t)__float_as_int(x) & 0x7fffffffu;
     const uint32_t lb = min(ab, bb), hb = max(ab, bb);
     const int s = (int)(hb >> 23) - (int)(lb >> 23);
-    if (lb < 0x00800000u || hb >= 0x7f800000u || s > 60) {   // not both normal and of like size
+    // not both normal and of like size, or so large that the quotient's 1 / hi would flush to zero
+    if (lb < 0x00800000u || hb > 0x7e800000u || s > 60) {
         if (ab == 0 && bb <= 0x7f800000u) return copysignf(__float_as_int(x) < 0 ? 3.14159274f : 0.f, y);
         if (bb == 0 && ab <= 0x7f800000u) return copysignf(1.57079637f, y);
         return atan2_general(y, x);

@@ -7,15 +7,23 @@
 namespace sphfem {
 namespace {
 
-enum Op { kFixDouble, kFixScale, kFixDiv, kDiv };
+enum Op { kFixDouble, kFixScale, kFixDiv, kDiv, kFixAtan2, kAtan2, kFixSin, kFixCos, kSin, kCos };
 
 __device__ uint64_t evaluate(int op, uint64_t a, uint64_t b, int e) {
     const double x = __longlong_as_double((long long)a), y = __longlong_as_double((long long)b);
+    const float xf = __uint_as_float((uint32_t)a), yf = __uint_as_float((uint32_t)b);
+    float sn, cs;
     switch (op) {
         case kFixDouble: return (uint64_t)__double_as_longlong(fix_double({a, e}));
         case kFixScale: return (uint64_t)__double_as_longlong(fix_scale({a, e}, y, (e & 1) != 0));
         case kFixDiv: return (uint64_t)__double_as_longlong(fix_div(x, y));
         case kDiv: return (uint64_t)__double_as_longlong(x / y);
+        case kFixAtan2: return __float_as_uint(fix_atan2f(yf, xf));
+        case kAtan2: return __float_as_uint((float)atan2((double)yf, (double)xf));
+        case kFixSin: fix_sincosf(xf, sn, cs); return __float_as_uint(sn);
+        case kFixCos: fix_sincosf(xf, sn, cs); return __float_as_uint(cs);
+        case kSin: return __float_as_uint((float)sin((double)xf));
+        case kCos: return __float_as_uint((float)cos((double)xf));
     }
     return 0;
 }

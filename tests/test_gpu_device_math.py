@@ -14,7 +14,7 @@ from sph_fem_2d_cutting_gpu_gb300 import build
 
 pytestmark = pytest.mark.gpu
 
-OPS = ("fix_double", "fix_scale", "fix_div", "div")
+OPS = ("fix_double", "fix_scale", "fix_div", "div", "fix_atan2f", "atan2", "fix_sinf", "fix_cosf", "sin", "cos")
 
 
 @pytest.fixture(scope="module")
@@ -124,3 +124,60 @@ def test_division(evaluate):
     got, want = evaluate("fix_div", bits(a), bits(b)), evaluate("div", bits(a), bits(b))
     bad = np.flatnonzero(~same(got, want))
     assert len(bad) == 0, [(a[i].hex(), b[i].hex(), hex(int(got[i])), hex(int(want[i]))) for i in bad[:5]]
+
+
+EDGES_F = [0.0, 1e-45, 2.0 ** -149 * 3, 1.1754942e-38, 2.0 ** -126, 2.0 ** -125, 1e-20, 1.0, 1.0000001, 0.99999994, 63 / 64,
+           1 / 64, 2.0 ** 60, 2.0 ** 61, 2.0 ** 125, 1.9999999 * 2.0 ** 125, 2.0 ** 126, 1.5 * 2.0 ** 126, 2.0 ** 127,
+           3.4028235e38, math.inf, math.nan]
+
+
+def bits_f(x):
+    return np.asarray(x, np.float32).view(np.uint32).astype(np.uint64)
+
+
+def compare_floats(got, want, what, allowed):
+    """Within one float of each other, and equal but for `allowed` of them; NaN and infinities equal."""
+    g, w = got.astype(np.uint32).view(np.float32), want.astype(np.uint32).view(np.float32)
+    finite = np.isfinite(w)
+    assert np.array_equal(np.isnan(g), np.isnan(w)) and np.array_equal(g[np.isinf(w)], w[np.isinf(w)]), what
+    steps = np.abs(got.astype(np.int64) - want.astype(np.int64))[finite]   # adjacent bit patterns: adjacent floats
+    assert steps.max() <= 1 and np.count_nonzero(steps) <= allowed, (what, steps.max(), np.count_nonzero(steps))
+
+
+def test_atan2(evaluate):
+    """fix_atan2f against the double function rounded to float.  Both round a value known to about
+    2^-52 of it or better, so they differ where the value lies that close to the middle of two
+    floats, once in 2^27 values: not at all in these but by chance (1.5 % in two million), so one
+    is allowed.  The edges: zeros, subnormals, ratios around the table's, infinities and NaN, and
+    numbers of 2^126 and more, whose reciprocal the hardware's approximation flushes to zero."""
+    rng = np.random.default_rng(5)
+    n = 2_000_000
+    y, x = (rng.choice([-1.0, 1.0], n) * rng.uniform(1.0, 2.0, n) * 2.0 ** rng.integers(lo, hi, n).astype(np.float64)
+            for lo, hi in ((-60, 40), (-20, 40)))
+    close = rng.random(n) < 0.5
+    y[close] = x[close] * rng.uniform(-2.0, 2.0, close.sum())
+    y, x = y.astype(np.float32), x.astype(np.float32)
+    signed = [s * v for v in EDGES_F for s in (1, -1)]
+    pairs = np.array([(p, q) for p in signed for q in signed], np.float32)
+    for k in range(2):
+        large = rng.uniform(-3.4e38, 3.4e38, (20_000, 2)).astype(np.float32)   # mostly 2^126 and more
+        pairs = np.concatenate([pairs, large])
+    y, x = np.concatenate([y, pairs[:, 0]]), np.concatenate([x, pairs[:, 1]])
+    compare_floats(evaluate("fix_atan2f", bits_f(x), bits_f(y)), evaluate("atan2", bits_f(x), bits_f(y)), "atan2", 1)
+
+
+def test_sine_and_cosine(evaluate):
+    """fix_sincosf likewise, over every magnitude up to pi/2 (the half of an arctangent)."""
+    rng = np.random.default_rng(6)
+    half_pi = np.float32(math.pi / 2)
+    x = (rng.uniform(-1.0, 1.0, 2_000_000) * half_pi).astype(np.float32)
+    x[::4] *= (2.0 ** -rng.integers(1, 40, len(x[::4]))).astype(np.float32)
+    near = np.arange(-2000, 1) + int(half_pi.view(np.uint32))
+    quarter = np.arange(-2000, 2000) + int(np.float32(math.pi / 4).view(np.uint32))
+    x = np.concatenate([x, *(v.astype(np.uint32).view(np.float32) for v in (near, quarter)),
+                        np.array([0.0, -0.0, 1e-45, 2.0 ** -126, 2.0 ** -13, 2.0 ** -13 * (1 - 2.0 ** -24), -half_pi], np.float32)])
+    for f in ("sin", "cos"):
+        compare_floats(evaluate(f"fix_{f}f", bits_f(x)), evaluate(f, bits_f(x)), f, 1)
+    bad = np.array([1.7, -2.0, 1e30, math.inf, -math.inf, math.nan], np.float32)
+    for f in ("fix_sinf", "fix_cosf"):
+        assert np.isnan(evaluate(f, bits_f(bad)).astype(np.uint32).view(np.float32)).all()
