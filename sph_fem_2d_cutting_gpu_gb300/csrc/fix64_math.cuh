@@ -9,7 +9,7 @@
 // function in IEEE floating-point arithmetic" (ACM TOMS 16, 1990) and "... of the
 // exponential function ..." (ACM TOMS 15, 1989), with series and tables of this
 // file's own: log2 within 2 units of 2^-64, exp2 within 40 units of 2^-63
-// (tests/test_fix64.py), so pow() is within 0.6 units in the last place.
+// (tests/test_fix64.py), so pow() is within 0.6 units in the last place on its range.
 #pragma once
 
 #include "fix64.cuh"
@@ -167,14 +167,15 @@ __device__ __forceinline__ double fix_div(double a, double b) {
 }
 
 // pow(x, n) for x > 0 and n in [2^-9, 2), within 0.6 units in the last place; other
-// arguments, and results beyond 2^+-512, go to the library's pow().
+// arguments, and results beyond 2^+-32, go to the library's pow(): n log2(x) has 64 bits, and
+// nine of them before the point would cost the result 0.4 units.
 static __device__ __noinline__ double pow_general(double x, double n) { return pow(x, n); }
 __device__ __forceinline__ double fix_pow(double x, double n) {
     const uint32_t xh = (uint32_t)__double2hiint(x), nh = (uint32_t)__double2hiint(n);
     bool neg;
     const Fix64 l = fix_log2(x, neg);
     const Fix64 y = fix_norm(l * fix_abs(n));
-    if (nh - 0x3f600000u >= 0x00a00000u || xh - 0x00100000u >= 0x7fe00000u || y.e + 63 >= 9) {
+    if (nh - 0x3f600000u >= 0x00a00000u || xh - 0x00100000u >= 0x7fe00000u || y.e + 63 >= 5) {
         if (nh - 0x3f600000u < 0x00a00000u && (xh | (uint32_t)__double2loint(x)) == 0u) return 0.;
         return pow_general(x, n);
     }
@@ -198,7 +199,7 @@ __device__ __forceinline__ double fix_pow_or_log(double x, double n, bool lg) {
     const Fix64 l = fix_log2(x, neg);
     if (lg) return xh >= 0x7ff00000u ? log_general(x) : fix_double(l * Fix64{0xb17217f7d1cf79acull, -64});
     const Fix64 y = fix_norm(l * fix_abs(n));
-    if (nh - 0x3f600000u >= 0x00a00000u || xh - 0x00100000u >= 0x7fe00000u || y.e + 63 >= 9) {
+    if (nh - 0x3f600000u >= 0x00a00000u || xh - 0x00100000u >= 0x7fe00000u || y.e + 63 >= 5) {
         if (nh - 0x3f600000u < 0x00a00000u && (xh | (uint32_t)__double2loint(x)) == 0u) return 0.;
         return pow_general(x, n);
     }

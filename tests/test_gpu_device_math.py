@@ -4,6 +4,7 @@ over random arguments and over the ends of their ranges."""
 import ctypes as C
 import math
 import subprocess
+from decimal import Decimal, localcontext
 from fractions import Fraction
 from pathlib import Path
 
@@ -14,7 +15,9 @@ from sph_fem_2d_cutting_gpu_gb300 import build
 
 pytestmark = pytest.mark.gpu
 
-OPS = ("fix_double", "fix_scale", "fix_div", "div", "fix_atan2f", "atan2", "fix_sinf", "fix_cosf", "sin", "cos")
+OPS = ("fix_double", "fix_scale", "fix_div", "div", "fix_atan2f", "atan2", "fix_sinf", "fix_cosf", "sin", "cos", "fix_pow",
+       "pow", "fix_log_above_1", "log", "fix_pow_or_log_pow", "fix_pow_or_log_log", "rho_inv2", "rho_vol", "rho_sound",
+       "float_trunc", "float_of_normal", "cand_pack64", "cand_pack32", "cand_far", "cand_row_diff")
 
 
 @pytest.fixture(scope="module")
@@ -33,6 +36,7 @@ def evaluate(tmp_path_factory):
         assert r == 0, f"{op}: CUDA error {r}"
         return out
 
+    call.lib = lib
     return call
 
 
@@ -181,3 +185,174 @@ def test_sine_and_cosine(evaluate):
     bad = np.array([1.7, -2.0, 1e30, math.inf, -math.inf, math.nan], np.float32)
     for f in ("fix_sinf", "fix_cosf"):
         assert np.isnan(evaluate(f, bits_f(bad)).astype(np.uint32).view(np.float32)).all()
+
+
+def units_off(got, exact):
+    """Distance in units in the last place of the exact value's double."""
+    return abs(Decimal(got) - exact) / Decimal(math.ulp(float(exact)))
+
+
+def test_power(evaluate):
+    """fix_pow within 0.6 units in its range (x > 0, 2^-9 <= n < 2, results within 2^+-32): n log2(x),
+    64 bits with five before the point, is off by under five units of 2^-59, exp2 by 40 of 2^-63, so
+    the value is off by under 0.1 units before its last rounding.  Outside, the library's pow."""
+    rng = np.random.default_rng(7)
+    n = 4000
+    x = np.exp2(rng.uniform(-300.0, 300.0, n))
+    x[::4] = 1.0 + rng.choice([-1, 1], len(x[::4])) * np.exp2(-rng.uniform(1.0, 52.0, len(x[::4])))
+    x[1::4] = rng.uniform(0.0, 2.0, len(x[1::4]))
+    k = np.exp2(rng.uniform(-9.0, 0.99, n))
+    k[:6] = [2.0 ** -9, 2.0 - 2.0 ** -52, 1.0, 0.5, 1.5, 0.34]
+    got, both = evaluate("fix_pow", bits(x), bits(k)), evaluate("fix_pow_or_log_pow", bits(x), bits(k))
+    assert np.array_equal(got, both)
+    size = np.abs(k * np.log2(x))
+    own, far = size < 31.99, size > 32.01
+    assert own.sum() > n // 2 and far.sum() > n // 10
+    assert np.array_equal(got[far], evaluate("pow", bits(x[far]), bits(k[far])))
+    with localcontext() as c:
+        c.prec = 50
+        for g, xi, ki in zip(got.view(np.float64)[own].tolist(), x[own].tolist(), k[own].tolist()):
+            assert units_off(g, Decimal(xi) ** Decimal(ki)) <= Decimal("0.6"), (xi, ki)
+    exponents = [0.0, -0.0, 2.0 ** -9 * (1 - 2.0 ** -53), 2.0, 3.0, -0.5, 300.0, math.inf, -math.inf, math.nan]
+    pairs = [(p, q) for p in EDGES for q in EDGES + exponents + [0.5, 1.9]]
+    a, b = (bits([p[i] for p in pairs]) for i in (0, 1))
+    got, want = evaluate("fix_pow", a, b), evaluate("pow", a, b)
+    assert np.array_equal(got, evaluate("fix_pow_or_log_pow", a, b))
+    g, w = got.view(np.float64), want.view(np.float64)
+    assert np.array_equal(np.isnan(g), np.isnan(w))
+    ok = same(got, want) | (np.isfinite(w) & (np.abs(g - w) <= 2.6 * np.spacing(np.abs(w))))   # the library's own 2 units
+    assert ok.all(), [(pairs[i], g[i], w[i]) for i in np.flatnonzero(~ok)[:5]]
+
+
+def test_logarithm(evaluate):
+    """fix_log_above_1: log2 is off by less than 2 units of 2^-64 and a truncation of 2^-64 of its
+    value; with the product by ln 2 under 2^-62 in all, beside the last rounding."""
+    rng = np.random.default_rng(8)
+    x = np.concatenate([np.exp2(rng.uniform(0.0, 1023.0, 1500)), 1.0 + np.exp2(-rng.uniform(0.0, 52.0, 1500)),
+                        [1.0 + 2.0 ** -52, 2.0, 2.0 - 2.0 ** -52, 1.7976931348623157e308]])
+    got = evaluate("fix_log_above_1", bits(x))
+    assert np.array_equal(got, evaluate("fix_pow_or_log_log", bits(x), bits(np.full(len(x), 0.3))))
+    with localcontext() as c:
+        c.prec = 50
+        for g, xi in zip(got.view(np.float64).tolist(), x.tolist()):
+            exact = Decimal(xi).ln()
+            slack = Decimal(2) ** -62 * (1 + exact)
+            assert abs(Decimal(g) - exact) <= Decimal("0.5") * Decimal(math.ulp(float(exact))) + slack, xi
+    ends = bits([math.inf, math.nan])
+    for op in ("fix_log_above_1", "fix_pow_or_log_log"):
+        assert same(evaluate(op, ends), evaluate("log", ends)).all()
+
+
+def test_density_quotients(evaluate):
+    """rho_terms: 1 / rho^2 and mass / rho within 0.51 units, the root of K / rho rounded to float
+    equal to the float root of the rounded quotient; densities out of range as IEEE gives them."""
+    rng = np.random.default_rng(9)
+    n = 3000
+    rho = np.exp2(rng.uniform(-63.0, 63.0, n))
+    rho[::2] = rng.uniform(1.0, 20.0, len(rho[::2]))
+    mass, bulk = np.exp2(rng.uniform(-40.0, 2.0, n)), np.exp2(rng.uniform(-30.0, 30.0, n))
+    out = {f: evaluate(f, bits(rho), bits(v)).view(np.float64)
+           for f, v in (("rho_inv2", mass), ("rho_vol", mass), ("rho_sound", bulk))}
+    for i in range(n):
+        for f, exact in (("rho_inv2", 1 / Fraction(rho[i]) ** 2), ("rho_vol", Fraction(mass[i]) / Fraction(rho[i]))):
+            assert abs(Fraction(out[f][i]) - exact) <= Fraction(51, 100) * Fraction(math.ulp(float(exact))), (f, rho[i])
+    want = np.sqrt((bulk / rho).astype(np.float32)).astype(np.float64)
+    assert np.array_equal(out["rho_sound"], want)   # once in 2^29 the two roundings of bulk / rho would differ
+    with np.errstate(all="ignore"):
+        r = np.array([v for v in EDGES if abs(v) > 2.0 ** 64 or not 2.0 ** -64 < abs(v) or v < 0])
+        for f, m, want in (("rho_inv2", 0.5, 1.0 / (r * r)), ("rho_vol", 0.5, 0.5 / r),
+                           ("rho_sound", 2.0, np.sqrt((2.0 / r).astype(np.float32)).astype(np.float64))):
+            got = evaluate(f, bits(r), bits(np.full(len(r), m)))
+            assert same(got, bits(want)).all(), f
+
+
+def test_conversions(evaluate):
+    """float_of_normal is the conversion to float; float_trunc truncates, and bounds what it cannot hold."""
+    rng = np.random.default_rng(10)
+    x = np.exp2(rng.uniform(-125.9, 127.0, 100_000))
+    assert np.array_equal(evaluate("float_of_normal", bits(x)), bits_f(x.astype(np.float32)))
+    x *= rng.choice([-1.0, 1.0], len(x))
+    t = evaluate("float_trunc", bits(x)).astype(np.uint32).view(np.float32).astype(np.float64)
+    assert (np.abs(t) <= np.abs(x)).all() and (np.abs(t) >= np.abs(x) * (1 - 2.0 ** -23)).all() and (t * x > 0).all()
+    ends = np.array([0.0, 5e-324, 1e-300, 2.0 ** -127, 2.0 ** 127, 1e300, math.inf, math.nan, -1e300, -1e-300])
+    t = evaluate("float_trunc", bits(ends)).astype(np.uint32).view(np.float32)
+    assert np.array_equal(np.abs(t), np.array([0, 0, 0, 0, *[math.inf] * 5, 0], np.float32)) and t[8] < 0
+
+
+def test_sigmoid_reciprocal(evaluate):
+    """recip_ge1 at every float from 1 on: the correctly rounded reciprocal below 2^126, where the
+    result is normal, and within one unit beyond."""
+    counts, ends = (C.c_ulonglong * 2)(), (C.c_float * 2)()
+    assert evaluate.lib.device_recip(counts, ends) == 0
+    assert list(counts) == [0, 0] and ends[0] == 0.0 and math.isnan(ends[1])
+
+
+def words(x, y):
+    return bits_f(x) | (bits_f(y) << np.uint64(32))
+
+
+def halves(v):
+    return (v & np.uint64(0xFFFFFFFF)).astype(np.uint32).view(np.float32), (v >> np.uint64(32)).astype(np.uint32).view(np.float32)
+
+
+BLANKED, NON_FINITE, FAR = 1 << 30, 1 << 28, -(1 << 31)
+
+
+@pytest.mark.parametrize("cell", [4.25e-4, 8.5e-4, 1.0, 3.7e3])
+def test_candidate_entries_64(evaluate, cell):
+    """cand_pack64: the offsets in the cell to 8 units of the last place, the flags and the row
+    (mod 8) in the lowest bits, from which cand_row_diff has the row difference up to the widest
+    stencil; a record marked non-finite, or further than 4 cells off, may not be sorted out."""
+    rng = np.random.default_rng(11)
+    n = 40_000
+    c = np.float32(cell)
+    x, y = (rng.uniform(-6.0, 6.0, n).astype(np.float32) * c for _ in range(2))
+    x[:4], y[4:8] = [np.nan, np.inf, -np.inf, 4 * c], [np.nan, np.inf, -np.inf, -4 * c]
+    row = rng.integers(0, 5000, n).astype(np.int32)
+    flags = rng.choice([0, BLANKED, NON_FINITE], n).astype(np.int32)
+    v = evaluate("cand_pack64", words(x, y), bits_f(np.full(n, c)), row | flags)
+    px, py = halves(v)
+    low = px.view(np.uint32) & 3
+    near = (np.abs(x) <= 4 * c) & (np.abs(y) <= 4 * c)
+    assert np.array_equal(low & 1 == 1, flags == BLANKED)
+    assert np.array_equal(low & 2 == 2, ~near | (flags == NON_FINITE))
+    ok = np.isfinite(x) & np.isfinite(y)
+    for p, q in ((px, x), (py, y)):
+        assert (np.abs(p[ok] - q[ok]) <= 8 * np.spacing(np.abs(q[ok]))).all()
+    diff = rng.integers(-3, 4, n).astype(np.int32)
+    d = evaluate("cand_row_diff", bits_f(py), e=row + diff).view(np.int64)
+    assert np.array_equal(d, diff)
+
+
+@pytest.mark.parametrize("cell", [4.25e-4, 8.5e-4, 1.0, 3.7e3])
+def test_candidate_entries_32(evaluate, cell):
+    """cand_pack32: x as it is, infinite for a blanked record and NaN for one that the entry cannot
+    stand for; y in the frame that repeats every 8 rows, in which two entries of a stencil have their
+    distance to 2^-19 of a cell.  cand_far: further than a quarter of a cell from the cell's box."""
+    rng = np.random.default_rng(12)
+    n = 40_000
+    c = np.float32(cell)
+    edge = bits_f(np.full(n, c))
+    rows, y8 = [rng.integers(3, 5000, n).astype(np.int32)], []
+    rows.append(rows[0] + rng.integers(-3, 4, n).astype(np.int32))
+    ys = [rng.uniform(-0.25, 1.25, n).astype(np.float32) * c for _ in rows]
+    x = rng.uniform(-0.25, 1.25, n).astype(np.float32) * c
+    for row, y in zip(rows, ys):
+        px, py = halves(evaluate("cand_pack32", words(x, y), edge, row))
+        assert np.array_equal(px, x)
+        y8.append(py)
+    d = np.abs(y8[0] - y8[1])
+    wrapped = np.abs(np.minimum(d, np.float32(8) * c - d))
+    true = np.abs((rows[0] - rows[1]) * np.float64(c) + ys[0].astype(np.float64) - ys[1])
+    close = true <= 4 * np.float64(c)
+    assert np.abs(wrapped[close] - true[close]).max() <= 2.0 ** -19 * cell
+    assert (~close).any() and wrapped[~close].min() >= 3.4 * cell
+    for flag, expect in ((BLANKED, np.isposinf), (NON_FINITE, np.isnan), (FAR, np.isnan), (BLANKED | FAR, np.isposinf)):
+        e = (rows[0].astype(np.int64) | flag).astype(np.int32)
+        assert expect(halves(evaluate("cand_pack32", words(x, ys[0]), edge, e))[0]).all()
+    x, y = (rng.uniform(-0.6, 1.6, n).astype(np.float32) * c for _ in range(2))
+    x[:4] = [np.nan, np.inf, -np.inf, 0.5 * c]
+    far = evaluate("cand_far", words(x, y), edge).astype(np.uint32)
+    mid = np.float32(0.5) * c
+    inside = (np.abs(x - mid) <= np.float32(0.75) * c) & (np.abs(y - mid) <= np.float32(0.75) * c)
+    assert np.array_equal(far, np.where(inside, 0, 1 << 31).astype(np.uint32))
