@@ -227,7 +227,7 @@ template <bool kNodes, bool kNextHash, class SF>
 __global__ void __launch_bounds__(kBlock, 8) k_step_tail_fem(int N, KConsts K, SF A, SegDev seg, FemDev F,
                                                           const ToolDev *__restrict__ tool, SortScratch X,
                                                           uint32_t *status) {
-    begin_after();
+    begin_after(tool);
     const int node_blocks = kNodes ? div_up(F.n_nodes, blockDim.x) : 0;
     if (kNodes && (int)blockIdx.x < node_blocks) {
         const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -251,7 +251,7 @@ template <bool kNextHash, class SF>
 __global__ void __launch_bounds__(128) k_contact_queue(KConsts K, SF A, SegDev seg, const ToolDev *__restrict__ tool,
                                                        const double *__restrict__ T_nodes, SortScratch X,
                                                        uint32_t *status) {
-    begin_after();
+    begin_after(tool, T_nodes);
     const int count = X.counts[K.g.num_cell + 1], warps = (int)(gridDim.x * 4u);
     for (int q = (int)(blockIdx.x * 4u + (threadIdx.x >> 5)); q < count; q += warps) {
         const int i = X.slots[q];
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kBlock) k_step_tail(int N, KConsts K, SF A, Se
                                                       const ToolDev *__restrict__ tool,
                                                       const double *__restrict__ T_nodes, SortScratch X,
                                                       uint32_t *status) {
-    begin_after();
+    begin_after(tool, T_nodes);
     PARTICLE_LOOP_HEAD
     step_tail_one<kMode, kNextHash>(i, K, A, X, status);
 }

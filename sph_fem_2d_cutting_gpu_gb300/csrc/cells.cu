@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(kBlock) k_hash_count(int N, const double2 *__r
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int32_t *__restrict__ in, int n,
                                                               int32_t *__restrict__ block_sums) {
-    begin_after();
+    begin_after(in, block_sums);
     __shared__ int sw[32];
     int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     int s = 0;
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int32_t *__r
 }
 
 __global__ void __launch_bounds__(1024) k_scan_top(int32_t *__restrict__ block_sums, int nb) {
-    begin_after();
+    begin_after(block_sums);
     __shared__ int sw[32];
     int carry = 0;
     for (int base = 0; base < nb; base += blockDim.x) {
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(int32_t *__restrict_
                                                             int32_t *__restrict__ offsets,
                                                             int32_t *__restrict__ cell_start,
                                                             int32_t *__restrict__ cell_end, int num_cell) {
-    begin_after();
+    begin_after(counts, block_sums, offsets, cell_start, cell_end);
     __shared__ int sw[32];
     int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     int v[kScanItems];
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kBlock) k_scatter(int N, const int32_t *__rest
                                                     const int32_t *__restrict__ offsets, int32_t *__restrict__ slots,
                                                     KConsts K, FemDev F, const ToolDev *__restrict__ tool,
                                                     sph_rigid_tool *rigid) {
-    begin_after();
+    begin_after(key, arrival, offsets, slots, tool);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) scatter_one(i, key, arrival, offsets, slots);
     else if (rigid) rigid_move_part(*rigid, i - N, K.dt);
@@ -279,14 +279,10 @@ __global__ void __launch_bounds__(kBlock) k_build_records(int N, KConsts K, Sort
 // artificial stress run on the integer pipes (fix64_math.cuh), which leaves it between the
 // FP64 pipe and HBM: 1,048,576 particles 403 -> 195 us (0.75 KB each, 4.0 TB/s),
 // 640,000 particles 259 -> 127 us.
-__global__ void __launch_bounds__(kBlock) k_gather_fused(int N, SortScratch X, KConsts K,
-                                                         SortedFields A, SortedFields B, FixedFields F,
-                                                         dbl4 *__restrict__ rec64, float2 *__restrict__ cand32,
-                                                         const ToolDev *__restrict__ tools, uint32_t *status) {
-    begin_after();
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= N) return;
-    const int i = X.slots[s], k = rank_of(s, i, X.key, X.offsets, X.slots, status);
+__device__ __forceinline__ void gather64_one(int k, int i, const KConsts &K, const SortedFields &A, const SortedFields &B,
+                                             const FixedFields &F, const int32_t *__restrict__ hash_src,
+                                             dbl4 *__restrict__ rec64, float2 *__restrict__ cand32,
+                                             const ToolDev *__restrict__ tools) {
     F.idx[k] = i;
     double2 pos = A.pos[i], vel = A.vel[i];
     dbl4 S = A.S[i];
@@ -295,7 +291,7 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused(int N, SortScratch X, K
     double2 pos_t = A.pos_t[i], vel_t = A.vel_t[i];
     double rho_t = A.rho_t[i], T_t = A.T_t[i];
     dbl4 S_t = A.S_t[i];
-    int hash = X.hash_next[i];
+    int hash = hash_src[i];
     B.pos[k] = pos;
     B.vel[k] = vel;
     B.fc[k] = A.fc[i];
@@ -344,13 +340,24 @@ __global__ void __launch_bounds__(kBlock) k_gather_fused(int N, SortScratch X, K
     write_record64(rec64, cand32, k, K, pos, vel, S, R, p, h, rho, q, T, blanked, tool, hash);
 }
 
+__global__ void __launch_bounds__(kBlock) k_gather_fused(int N, SortScratch X, KConsts K,
+                                                         SortedFields A, SortedFields B, FixedFields F,
+                                                         dbl4 *__restrict__ rec64, float2 *__restrict__ cand32,
+                                                         const ToolDev *__restrict__ tools, uint32_t *status) {
+    begin_after(rec64, cand32, tools);
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= N) return;
+    const int i = X.slots[s], k = rank_of(s, i, X.key, X.offsets, X.slots, status);
+    gather64_one(k, i, K, A, B, F, X.hash_next, rec64, cand32, tools);
+}
+
 template <class SF, class FF>
 __global__ void __launch_bounds__(kBlock) k_gather_fused32(int N, SortScratch X, KConsts K, SF A, FF Fsrc,
                                                            SortedFields32 B, FixedFields32 F,
                                                            int32_t *__restrict__ idx, float4 *__restrict__ rec,
                                                            float2 *__restrict__ cand,
                                                            const ToolDev *__restrict__ tools, uint32_t *status) {
-    begin_after();
+    begin_after(idx, rec, cand, tools);
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= N) return;
     const int i = X.slots[s], k = rank_of(s, i, X.key, X.offsets, X.slots, status);

@@ -66,7 +66,7 @@ __device__ __forceinline__ int rank_of(int s, int i, const int32_t *__restrict__
     int cs = offsets[c], ce = offsets[c + 1];
     if (ce - cs > kCellRankCap && s == cs) set_status(status, SPH_STATUS_CELL_OVERFLOW);
     int rank = 0;
-    for (int t = cs; t < ce; t++) rank += (__ldg(slots + t) < i) ? 1 : 0;
+    for (int t = cs; t < ce; t++) rank += (slots[t] < i) ? 1 : 0;
     return cs + rank;
 }
 // perm[k] = original index of the particle that lands at sorted position k.

@@ -239,8 +239,17 @@ __device__ __forceinline__ void set_status(uint32_t *status, uint32_t bits) {
 // that take their places beside a running kernel end up unevenly on the SMs
 // (12,000-particle cut, FP32K: 78 us a step with ordinary launches, 93 with the early
 // start, 76 as it is).  Without effect in a kernel launched the ordinary way.
-__device__ __forceinline__ void begin_after() {
+// pointers: the kernel's __restrict__ pointers.  A load through one of those, read-only
+// for the whole kernel as it says, the compiler may place before any instruction, a wait
+// included; with their values coming out of an instruction behind the wait it cannot.
+template <class P>
+__device__ __forceinline__ void known_after(P &pointer) {
+    asm volatile("" : "+l"(pointer) : : "memory");
+}
+template <class... P>
+__device__ __forceinline__ void begin_after(P &...pointers) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    (known_after(pointers), ...);
 }
 
 // Non-contracted a + b*c (keeps host and device bit-identical for the tool kinematics).

@@ -19,7 +19,7 @@ namespace sphfem {
 template <bool kMove>
 __global__ void __launch_bounds__(kBlock) k_fem_rate_update(KConsts K, FemDev F, SegDev seg,
                                                             const ToolDev *__restrict__ tool) {
-    begin_after();
+    begin_after(tool);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= F.n_nodes) return;
     fem_rate_update_one(i, K, F, seg, tool);

@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(kB, kMinB) k_interact32(int N, KConsts K, cons
                                                        const ToolDev *__restrict__ tool,
                                                        int32_t *__restrict__ secant_iters, uint32_t *status,
                                                        int cap, MlpDev mlp) {
-    begin_after();
+    begin_after(offsets, rec, cand, tool, secant_iters);
     interact32_block<kFused, kB, kStaged, kMlp, kSplit>(blockIdx.x, N, K, offsets, rec, cand, B, F, seg, tool,
                                                         secant_iters, status, cap, mlp);
 }

@@ -29,6 +29,14 @@
 
 namespace sphfem {
 
+// A quarter of a record, which nothing writes while the sums run.  (Not volatile: the compiler
+// places it as it does its own loads.)
+__device__ __forceinline__ dbl4 ld_nc(const dbl4 *p) {
+    dbl4 v;
+    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+
 constexpr int kLanes64 = 4;                            // lanes per particle
 constexpr int kThreads64 = 128;                        // threads per block
 constexpr int kParts64 = kThreads64 / kLanes64;        // particles per block
@@ -233,14 +241,12 @@ inline bool map_by_quads(int N) { return div_up(N, kParts64) <= 5 * 152; }
 // of 7,355 (rigid, PSE) 93.2 -> 89.4, of 1,600 (lattice) 58.5 -> 53.3; but of 19,600 99.6 ->
 // 117.4.
 inline bool three_blocks(int N) { return div_up(N, kParts64) <= 3 * 152; }
-template <Map64 kMap, int kBlocks = 5>
-__global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KConsts K, const int32_t *__restrict__ offsets,
-                                                              const dbl4 *__restrict__ rec,
-                                                              const float2 *__restrict__ cand, SortedFields B,
-                                                              FixedFields F, SegDev seg,
-                                                              const ToolDev *__restrict__ tool,
-                                                              int32_t *__restrict__ secant_iters, uint32_t *status) {
-    begin_after();
+template <Map64 kMap>
+__device__ __forceinline__ void interact64_block(int N, const KConsts &K, const int32_t *__restrict__ offsets,
+                                                 const dbl4 *__restrict__ rec, const float2 *__restrict__ cand,
+                                                 const SortedFields &B, const FixedFields &F, const SegDev &seg,
+                                                 const ToolDev *__restrict__ tool, int32_t *__restrict__ secant_iters,
+                                                 uint32_t *status) {
     constexpr bool kFused = kMap != kMapNone;
     constexpr int kSums = kFused ? 9 : 13;
     __shared__ int s_list[kParts64 * kListPitch64];
@@ -251,7 +257,8 @@ __global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KCons
     const int k = (int)blockIdx.x * kParts64 + part;
     int *list = s_list + part * kListPitch64;
     const int kk = min(k, N - 1);
-    const dbl4 i0 = rec[4 * kk + 0], i1 = rec[4 * kk + 1], i2 = rec[4 * kk + 2], i3 = rec[4 * kk + 3];
+    const dbl4 i0 = ld_nc(rec + 4 * kk), i1 = ld_nc(rec + 4 * kk + 1), i2 = ld_nc(rec + 4 * kk + 2),
+               i3 = ld_nc(rec + 4 * kk + 3);
     const int fi = (int)__double_as_longlong(i3.w);
     const int hash = B.hash[kk];
     const sph_geom_constants &geo = K.g;
@@ -329,7 +336,8 @@ __global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KCons
         // phase 2: the pair body over the list, shared by the group's lanes
         for (int t = sub; t < cnt; t += kLanes64) {
             const int jn = list[t];
-            const dbl4 n0 = rec[4 * jn + 0], n1 = rec[4 * jn + 1], n2 = rec[4 * jn + 2], n3 = rec[4 * jn + 3];
+            const dbl4 n0 = ld_nc(rec + 4 * jn), n1 = ld_nc(rec + 4 * jn + 1), n2 = ld_nc(rec + 4 * jn + 2),
+                       n3 = ld_nc(rec + 4 * jn + 3);
             const int fj = (int)__double_as_longlong(n3.w);
             const double ex = n0.x - xi, ey = n0.y - yi;   // minus the reference's distance vector
             const double rr2 = ex * ex + ey * ey;
@@ -450,7 +458,7 @@ __global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KCons
     const int e = (int)blockIdx.x * kParts64 + (int)threadIdx.x;
     auto particle = [&]() -> bool {
         if (e >= N) return false;
-        const dbl4 e0 = rec[4 * e + 0], e2 = rec[4 * e + 2], e3 = rec[4 * e + 3];
+        const dbl4 e0 = ld_nc(rec + 4 * e), e2 = ld_nc(rec + 4 * e + 2), e3 = ld_nc(rec + 4 * e + 3);
         const int fe = (int)__double_as_longlong(e3.w);
         if (fe & kFlagBlanked) {
             if (kFused) rigid_heat_blanked(e, K, B);
@@ -499,6 +507,17 @@ __global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KCons
     } else {
         particle();
     }
+}
+
+template <Map64 kMap, int kBlocks = 5>
+__global__ void __launch_bounds__(kThreads64, kBlocks) k_interact64(int N, KConsts K, const int32_t *__restrict__ offsets,
+                                                              const dbl4 *__restrict__ rec,
+                                                              const float2 *__restrict__ cand, SortedFields B,
+                                                              FixedFields F, SegDev seg,
+                                                              const ToolDev *__restrict__ tool,
+                                                              int32_t *__restrict__ secant_iters, uint32_t *status) {
+    begin_after(offsets, rec, cand, tool, secant_iters);
+    interact64_block<kMap>(N, K, offsets, rec, cand, B, F, seg, tool, secant_iters, status);
 }
 
 }  // namespace sphfem

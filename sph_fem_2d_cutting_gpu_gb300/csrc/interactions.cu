@@ -85,10 +85,10 @@ static __device__ __noinline__ double pse_weight_general(double rr2, double inv_
 __global__ void __launch_bounds__(128) k_heat_pse64(int N, KConsts K, const int32_t *__restrict__ offsets,
                                                     const dbl4 *__restrict__ rec,
                                                     const int32_t *__restrict__ hashes, double *__restrict__ T_t) {
-    begin_after();
+    begin_after(offsets, rec, hashes, T_t);
     const int k = (int)(blockIdx.x * 128u + threadIdx.x) / kPseLanes, sub = (int)threadIdx.x % kPseLanes;
     const int kk = min(k, N - 1);
-    const dbl4 i0 = rec[4 * kk + 0], i2 = rec[4 * kk + 2], i3 = rec[4 * kk + 3];
+    const dbl4 i0 = ld_nc(rec + 4 * kk), i2 = ld_nc(rec + 4 * kk + 2), i3 = ld_nc(rec + 4 * kk + 3);
     const int fi = (int)__double_as_longlong(i3.w);
     const bool live = k < N && !(fi & kFlagBlanked);
     const double xi = i0.x, yi = i0.y, Ti = i3.z;
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(128) k_heat_pse64(int N, KConsts K, const int3
                 j1 = __ldg(offsets + ii * g.ny + hi_j);
             }
             if (j >= j1) break;
-            const dbl4 n0 = rec[4 * j + 0], n3 = rec[4 * j + 3];
+            const dbl4 n0 = ld_nc(rec + 4 * j), n3 = ld_nc(rec + 4 * j + 3);
             const double ex = n0.x - xi, ey = n0.y - yi;
             const double rr2 = ex * ex + ey * ey;
             double w;
@@ -141,7 +141,7 @@ template <class TT>   // T_t: double (staged call, FP64 arrays) or float (the co
 __global__ void __launch_bounds__(kBlock) k_heat_pse32(int N, KConsts K, const int32_t *__restrict__ offsets,
                                                        const float4 *__restrict__ rec,
                                                        const int32_t *__restrict__ hashes, TT *__restrict__ T_t) {
-    begin_after();
+    begin_after(offsets, rec, hashes, T_t);
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= N) return;
     const float4 *rec_c = rec + 2 * (size_t)N, *rec_d = rec + 3 * (size_t)N;   // the records' last two quarters

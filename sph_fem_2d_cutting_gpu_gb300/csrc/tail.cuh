@@ -126,7 +126,7 @@ __device__ __forceinline__ int inside_binned(double2 qp, const SegDev &seg, cons
     if (n < 0) {
         if (!seg.geo) return inside_judgement(qp, seg.left, seg.right, seg.n);
         for (int i = 0; i < seg.n; i++)
-            crossings += on_segment_mesh_geo(__ldg(seg.left + i), __ldg(seg.right + i), seg.geo[i], qp);
+            crossings += on_segment_mesh_geo(seg.left[i], seg.right[i], seg.geo[i], qp);
         return crossings & 1;
     }
     const int32_t *list = seg.bin_list + b * kSegBinCap;
@@ -139,8 +139,8 @@ __device__ __forceinline__ int inside_binned(double2 qp, const SegDev &seg, cons
             double Q[2];
 #pragma unroll
             for (int u = 0; u < 2; u++) {
-                L[u] = __ldg(seg.left + ii[u]);
-                R[u] = __ldg(seg.right + ii[u]);
+                L[u] = seg.left[ii[u]];
+                R[u] = seg.right[ii[u]];
                 Y[u] = *reinterpret_cast<const double2 *>(&seg.geo[ii[u]].ymin_f);
                 Q[u] = seg.geo[ii[u]].inv_slope;
             }
@@ -156,8 +156,8 @@ __device__ __forceinline__ int inside_binned(double2 qp, const SegDev &seg, cons
     }
     for (; k < n; k++) {
         const int i = list[k];
-        crossings += seg.geo ? on_segment_mesh_geo(__ldg(seg.left + i), __ldg(seg.right + i), seg.geo[i], qp)
-                             : on_segment_mesh(__ldg(seg.left + i), __ldg(seg.right + i), qp);
+        crossings += seg.geo ? on_segment_mesh_geo(seg.left[i], seg.right[i], seg.geo[i], qp)
+                             : on_segment_mesh(seg.left[i], seg.right[i], qp);
     }
     return crossings & 1;
 }
@@ -191,10 +191,10 @@ __device__ __forceinline__ int find_shortest_distance_geo(double2 qp, double &dN
         const int i = i0 + u;
         if (!hit[u]) continue;
         {
-            const double2 L = __ldg(seg.left + i), Rr = __ldg(seg.right + i);
+            const double2 L = seg.left[i], Rr = seg.right[i];
             const double ymax = find_max(L.y, Rr.y), ymin = find_min(L.y, Rr.y);
             const double xmax = find_max(L.x, Rr.x), xmin = find_min(L.x, Rr.x);
-            const double2 ni = __ldg(seg.normal + i);
+            const double2 ni = seg.normal[i];
             const double d = (qp.x - L.x) * ni.x + (qp.y - L.y) * ni.y;
             if (d >= 0. && d < depth) {
                 const double intersec_x = qp.x - d * ni.x;
@@ -208,7 +208,7 @@ __device__ __forceinline__ int find_shortest_distance_geo(double2 qp, double &dN
       }
     }
     if (sg != -1 && depth <= limit_value) {
-        const double2 ns = __ldg(seg.normal + sg);
+        const double2 ns = seg.normal[sg];
         n_re = make_double2(-ns.x, -ns.y);
         dN = -depth;
         return sg;
@@ -408,12 +408,12 @@ __device__ __forceinline__ int crossings_lanes(double2 qp, const SegDev &seg, co
     int crossings = 0;
     if (n < 0) {
         for (int i = lane; i < seg.n; i += 32)
-            crossings += on_segment_mesh_geo(__ldg(seg.left + i), __ldg(seg.right + i), seg.geo[i], qp);
+            crossings += on_segment_mesh_geo(seg.left[i], seg.right[i], seg.geo[i], qp);
     } else {
         const int32_t *list = seg.bin_list + b * kSegBinCap;
         for (int k = lane; k < n; k += 32) {
             const int i = list[k];
-            crossings += on_segment_mesh_geo(__ldg(seg.left + i), __ldg(seg.right + i), seg.geo[i], qp);
+            crossings += on_segment_mesh_geo(seg.left[i], seg.right[i], seg.geo[i], qp);
         }
     }
     return crossings;
@@ -428,10 +428,10 @@ __device__ __forceinline__ int shortest_distance_lanes(double2 qp, double &dN, d
     for (int i = lane; i < seg.n; i += 32) {
         const SegGeo &g = seg.geo[i];
         if (kx > g.kx0 && kx < g.kx1 && ky > g.ky0 && ky < g.ky1) {
-            const double2 L = __ldg(seg.left + i), Rr = __ldg(seg.right + i);
+            const double2 L = seg.left[i], Rr = seg.right[i];
             const double ymax = find_max(L.y, Rr.y), ymin = find_min(L.y, Rr.y);
             const double xmax = find_max(L.x, Rr.x), xmin = find_min(L.x, Rr.x);
-            const double2 ni = __ldg(seg.normal + i);
+            const double2 ni = seg.normal[i];
             const double d = (qp.x - L.x) * ni.x + (qp.y - L.y) * ni.y;
             if (d >= 0. && d < best) {
                 const double intersec_x = qp.x - d * ni.x;
@@ -447,7 +447,7 @@ __device__ __forceinline__ int shortest_distance_lanes(double2 qp, double &dN, d
     const int sg = bi == 0x7fffffff ? -1 : bi;
     const double depth = sg == -1 ? (double)FLT_MAX : best;
     if (sg != -1 && depth <= 2.5e-4) {
-        const double2 ns = __ldg(seg.normal + sg);
+        const double2 ns = seg.normal[sg];
         n_re = make_double2(-ns.x, -ns.y);
         dN = -depth;
         return sg;
@@ -456,7 +456,7 @@ __device__ __forceinline__ int shortest_distance_lanes(double2 qp, double &dN, d
     double bd = FLT_MAX;
     int bj = 0x7fffffff;
     for (int i = lane; i < seg.n; i += 32) {
-        const double2 Rr = __ldg(seg.right + i);
+        const double2 Rr = seg.right[i];
         const double d_trial = sqrtf_d((qp.x - Rr.x) * (qp.x - Rr.x) + (qp.y - Rr.y) * (qp.y - Rr.y));
         if (d_trial < bd) {
             bd = d_trial;
@@ -467,11 +467,11 @@ __device__ __forceinline__ int shortest_distance_lanes(double2 qp, double &dN, d
     const int s_near = bj == 0x7fffffff ? sg : bj;
     const double dep = bj == 0x7fffffff ? (double)FLT_MAX : bd;
     if (s_near == -1) return -1;
-    const double2 ns = __ldg(seg.normal + s_near);
-    const double2 rs = __ldg(seg.right + s_near);
+    const double2 ns = seg.normal[s_near];
+    const double2 rs = seg.right[s_near];
     int jm = 0x7fffffff;
     for (int j = lane; j < seg.n; j += 32) {
-        const double2 Lj = __ldg(seg.left + j);
+        const double2 Lj = seg.left[j];
         if (Lj.y == rs.y && Lj.x == rs.x) {
             jm = j;
             break;
@@ -481,7 +481,7 @@ __device__ __forceinline__ int shortest_distance_lanes(double2 qp, double &dN, d
     for (int o = 16; o > 0; o >>= 1) jm = min(jm, __shfl_xor_sync(kFullMask, jm, o));
     double nsx = ns.x, nsy = ns.y;
     if (jm != 0x7fffffff) {
-        const double2 nj = __ldg(seg.normal + jm);
+        const double2 nj = seg.normal[jm];
         nsx = (nj.x + ns.x) / 2.;
         nsy = (nj.y + ns.y) / 2.;
     }

@@ -17,7 +17,7 @@ namespace sphfem {
 // positions (do_mass_ele_matrix_construction_p1q3 /
 // do_stiffness_ele_matrix_construction_p1q3), one element per thread.
 __global__ void __launch_bounds__(kBlock) k_wear_elements(KConsts K, FemDev F, WearDev W, double *__restrict__ out) {
-    begin_after();
+    begin_after(out);
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= W.n_elem) return;
     const int4 el = W.elements[W.elem[k]];
