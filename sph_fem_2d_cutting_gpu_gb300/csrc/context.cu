@@ -1974,6 +1974,7 @@ int sph_mlp_attach(sph_ctx *ctx, const sph_mlp *m) {
         DALLOC(ctx->jc_list, ctx->N);
         DALLOC(ctx->jc_list_count, 1);
     }
+    std::lock_guard<std::mutex> only(m->busy);
     CK(cudaStreamSynchronize(m->stream));
     CK(cudaMemcpy(ctx->mlp_params, m->params, sizeof(float) * kMlpParams, cudaMemcpyDeviceToDevice));
     CK(cudaMemcpy(ctx->mlp_wb, m->wb, sizeof(uint16_t) * kMlpWb, cudaMemcpyDeviceToDevice));

@@ -217,6 +217,7 @@ const char *sph_mlp_last_error(const sph_mlp *m) { return m ? m->err.c_str() : "
 
 int sph_mlp_get_params(sph_mlp *m, float *params, sph_mlp_norm *norm) {
     if (!m) return SPH_ERR_INVALID;
+    std::lock_guard<std::mutex> only(m->busy);
     MCK(cudaSetDevice(m->device));
     if (params) {
         MCK(cudaMemcpyAsync(params, m->params, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, m->stream));
@@ -228,6 +229,7 @@ int sph_mlp_get_params(sph_mlp *m, float *params, sph_mlp_norm *norm) {
 
 int sph_mlp_set_params(sph_mlp *m, const float *params, const sph_mlp_norm *norm) {
     if (!m) return SPH_ERR_INVALID;
+    std::lock_guard<std::mutex> only(m->busy);
     MCK(cudaSetDevice(m->device));
     if (norm) {
         for (int c = 0; c < 4; c++)
@@ -268,6 +270,7 @@ int sph_mlp_fit_norm(sph_mlp *m, const float *x, const float *t, int64_t n) {
     double mu = st / n, var = std::max(stt / n - mu * mu, 0.0);
     nm.y_mean = (float)mu;
     nm.y_std = (float)std::max(std::sqrt(var), 1e-6);
+    std::lock_guard<std::mutex> only(m->busy);
     m->norm = nm;
     return SPH_OK;
 }
@@ -347,8 +350,8 @@ int sph_mlp_adam_step(sph_mlp *m, const float *x, const float *t, int64_t n, flo
 int sph_mlp_train(sph_mlp *m, const float *x, const float *t, int64_t n, int32_t epochs, int32_t batch, float lr,
                   uint64_t seed, float *epoch_loss) {
     if (!m || !x || !t || n < 1 || epochs < 1 || batch < 1) return SPH_ERR_INVALID;
-    if (n > INT32_MAX) return mfail(m, SPH_ERR_INVALID, "too many samples");
     std::lock_guard<std::mutex> only(m->busy);
+    if (n > INT32_MAX) return mfail(m, SPH_ERR_INVALID, "too many samples");
     MCK(cudaSetDevice(m->device));
     Batch b;
     int r = upload_batch(m, x, t, n, b);

@@ -21,12 +21,13 @@ struct sph_mlp {
     int64_t loss_cap = 0;
     uint32_t *status = nullptr;
     // Scratch kept for the next call: a batch's features and targets on the device (up to
-    // kKeepSamples), and a page-locked copy of gradient, loss and status.  One call at a
-    // time uses it and the stream (busy).
+    // kKeepSamples), and a page-locked copy of gradient, loss and status.
     float *batch = nullptr;
     int64_t batch_cap = 0;
     float *result = nullptr;
-    std::mutex busy;
+    // Held by every call that uses the scratch, the stream, the parameters or the norm, a
+    // context's attachment included: one at a time.
+    mutable std::mutex busy;
     sph_mlp_norm norm{};
     int64_t adam_t = 0;
     std::vector<void *> allocs;
