@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kBlock) k_fric_heat_rigid(int N, KConsts K, So
 // kNodes (tail_takes_nodes): the first blocks take the tool's nodes, their thermal update
 // from the segments' kept Robin terms and their motion; neither needs the tail or is
 // needed by it.
-template <bool kNodes, bool kNextHash, class SF>
+template <bool kNodes, class SF>
 __global__ void __launch_bounds__(kBlock, 8) k_step_tail_fem(int N, KConsts K, SF A, SegDev seg, FemDev F,
                                                           const ToolDev *__restrict__ tool, SortScratch X,
                                                           uint32_t *status) {
@@ -243,11 +243,11 @@ __global__ void __launch_bounds__(kBlock, 8) k_step_tail_fem(int N, KConsts K, S
         X.slots[histogram_slot(X.counts, K.g.num_cell + 1)] = i;
         return;
     }
-    step_tail_one<0, kNextHash>(i, K, A, X, status);
+    step_tail_one<0>(i, K, A, X, status);
 }
 
 // One warp per queued particle: its contact, then its tail.
-template <bool kNextHash, class SF>
+template <class SF>
 __global__ void __launch_bounds__(128) k_contact_queue(KConsts K, SF A, SegDev seg, const ToolDev *__restrict__ tool,
                                                        const double *__restrict__ T_nodes, SortScratch X,
                                                        uint32_t *status) {
@@ -256,19 +256,19 @@ __global__ void __launch_bounds__(128) k_contact_queue(KConsts K, SF A, SegDev s
     for (int q = (int)(blockIdx.x * 4u + (threadIdx.x >> 5)); q < count; q += warps) {
         const int i = X.slots[q];
         contact_fem_warp(i, K, A, seg, tool, T_nodes, status);
-        if ((threadIdx.x & 31u) == 0) step_tail_one<0, kNextHash>(i, K, A, X, status);
+        if ((threadIdx.x & 31u) == 0) step_tail_one<0>(i, K, A, X, status);
         __syncwarp();
     }
 }
 
-template <int kMode, bool kNextHash, class SF>
+template <int kMode, class SF>
 __global__ void __launch_bounds__(kBlock) k_step_tail(int N, KConsts K, SF A, SegDev seg,
                                                       const ToolDev *__restrict__ tool,
                                                       const double *__restrict__ T_nodes, SortScratch X,
                                                       uint32_t *status) {
     begin_after(tool, T_nodes);
     PARTICLE_LOOP_HEAD
-    step_tail_one<kMode, kNextHash>(i, K, A, X, status);
+    step_tail_one<kMode>(i, K, A, X, status);
 }
 
 // ---- measurement hooks: output.cu:41-49 report_force (sum of fc + ft); peak T ----------------------
@@ -427,34 +427,27 @@ void launch_invalidate(cudaStream_t s, int N, const SortedFields &A, uint32_t *s
 }
 template <class SF>
 static void step_tail(cudaStream_t s, int N, const KConsts &K, const SF &A, const SegDev &seg, const FemDev &F,
-                      ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status, bool next_hash) {
+                      ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status) {
     const int tb = fp64_block(N);   // the rigid contact is FP64 work: spread small systems over all SMs
     if (K.has_tool) {
         const int grid = std::min(2 * 152, div_up(N, 4));   // a queue of any length; two blocks on each SM
         const int nodes = div_up(F.n_nodes, tb);
-        launch_after(s,
-                     next_hash ? (nodes ? k_step_tail_fem<true, true, SF> : k_step_tail_fem<false, true, SF>)
-                               : (nodes ? k_step_tail_fem<true, false, SF> : k_step_tail_fem<false, false, SF>),
-                     div_up(N, tb) + nodes, tb, 0, N, K, A, seg, F, tool, X, status);
-        launch_after(s, next_hash ? k_contact_queue<true, SF> : k_contact_queue<false, SF>, grid, 128, 0, K, A, seg,
-                     tool, T_nodes, X, status);
+        launch_after(s, nodes ? k_step_tail_fem<true, SF> : k_step_tail_fem<false, SF>, div_up(N, tb) + nodes, tb, 0, N,
+                     K, A, seg, F, tool, X, status);
+        launch_after(s, k_contact_queue<SF>, grid, 128, 0, K, A, seg, tool, T_nodes, X, status);
     } else if (K.rigid) {
-        launch_after(s, next_hash ? k_step_tail<2, true, SF> : k_step_tail<2, false, SF>, div_up(N, tb), tb, 0, N, K, A, seg,
-                     tool, T_nodes, X, status);
+        launch_after(s, k_step_tail<2, SF>, div_up(N, tb), tb, 0, N, K, A, seg, tool, T_nodes, X, status);
     } else {
-        launch_after(s, next_hash ? k_step_tail<0, true, SF> : k_step_tail<0, false, SF>, div_up(N, tb), tb, 0, N, K, A, seg,
-                     tool, T_nodes, X, status);
+        launch_after(s, k_step_tail<0, SF>, div_up(N, tb), tb, 0, N, K, A, seg, tool, T_nodes, X, status);
     }
 }
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields &A, const SegDev &seg,
-                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
-                      bool next_hash) {
-    step_tail(s, N, K, A, seg, F, tool, T_nodes, X, status, next_hash);
+                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status) {
+    step_tail(s, N, K, A, seg, F, tool, T_nodes, X, status);
 }
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields32 &A, const SegDev &seg,
-                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
-                      bool next_hash) {
-    step_tail(s, N, K, A, seg, F, tool, T_nodes, X, status, next_hash);
+                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status) {
+    step_tail(s, N, K, A, seg, F, tool, T_nodes, X, status);
 }
 void launch_rigid_move(cudaStream_t s, sph_rigid_tool *t, double dt) { launch_after(s, k_rigid_move, 1, 32, 0, t, dt); }
 void launch_rigid_move_particles(cudaStream_t s, int N, const SortedFields &A, const sph_rigid_tool *t, double dt) {

@@ -520,9 +520,9 @@ int issue_fused_body(sph_ctx *ctx, int64_t &n, int w, cudaEvent_t *ev = nullptr)
     }
     if (ev) CK(cudaEventRecord(ev[4], s));
     if (f32)
-        launch_step_tail(s, N, ctx->K, B32, ctx->seg, tail_fem, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status, true);
+        launch_step_tail(s, N, ctx->K, B32, ctx->seg, tail_fem, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status);
     else
-        launch_step_tail(s, N, ctx->K, B, ctx->seg, tail_fem, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status, true);
+        launch_step_tail(s, N, ctx->K, B, ctx->seg, tail_fem, ctx->tool_dev, ctx->fem.T, ctx->X, ctx->W.status);
     n += ctx->has_tool ? 2 : 1;   // with the FEM tool: the tail and the contact queue
     if (ev) CK(cudaEventRecord(ev[5], s));
     CK_LAUNCH();

@@ -103,11 +103,9 @@ constexpr bool tail_takes_nodes(int N) { return N <= 8 * 152 * 256; }
 // with the FEM tool (its y-bins built): the contact queue after it (one more launch).  F:
 // the nodes whose thermal update (from seg.robin) and motion go with it; none: n_nodes 0.
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields &A, const SegDev &seg,
-                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
-                      bool next_hash);
+                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status);
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields32 &A, const SegDev &seg,
-                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status,
-                      bool next_hash);
+                      const FemDev &F, ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status);
 void launch_rigid_move(cudaStream_t s, sph_rigid_tool *t, double dt);
 void launch_rigid_move_particles(cudaStream_t s, int N, const SortedFields &A, const sph_rigid_tool *t, double dt);
 void launch_contact_rigid(cudaStream_t s, int N, const KConsts &K, const SortedFields &A);

@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kPB, kPMinBlocks) k_step_persistent(PersistArg
         if (!grid_barrier(P.bar, status)) return;
     }
     // boundary conditions, invalidation, the next step's hashes and histogram
-    for (int i = gtid; i < N; i += gstride) step_tail_one<0, true>(i, K, P.B, P.X, status);
+    for (int i = gtid; i < N; i += gstride) step_tail_one<0>(i, K, P.B, P.X, status);
 }
 
 template <bool kTool, bool kMlp>

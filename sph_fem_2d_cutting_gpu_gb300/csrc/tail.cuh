@@ -593,9 +593,9 @@ __device__ __forceinline__ void contact_fem_warp(int i, const KConsts &K, const 
 // and do_compute_contact_forces (tool_gpu.cu:146-216); kMode 0: no tool, or the
 // FEM tool whose contact has been applied just before -- then
 // do_boundary_conditions, do_boundary_conditions_thermal, do_invalidate
-// (actions_gpu.cu:756-824) and (kNextHash) the next step's compute_hashes and
-// the counting-sort histogram (grid.cu:25-42) on the final state.
-template <int kMode, bool kNextHash, class SF>
+// (actions_gpu.cu:756-824) and the next step's compute_hashes and the counting-sort
+// histogram (grid.cu:25-42) on the final state.
+template <int kMode, class SF>
 __device__ __forceinline__ void step_tail_one(int i, const KConsts &K, const SF &A, const SortScratch &X,
                                               uint32_t *status) {
     bool blanked = flag_is_one(A.blanked[i]);
@@ -633,25 +633,23 @@ __device__ __forceinline__ void step_tail_one(int i, const KConsts &K, const SF 
             st |= SPH_STATUS_NAN_BLANKED;
         }
     }
-    if (kNextHash) {
-        int h;
-        if (!blanked) {
-            const sph_geom_constants &g = K.g;
-            int ix = cell_coord(pos.x, g.bbmin_x, g.dx, K.f.inv_cell);
-            int iy = cell_coord(pos.y, g.bbmin_y, g.dx, K.f.inv_cell);
-            h = ix * g.ny + iy;
-        } else {
-            h = A.hash[i];   // blanked particles keep their stale hash
-        }
-        int key = h;
-        if (h < 0 || h >= K.g.num_cell) {
-            key = K.g.num_cell;
-            st |= SPH_STATUS_OUT_OF_GRID;
-        }
-        X.key[i] = key;
-        X.arrival[i] = histogram_slot(X.counts, key);
-        X.hash_next[i] = h;   // the visible hash array changes only at the next sort
+    int h;
+    if (!blanked) {
+        const sph_geom_constants &g = K.g;
+        int ix = cell_coord(pos.x, g.bbmin_x, g.dx, K.f.inv_cell);
+        int iy = cell_coord(pos.y, g.bbmin_y, g.dx, K.f.inv_cell);
+        h = ix * g.ny + iy;
+    } else {
+        h = A.hash[i];   // blanked particles keep their stale hash
     }
+    int key = h;
+    if (h < 0 || h >= K.g.num_cell) {
+        key = K.g.num_cell;
+        st |= SPH_STATUS_OUT_OF_GRID;
+    }
+    X.key[i] = key;
+    X.arrival[i] = histogram_slot(X.counts, key);
+    X.hash_next[i] = h;   // the visible hash array changes only at the next sort
     if (st) set_status(status, st);
 }
 
