@@ -430,7 +430,7 @@ static void step_tail(cudaStream_t s, int N, const KConsts &K, const SF &A, cons
                       ToolDev *tool, const double *T_nodes, const SortScratch &X, uint32_t *status) {
     const int tb = fp64_block(N);   // the rigid contact is FP64 work: spread small systems over all SMs
     if (K.has_tool) {
-        const int grid = std::min(2 * 152, div_up(N, 4));   // a queue of any length; two blocks on each SM
+        const int grid = std::min(2 * sm_count(), div_up(N, 4));   // a queue of any length; two blocks on each SM
         const int nodes = div_up(F.n_nodes, tb);
         launch_after(s, nodes ? k_step_tail_fem<true, SF> : k_step_tail_fem<false, SF>, div_up(N, tb) + nodes, tb, 0, N,
                      K, A, seg, F, tool, X, status);

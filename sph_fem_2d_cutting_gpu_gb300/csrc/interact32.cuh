@@ -738,7 +738,7 @@ static void launch_i32(cudaStream_t s, int N, const KConsts &K, const int32_t *o
 // to matter: step of 12,000 particles (cut) 71.1 -> 68.9 us, 90,000 (lattice) 62.7 -> 59.6,
 // 250,000 128.0 -> 124.4; but 422,500 194.6 -> 197.5.  The sums are the same; as between
 // all shapes, the compiler may fuse a multiply-add of the epilogue differently.
-constexpr bool few_waves32(int N) { return N <= 3 * 5 * 152 * 128; }
+inline bool few_waves32(int N) { return N <= 3 * 5 * sm_count() * 128; }
 
 // The launch shapes of kInteractVariants (interactions.cu), in its order.
 template <bool kMlp>

@@ -232,7 +232,7 @@ static __device__ __noinline__ void return_map(int k, const KConsts &K, const So
 // start in their place, 2 % slower (1,048,576 particles 2,891 -> 2,949 us).  So: groups on
 // grids of up to one wave (map_by_quads).
 enum Map64 { kMapNone, kMapLane, kMapQuads };
-inline bool map_by_quads(int N) { return div_up(N, kParts64) <= 5 * 152; }
+inline bool map_by_quads(int N) { return div_up(N, kParts64) <= 5 * sm_count(); }
 // kBlocks: blocks an SM that the registers must leave room for.  5 (20 warps, 96
 // registers, 164 bytes spilled) on a grid of many waves, where warps alternate between the
 // integer and the FP64 pipe: 4 blocks at 128 registers were 5 % slower on the
@@ -240,7 +240,7 @@ inline bool map_by_quads(int N) { return div_up(N, kParts64) <= 5 * 152; }
 // a grid that needs no more (three_blocks): step of 12,000 particles (cut) 112.2 -> 107.4 us,
 // of 7,355 (rigid, PSE) 93.2 -> 89.4, of 1,600 (lattice) 58.5 -> 53.3; but of 19,600 99.6 ->
 // 117.4.
-inline bool three_blocks(int N) { return div_up(N, kParts64) <= 3 * 152; }
+inline bool three_blocks(int N) { return div_up(N, kParts64) <= 3 * sm_count(); }
 template <Map64 kMap>
 __device__ __forceinline__ void interact64_block(int N, const KConsts &K, const int32_t *__restrict__ offsets,
                                                  const dbl4 *__restrict__ rec, const float2 *__restrict__ cand,

@@ -48,12 +48,8 @@ void interact_variant_shape(int v, int *block, int *min_blocks, int *staged, int
     *lanes = kInteractVariants[v][3];
 }
 
-// Threads per block of the per-particle kernels with FP64 work: the largest of 256, 128,
-// 64 that still gives every SM two blocks, else 32.  The FP64 pipe is narrow, so
-// a small system (the reference's own cases are 7k-12k particles) must spread
-// over all SMs rather than fill a few.  Results do not depend on it: each
-// particle's sums run in one thread in the same order.
-int fp64_block(int N) {
+// SMs of the current device.
+int sm_count() {
     static int sms[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -62,6 +58,16 @@ int fp64_block(int N) {
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         if (n <= 0) n = 152;
     }
+    return n;
+}
+
+// Threads per block of the per-particle kernels with FP64 work: the largest of 256, 128,
+// 64 that still gives every SM two blocks, else 32.  The FP64 pipe is narrow, so
+// a small system (the reference's own cases are 7k-12k particles) must spread
+// over all SMs rather than fill a few.  Results do not depend on it: these kernels'
+// particles do not share their work.
+int fp64_block(int N) {
+    const int n = sm_count();
     for (int kb : {256, 128, 64})
         if (div_up(N, kb) >= 2 * n) return kb;
     return 32;

@@ -71,6 +71,7 @@ void launch_heat_pse(cudaStream_t s, int N, const KConsts &K, const int32_t *off
 void launch_heat_pse(cudaStream_t s, int N, const KConsts &K, const int32_t *offsets, const StepScratch &W,
                      const SortedFields32 &B);
 int interact_variant_count();
+int sm_count();          // SMs of the current device
 int fp64_block(int N);   // threads per block of the FP64 per-particle kernels for N particles
 void interact_variant_shape(int v, int *block, int *min_blocks, int *staged, int *lanes);
 
@@ -99,7 +100,7 @@ void launch_invalidate(cudaStream_t s, int N, const SortedFields &A, uint32_t *s
 // (8 blocks an SM), where a launch less counts -- 12,000 particles 5 us of a step of 76.
 // On a longer one the nodes' part, which needs more registers, costs more than a launch:
 // 1.33 M particles 625 us a step against 621, 640,000 particles 329 against 327.
-constexpr bool tail_takes_nodes(int N) { return N <= 8 * 152 * 256; }
+inline bool tail_takes_nodes(int N) { return N <= 8 * sm_count() * 256; }
 // with the FEM tool (its y-bins built): the contact queue after it (one more launch).  F:
 // the nodes whose thermal update (from seg.robin) and motion go with it; none: n_nodes 0.
 void launch_step_tail(cudaStream_t s, int N, const KConsts &K, const SortedFields &A, const SegDev &seg,
