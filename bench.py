@@ -1,5 +1,6 @@
 #!/usr/bin/env python
-"""Benchmark of the SPH workpiece hot path on GB300 (one JSON line on rank 0).
+"""Benchmark of the SPH workpiece hot path on GB300 (one JSON line on rank 0, a few KB;
+every section's full record goes to bench_details.json beside this file).
 
 Workload: the interaction micro-benchmark -- 4,194,304 particles on a
 2048 x 2048 lattice (dx = 2.5 um, positions jittered +-0.05 dx, velocity
@@ -172,6 +173,40 @@ def cpu_sample(case, max_seconds=15.0, min_steps=1):
         if el + el / n > 2.5 * max_seconds:
             break
     return case.N * n / el, num_threads(), n, el
+
+
+# What the printed line has of a run: the headline with its evidence, and of every other
+# section the times a step.
+HEADLINE = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "config", "clocks", "gpu_launches", "e2e", "e2e_sync", "roofline", "compute",
+            "stage_ms", "status", "speedup_vs_fp64", "cpu_baseline")
+
+
+def step_times(section):
+    """The ms_per_step entries of a section: numbers by name, a section's own under its name alone."""
+    out = {}
+    for k, v in section.items():
+        if k == "ms_per_step":
+            if isinstance(v, dict):
+                out.update(v)
+            else:
+                out[""] = v
+        elif isinstance(v, dict) and k not in ("launch_tuning", "autotune") and "ms_per_step" in v:
+            out.update({f"{k}.{n}".rstrip("."): t for n, t in step_times(v).items()})
+    return {n: float(f"{t:.6g}") for n, t in out.items() if isinstance(t, (int, float))}
+
+
+def emit(line, details=ROOT / "bench_details.json"):
+    """Prints the run's one line and writes all of it to `details`."""
+    try:
+        details.write_text(json.dumps(line, indent=1) + "\n")
+    except OSError as e:
+        print(f"bench: {details} not written: {e}", file=sys.stderr)
+    short = {k: line[k] for k in HEADLINE if k in line}
+    times = {k: step_times(v) for k, v in line.items() if k not in HEADLINE and isinstance(v, dict)}
+    short["sections_ms_per_step"] = {k: t[""] if list(t) == [""] else t for k, t in times.items() if t}
+    short["details"] = details.name
+    print(json.dumps(short))
 
 
 def run_reference(args):
@@ -1035,7 +1070,7 @@ def run_product(args):
         line["cpu_baseline"] = {"value": v, "unit": UNIT, "cores": cores, "kind": "port",
                                 "sample": f"{n} whole steps of the full workload in {el:.1f}s "
                                           f"(CPU oracle restatement, OpenMP)"}
-    print(json.dumps(line))
+    emit(line)
     if dist is not None:
         dist.destroy_process_group()
     return 0
