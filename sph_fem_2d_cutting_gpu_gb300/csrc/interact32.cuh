@@ -732,13 +732,20 @@ static void launch_i32(cudaStream_t s, int N, const KConsts &K, const int32_t *o
                  W.rec32, W.cand32, B, F, seg, tool, W.secant_iters, W.status, cap, mlp);
 }
 
-// The default shape up to three waves of five blocks an SM: no bound on the registers (95
-// instead of 79, five blocks instead of six), so that the loads of a pair and of the
-// epilogue are issued further ahead.  A small system has too few warps for the sixth block
-// to matter: step of 12,000 particles (cut) 71.1 -> 68.9 us, 90,000 (lattice) 62.7 -> 59.6,
-// 250,000 128.0 -> 124.4; but 422,500 194.6 -> 197.5.  The sums are the same; as between
-// all shapes, the compiler may fuse a multiply-add of the epilogue differently.
-inline bool few_waves32(int N) { return N <= 3 * 5 * sm_count() * 128; }
+// The default shape on grids of few waves: no bound on the registers (95 instead of 79,
+// five blocks an SM instead of six), so that the loads of a pair and of the epilogue are
+// issued further ahead -- where a wave of five takes no more waves than one of six, by more
+// than a scrap of the last one, and up to three.  Steps, six blocks -> five (152 SMs, waves
+// of 116,736 and 97,280 particles): 12,000 particles (cut) 71.1 -> 68.9 us; lattices 90,000
+// 63.6 -> 59.8, 160,000 97.9 -> 94.4, 193,600 106.2 -> 100.5, 250,000 132.5 -> 129.7, 291,600
+// 148.9 -> 144.3; but with a wave more 99,225 69.0 -> 74.2, 105,625 71.3 -> 78.8, 202,500 111.0 ->
+// 113.4, 230,400 116.9 -> 120.6, 313,600 157.8 -> 159.5, 422,500 204.6 -> 206.3, and just past a
+// whole wave of six 119,025 82.1 -> 82.3, 235,225 125.6 -> 127.1.  The sums are the same; as
+// between all shapes, the compiler may fuse a multiply-add of the epilogue differently.
+inline bool few_waves32(int N) {
+    const int five = 5 * sm_count() * 128, six = 6 * sm_count() * 128;
+    return N <= 3 * five && div_up(N, five) == div_up(N, six) && (N <= five || (N - 1) % six >= six / 8);
+}
 
 // The launch shapes of kInteractVariants (interactions.cu), in its order.
 template <bool kMlp>

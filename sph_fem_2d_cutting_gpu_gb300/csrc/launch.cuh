@@ -97,7 +97,8 @@ void launch_bc(cudaStream_t s, int N, const SortedFields &A);
 void launch_bc_thermal(cudaStream_t s, int N, const KConsts &K, const SortedFields &A);
 void launch_invalidate(cudaStream_t s, int N, const SortedFields &A, uint32_t *status);
 // Whether the tool's nodes are updated in the tail's launch: on a tail of at most one wave
-// (8 blocks an SM), where a launch less counts -- 12,000 particles 5 us of a step of 76.
+// (8 blocks an SM), where a launch less counts -- 12,000 particles 5 us of a step of 76,
+// 40,000 74.8 -> 69.7 us, 100,000 100.5 -> 98.4, 203,000 144.4 -> 141.7, 307,200 182.4 -> 181.1.
 // On a longer one the nodes' part, which needs more registers, costs more than a launch:
 // 1.33 M particles 625 us a step against 621, 640,000 particles 329 against 327.
 inline bool tail_takes_nodes(int N) { return N <= 8 * sm_count() * 256; }
