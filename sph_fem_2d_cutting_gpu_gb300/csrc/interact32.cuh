@@ -742,7 +742,12 @@ static void launch_i32(cudaStream_t s, int N, const KConsts &K, const int32_t *o
 // 113.4, 230,400 116.9 -> 120.6, 313,600 157.8 -> 159.5, 422,500 204.6 -> 206.3, and just past a
 // whole wave of six 119,025 82.1 -> 82.3, 235,225 125.6 -> 127.1.  The sums are the same; as
 // between all shapes, the compiler may fuse a multiply-add of the epilogue differently.
+// With the warm start in the epilogue (kMlp) the unbounded shape takes 193 registers, two
+// blocks an SM: on grids of one such wave, 12,000 particles (cut) 78.5 -> 75.5 us, 22,500
+// (lattice) 57.4 -> 54.8; but 40,000 58.7 -> 69.0, 90,000 77.5 -> 112.2, 291,600 190 -> 284.
+template <bool kMlp>
 inline bool few_waves32(int N) {
+    if (kMlp) return N <= 2 * sm_count() * 128;
     const int five = 5 * sm_count() * 128, six = 6 * sm_count() * 128;
     return N <= 3 * five && div_up(N, five) == div_up(N, six) && (N <= five || (N - 1) % six >= six / 8);
 }
@@ -767,7 +772,7 @@ void launch_i32_variant(cudaStream_t s, int N, const KConsts &K, const int32_t *
         case 12: launch_i32<128, 5, false, kMlp>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp); break;
         case 13: launch_i32<64, 10, false, kMlp>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp); break;
         default:
-            if (few_waves32(N)) launch_i32<128, 1, false, kMlp>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp);
+            if (few_waves32<kMlp>(N)) launch_i32<128, 1, false, kMlp>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp);
             else launch_i32<128, 6, false, kMlp>(s, N, K, offsets, B, F, W, seg, tool, 0, mlp);
             break;
     }
