@@ -524,7 +524,11 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             gemm_issue(tmem + 64, adw, bdw, 128, 128, tiles_done > 0);
             mma_commit(mbar_dw);
         }
-        if (!mma_wait(mbar, phase)) { timeout = true; break; }
+        if (!mma_wait(mbar, phase)) {
+            mbar_wait(mbar_dw, phase_dw);   // (bounded) the weight gradient in flight, before its TMEM is freed
+            timeout = true;
+            break;
+        }
         tmem_ld16(trow, v);
 #pragma unroll
         for (int q = 0; q < 16; q++) sh.zs[r][c0 + q] = v[q] * d1[q];   // dZ1 (FP32)

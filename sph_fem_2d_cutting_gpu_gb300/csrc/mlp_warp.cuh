@@ -23,8 +23,9 @@ namespace sphfem {
 
 // 1 / x for x >= 1 (or NaN) without the branch of a division, which keeps the evaluations
 // of a thread's neurons from overlapping: one Newton step with an exact residual from the
-// hardware's approximation, correctly rounded (Markstein 1990: all but, possibly, a
-// mantissa of ones); the approximation itself where the result is subnormal or zero.
+// hardware's approximation (Markstein 1990), correctly rounded at every float below 2^126;
+// beyond, where the result is subnormal or zero, the approximation itself, within a unit
+// (tests/test_gpu_device_math.py: every float from 1 on).
 __device__ __forceinline__ float recip_ge1(float x) {
     float r;
     asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
