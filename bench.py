@@ -58,13 +58,13 @@ ALGO_BYTES = {
 # neighbour sums, from ncu on the 2048x2048 micro workload with 2h cells
 # (dram__bytes_read.sum 723,139,584 + dram__bytes_write.sum 398,211,584 for
 # 4,194,304 particles, k_interact32<fused, 128x6>; one-pass capture).
-NCU_TRAFFIC_PER_PARTICLE = {"fp32k": (723_139_584 + 398_211_584) / 4_194_304}
+NCU_TRAFFIC_PER_PARTICLE = {"fp32k": (723_672_320 + 397_976_064) / 4_194_304}
 # Floating-point work per particle of the fused neighbour sums, from ncu's SASS
 # instruction counters (dadd + dmul + 2 dfma; fadd + fmul + 2 ffma + 2 (fadd2 + fmul2) +
 # 4 ffma2, packed pairs counted as two) on the 512x512 micro workload with 2h cells
-# (262,144 particles): k_interact64 executes 540,407,316 FP64 flops (its products and
+# (262,144 particles): k_interact64 executes 540,395,984 FP64 flops (its products and
 # quotients are integer work), k_interact32 (compact state) 1,367,097,721 FP32 flops.
-NCU_FLOPS_PER_PARTICLE = {"fp64": 540_407_316 / 262_144, "fp32k": 1_367_097_721 / 262_144}
+NCU_FLOPS_PER_PARTICLE = {"fp64": 540_395_984 / 262_144, "fp32k": 1_367_097_721 / 262_144}
 # Nominal GB300 rates (no measured figure exists for these pipes): FP64 1.25 TFLOP/s;
 # FP32 152 SMs x 128 lanes x 2 flops x 2.07 GHz = 80.5 TFLOP/s.
 NOMINAL_TFLOPS = {"fp64": 1.25, "fp32k": 80.5}

@@ -492,12 +492,14 @@ int sph_mlp_set_inference(sph_ctx *ctx, int32_t mode);
  * (threads per block, minimum resident blocks per SM, and the number of
  * neighbour records a block stages in shared memory -- 0 for global loads);
  * an autotuner times the step with each and sets the fastest.  Variant 0 is
- * the default.  Shapes with lanes_per_particle > 1 (for small systems, which
+ * the default: the shape that sph_launch_variants reports for it, or, on systems
+ * of few waves of blocks, the same threads per block without its bound on the
+ * registers.  Shapes with lanes_per_particle > 1 (for small systems, which
  * leave most of the GPU idle) let that many lanes share a particle's
  * candidates and merge their compensated sums.
  * step_form: SPH_STEP_LAUNCHES (default) -- the fused step as its chain of
- * launches (scan, scatter, rank, gather, FEM, neighbour sums, tool, contact,
- * tail), replayed from a CUDA graph; SPH_STEP_PERSISTENT -- the same stages in
+ * launches (scan, scatter, gather, neighbour sums, FEM, tool, tail, contact),
+ * replayed from a CUDA graph; SPH_STEP_PERSISTENT -- the same stages in
  * one cooperative launch with every block resident, separated by bounded
  * grid-wide barriers (SPH_STATUS_GRID_TIMEOUT if one gives up), captured in the
  * graph the same way; the same results bit for bit.  FP32K contexts only; a

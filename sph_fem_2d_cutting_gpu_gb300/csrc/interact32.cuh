@@ -4,7 +4,7 @@
 // interactions_mlp.cu (the fused step with the learned warm start folded into
 // its epilogue).  The sums are described in interactions.cu's header.
 //
-// Bound: instruction issue (75 % busy) and the L1's passes (64 % of peak), with 24
+// Bound: instruction issue (74 % busy) and the L1's passes (56 % of peak), with 24
 // warps per SM.  The candidate entries are read four to a load and tested without
 // decoding (cand_pack32), every candidate is stored and the list grows past the ones
 // that are in, the spline and the viscosity are selections instead of branches, sums

@@ -3,7 +3,8 @@
 //
 // Bound: the FP64 pipe, two operations per SM and clock.  One thread per particle
 // with every operation in FP64 took 4,872 FP64 instructions per 32 particles on the
-// lattice of 2h cells and kept the pipe 87 % busy; this kernel takes 1,400 (79 %):
+// lattice of 2h cells and kept the pipe 87 % busy; this kernel takes 1,400 (67 % of
+// a launch of 262,144 particles):
 //  * candidates are tested in FP32 on the 8-byte entries with a margin that no
 //    in-support neighbour can fall outside of; the FP64 test then runs only on
 //    the ones that pass;
@@ -15,8 +16,8 @@
 //    system of a few thousand particles fills the schedulers, and the epilogue
 //    runs once per particle in full warps from partial sums in shared memory.
 // Neighbour stage, before and after: 1,048,576-particle lattice (2h cells) 9.40 ->
-// 2.88 ms; 640,000-particle cut (cells of h) 5.53 -> 1.78 ms; 12,000-particle cut
-// 0.247 -> 0.068 ms, the return mapping of the yielding particles (return_map) included.
+// 2.94 ms; 640,000-particle cut (cells of h) 5.53 -> 1.82 ms; 12,000-particle cut
+// 0.247 -> 0.069 ms, the return mapping of the yielding particles (return_map) included.
 // A particle with anything the mantissa forms do not take (a candidate marked
 // non-finite, a smoothing length, density or volume outside 2^+-64, a product of
 // relative velocity and distance that is subnormal or 2^300 and more) repeats its
@@ -236,7 +237,7 @@ inline bool map_by_quads(int N) { return div_up(N, kParts64) <= 5 * sm_count(); 
 // kBlocks: blocks an SM that the registers must leave room for.  5 (20 warps, 96
 // registers, 164 bytes spilled) on a grid of many waves, where warps alternate between the
 // integer and the FP64 pipe: 4 blocks at 128 registers were 5 % slower on the
-// 1,048,576-particle lattice, 3 blocks 13 %.  3, with 162 registers and nothing spilled, on
+// 1,048,576-particle lattice, 3 blocks 13 %.  3, with 156 registers and nothing spilled, on
 // a grid that needs no more (three_blocks): step of 12,000 particles (cut) 112.2 -> 107.4 us,
 // of 7,355 (rigid, PSE) 93.2 -> 89.4, of 1,600 (lattice) 58.5 -> 53.3; but of 19,600 99.6 ->
 // 117.4.

@@ -4,8 +4,8 @@
 // Brookshaw heat conduction) on sm_103a.
 //
 // One thread (FP32) or a few lanes (FP64) per particle in sorted order.
-// Neighbours are visited column by column: the cells (ii, gj-R .. gj+R) of one grid column are consecutive
-// keys, so their particles form one contiguous slot range [offsets[c0],
+// Neighbours are visited column by column: the cells (ii, gj-R .. gj+R) of one grid
+// column are consecutive keys, so their particles form one contiguous slot range [offsets[c0],
 // offsets[c1+1]) -- the reference's visiting order (ii outer, jj inner,
 // sorted order inside a cell) without per-cell bookkeeping.
 //
@@ -32,8 +32,8 @@ namespace sphfem {
 // Launch shapes of the fused FP32K neighbour-sum kernel: (threads per block,
 // minimum resident blocks per SM, staged records: 0 = global loads, lanes per
 // particle).  Variant 0 is the default: 6 blocks (24 warps) per SM at 79
-// registers (on grids of few waves without that bound, few_waves32).  On the 4.19 M lattice 128x6 and 256x3 are within 0.2 % of each
-// other, 64x12, 64x8 and 128x4 1-2 % behind, 128x5 and 64x10 5 %; on the
+// registers (on grids of few waves without that bound, few_waves32).  On the
+// 4.19 M lattice 128x6 and 256x3 are within 0.2 % of each other, 64x12, 64x8 and 128x4 1-2 % behind, 128x5 and 64x10 5 %; on the
 // 12,000-particle cut the shapes with 2 and 4 lanes per particle are ahead.
 const int kInteractVariants[][4] = {{128, 6, 0, 1},   {64, 12, 0, 1},   {64, 8, 0, 1},     {128, 4, 0, 1},
                                     {256, 3, 0, 1},   {256, 1, 0, 1},   {128, 3, 640, 1},  {128, 2, 1024, 1},

@@ -2,7 +2,8 @@
 
 Candidates: every compiled launch shape of the FP32K neighbour-sum kernel
 (``sph_launch_variants``: threads per block, minimum resident blocks per SM,
-neighbour records staged in shared memory), and the persistent one-launch
+neighbour records staged in shared memory; variant 0, reported as 128x6, runs
+without that bound on the registers on systems of few waves of blocks), and the persistent one-launch
 step (``SPH_STEP_PERSISTENT``), times every cell geometry in ``CELL_GEOMETRIES`` (cell edge = h x factor,
 stencil half-width in cells; both cover the 2h kernel support).  Each
 candidate is timed on the workload itself with CUDA events over whole fused
